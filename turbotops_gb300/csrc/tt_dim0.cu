@@ -329,29 +329,34 @@ __global__ void k_iota(u32* __restrict__ p, u32 n) {
 
 // For each live edge with endpoints in different components, offer its rank
 // to both components; edges inside a component are dropped from the list.
-// (The survivors' list grows by one atomic per warp: ranks from a ballot.
-// The first round offers all m edges; later rounds read their count from
-// the previous round's counter, so rounds run without a host round trip.)
+// A round's edges are the survivors of the rounds before (`live`, their count
+// read from the previous round's counter, so rounds run without a host round
+// trip) and the sorted edges [lo, hi) that join in this round. (The
+// survivors' list grows by one atomic per warp: ranks from a ballot.)
+// A component's best rank only falls, so an offer that a plain load already
+// shows to be too large is not issued: the largest component receives most of
+// the edges, and their atomics on its one word were most of the forest's time
+// (43 M edges of 12,000 points: 23 ms a round).
 __global__ void k_bv_offer(const u64* __restrict__ keys, EdgeFmt fmt, const u32* __restrict__ live,
-                           const u32* __restrict__ nlive_in, u32 m, const u32* __restrict__ comp,
-                           u32* __restrict__ best, u32* __restrict__ live_out, u32* __restrict__ nlive_out) {
+                           const u32* __restrict__ nlive_in, u32 lo, u32 hi, const u32* __restrict__ comp,
+                           u32* best, u32* __restrict__ live_out, u32* __restrict__ nlive_out) {
     pdl_wait();
     pdl_trigger();
     const u32 lane = threadIdx.x & 31;
-    const bool all = nlive_in == nullptr;
-    const u32 nlive = all ? m : *nlive_in;
-    for (u32 base = blockIdx.x * blockDim.x; base < nlive; base += gridDim.x * blockDim.x) {
-        const u32 t = base + threadIdx.x;   // whole warps iterate together
+    const u64 nlive = nlive_in ? *nlive_in : 0u;
+    const u64 total = nlive + (hi - lo);
+    for (u64 base = u64(blockIdx.x) * blockDim.x; base < total; base += u64(gridDim.x) * blockDim.x) {
+        const u64 t = base + threadIdx.x;   // whole warps iterate together
         bool keep = false;
         u32 r = 0;
-        if (t < nlive) {
-            r = all ? t : live[t];
+        if (t < total) {
+            r = t < nlive ? live[t] : lo + u32(t - nlive);
             u32 a, b;
             decode_edge(fmt.rips(keys[r]), a, b);
             const u32 ca = comp[a], cb = comp[b];
             if (ca != cb) {
-                atomicMin(&best[ca], r);
-                atomicMin(&best[cb], r);
+                if (*reinterpret_cast<volatile const u32*>(best + ca) > r) atomicMin(&best[ca], r);
+                if (*reinterpret_cast<volatile const u32*>(best + cb) > r) atomicMin(&best[cb], r);
                 keep = true;
             }
         }
@@ -598,12 +603,25 @@ void dim0(tt_ctx* c, const Complex& cx, u32 maxdim, Dim0Out& out, u64 m_known) {
         // Three rounds a host round trip (a round after convergence finds no
         // edge between components and changes nothing); the grid covers the
         // last live count the host knows (counts only shrink).
-        u32 known = u32(m);
-        for (int round = 0; known && round < kRounds;) {
+        // The edges join in rank order, one group a trip: a component's
+        // smallest live edge is its smallest edge of all as soon as any of
+        // its edges has joined, so the forest is the same, and the shortest
+        // few edges a point connect nearly everything: by the time the long
+        // ones join, one pass finds them inside a component (or the forest
+        // is complete and they are never read). Groups of 8 n, then 64 n
+        // edges, then the rest; with fewer than 16 n edges (kNN graphs) the
+        // extra trips would cost more than the passes they save, and all
+        // join at once.
+        const u64 group[3] = {m < 16 * u64(n) ? m : 8 * u64(n), std::min<u64>(m, 72 * u64(n)), m};
+        u32 known = 0, joined = 0;
+        for (int round = 0, trip = 0; round < kRounds; ++trip) {
+            const u32 upto = u32(trip < 3 ? group[trip] : m);
+            if (!known && joined == upto) break;
             const int first = round;
             for (int q = 0; q < kPerTrip && round < kRounds; ++q, ++round) {
-                launch_pdl(k_bv_offer, grid_for(known, 256), 256, 0, fs, 
-                    out.keys, fmt, live0, round ? ctr + 2 * (round - 1) : nullptr, u32(m), comp, best, live1, ctr + 2 * round);
+                launch_pdl(k_bv_offer, grid_for(u64(known) + (upto - joined), 256), 256, 0, fs, out.keys, fmt, live0,
+                           round ? ctr + 2 * (round - 1) : nullptr, joined, q ? joined : upto, comp, best, live1,
+                           ctr + 2 * round);
                 launch_pdl(k_bv_hook, grid_for(n, 256), 256, 0, fs, out.keys, fmt, comp, best, parent, tree, n,
                                                            ctr + 2 * round + 1, ctr + 2 * round);
                 launch_pdl(k_bv_flatten, grid_for(n, 256), 256, 0, fs, parent, comp, best, n, ctr + 2 * round);
@@ -611,6 +629,7 @@ void dim0(tt_ctx* c, const Complex& cx, u32 maxdim, Dim0Out& out, u64 m_known) {
                 c->launches += 3;
                 std::swap(live0, live1);
             }
+            joined = upto;
             u32 h[2 * kPerTrip] = {};
             TT_CUDA(cudaMemcpyAsync(h, ctr + 2 * first, sizeof(u32) * 2 * (round - first), cudaMemcpyDeviceToHost,
                                     fs));
@@ -618,7 +637,8 @@ void dim0(tt_ctx* c, const Complex& cx, u32 maxdim, Dim0Out& out, u64 m_known) {
             const int last = round - first - 1;
             for (int q = 0; q <= last; ++q) total_hooks += h[2 * q + 1];
             known = h[2 * last];
-            if (h[2 * last + 1] == 0) break;
+            if (total_hooks == u64(n) - 1) break;                      // one component
+            if (h[2 * last + 1] == 0) known = 0;                       // nothing left to merge among the joined
         }
     }
     side.join();   // the forest's tree flags
