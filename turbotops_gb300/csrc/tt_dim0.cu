@@ -102,7 +102,8 @@ __global__ void k_edge_count(Rows rows, u32 n, f32 thr, u64* __restrict__ cnt, u
     for (u32 v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += warps) {
         const u64 b = rows.begin(v), e = rows.end(v);
         u32 c = 0;
-        for (u64 t0 = b; t0 < e; t0 += 32) {
+#pragma unroll 4
+        for (u64 t0 = b; t0 < e; t0 += 32) {   // (unrolled: several row loads in flight)
             bool keep = false;
             if (t0 + lane < e) {
                 u32 u;
@@ -141,10 +142,12 @@ __global__ void k_edge_count(Rows rows, u32 n, f32 thr, u64* __restrict__ cnt, u
 // Kept edges in a fixed order: position p = off[v] + rank in row runs over
 // edge indices in increasing order (rows ascending, u ascending within a
 // row). Entry q (q = m - 1 - p for the Ripser order, idx descending; q = p
-// for the RedZeD order, idx ascending) gets sort key dbits << 32 | q and
-// idx. A stable sort on the dbits then yields (d, idx) in the filtration
-// order: the ties keep the order of q.
-template <typename Rows>
+// for the RedZeD order, idx ascending) gets its filtration key (DIRECT:
+// packed layout), or sort key dbits << 32 | q and, beside it, idx. A stable
+// sort on the dbits then yields (d, idx) in the filtration order: the ties
+// keep the order of q. DIRECT saves k_edge_pack's gather and scatter by q
+// (43 M edges of 12,000 points: 3.9 ms) where nothing needs the positions q.
+template <typename Rows, bool DIRECT>
 __global__ void k_edge_fill(Rows rows, u32 n, f32 thr, const u64* __restrict__ off, u64 m, int redzed,
                             u64* __restrict__ skey, u64* __restrict__ sidx, u32* __restrict__ err) {
     pdl_wait();
@@ -155,6 +158,7 @@ __global__ void k_edge_fill(Rows rows, u32 n, f32 thr, const u64* __restrict__ o
         const u64 b = rows.begin(v), e = rows.end(v);
         const u64 vbase = u64(v) * (v - 1) / 2;
         u64 base = off[v];
+#pragma unroll 4
         for (u64 t0 = b; t0 < e; t0 += 32) {
             bool keep = false;
             u32 u = 0;
@@ -168,8 +172,13 @@ __global__ void k_edge_fill(Rows rows, u32 n, f32 thr, const u64* __restrict__ o
                 const u64 p = base + __popc(bal & ((1u << lane) - 1));
                 if (p < m) {
                     const u64 q = redzed ? p : m - 1 - p;
-                    skey[q] = (u64(__float_as_uint(d)) << 32) | q;
-                    sidx[q] = vbase + u;
+                    if constexpr (DIRECT) {
+                        const u64 idx = vbase + u;
+                        skey[q] = (u64(__float_as_uint(d)) << kIdxBits) | (redzed ? idx : kIdxMask - idx);
+                    } else {
+                        skey[q] = (u64(__float_as_uint(d)) << 32) | q;
+                        sidx[q] = vbase + u;
+                    }
                 } else if (err) {
                     atomicOr(err, 1u);   // more kept edges than the caller announced
                 }
@@ -198,6 +207,160 @@ __global__ void k_edge_pack(const u64* __restrict__ skey, const u64* __restrict_
     }
 }
 
+// The scan's result for one edge in a word: the first cofacet's vertex (NOV
+// >> 2: none), whether the edge is apparent, whether the cofacet has a
+// zero-apparent facet.
+constexpr u32 kAppNone = NOV >> 2, kAppApparent = 1u << 30, kAppEm = 1u << 31;
+constexpr u32 kAppNear = 64;    // candidates a lane tests before its warp takes the edge over
+constexpr u32 kAppStep = 8;     // ... in steps (loads in flight)
+constexpr u32 kAppProbe = 32;   // candidates of the emergent probe a lane tests itself
+
+// Is there a vertex w > t, other than f0 and f1, with both lengths to f0 and
+// f1 at most cap? Whole-warp scan of w in (t, hi).
+__device__ __forceinline__ bool warp_any_above(const DenseCx& cx, u32 f0, u32 f1, f32 cap, u32 t, u32 hi) {
+    const u32 lane = threadIdx.x & 31;
+    const f32* r0 = cx.mat + u64(f0) * cx.n;
+    const f32* r1 = cx.mat + u64(f1) * cx.n;
+    for (int64_t top = hi; top > int64_t(t) + 1; top -= 32) {
+        const int64_t w = top - 32 + lane;
+        const bool ok = w > int64_t(t) && u32(w) != f0 && u32(w) != f1 && r0[w] <= cap && r1[w] <= cap;
+        if (__any_sync(0xffffffffu, ok)) return true;
+    }
+    return false;
+}
+
+// Apparent / emergent scan of a dense complex, edge by edge in index order:
+// res[idx] for every kept edge idx = (a, b), a > b.
+// One warp takes 32 edges of row a (lane = b): the candidates w run down
+// from n - 1, D[a][w] is one address for the warp and D[w][b] (= D[b][w], the
+// matrix is symmetric bit for bit) one row segment, so an iteration tests 32
+// edges with two coalesced loads from rows that all warps read (the top rows
+// stay in L1 / L2). An edge of typical length has a cofacet among the first
+// few candidates; the edges that none of the first kAppNear fits (short ones)
+// are finished by the whole warp, 32 candidates at a time. A warp for each
+// edge from the start spent its time on per-edge overhead and on random rows:
+// 43 M edges of 12,000 points took 16.9 ms, this takes 5.3 (3,000 lattice
+// points in R^4 under L1: 0.85 and 0.33 ms). Bound by load latency (L1 / L2).
+// Beside that order there is no dependence on the sorted keys: the results
+// are gathered by index when the columns are emitted.
+__global__ void __launch_bounds__(256)
+    k_apparent_pairs(const f32* __restrict__ mat, u32 n, f32 thr, u32* __restrict__ res) {
+    pdl_wait();
+    pdl_trigger();
+    const DenseCx cx{mat, n};
+    const u32 lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const u32 b0 = blockIdx.x * 32, b = b0 + lane;
+    for (u32 a = blockIdx.y * 8 + wid; a < n; a += gridDim.y * 8) {
+        if (b0 >= a) continue;   // warp-uniform
+        const f32* ra = mat + u64(a) * n;
+        const u32 bl = min(b, n - 1);   // lanes past the row read in bounds
+        const f32 d = b < a ? ra[b] : INFINITY;
+        const bool kept = b < a && d <= thr;
+        if (!__any_sync(0xffffffffu, kept)) continue;
+        u32 w = NOV;
+        f32 da = 0.0f, db = 0.0f;   // lengths (a, w), (b, w)
+        u32 hi = n;                 // candidates at and above hi are tested
+        const u32 lo = n > kAppNear ? n - kAppNear : 0u;
+        bool open = kept;
+        while (hi > lo && __any_sync(0xffffffffu, open)) {
+            f32 va[kAppStep], vb[kAppStep];
+#pragma unroll
+            for (u32 q = 0; q < kAppStep; ++q) {
+                const u32 c = hi > q ? hi - 1 - q : 0u;
+                va[q] = ra[c];
+                vb[q] = mat[u64(c) * n + bl];
+            }
+#pragma unroll
+            for (u32 q = 0; q < kAppStep; ++q) {
+                const u32 c = hi - 1 - q;
+                if (open && hi > q && va[q] <= d && vb[q] <= d && c != a && c != b) {
+                    w = c;
+                    da = va[q];
+                    db = vb[q];
+                    open = false;
+                }
+            }
+            hi = hi > kAppStep ? hi - kAppStep : 0u;
+        }
+        // the edges still open: the whole warp, one after the other
+        for (u32 rest = __ballot_sync(0xffffffffu, open); hi && rest; rest &= rest - 1) {
+            const int src = __ffs(rest) - 1;
+            const u32 eb = b0 + src;
+            const f32 ed = __shfl_sync(0xffffffffu, d, src);
+            const f32* rb = mat + u64(eb) * n;
+            u32 found = NOV;
+            for (int64_t top = hi; top > 0 && found == NOV; top -= 128) {
+                f32 xa[4], xb[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int64_t c = top - 32 * (q + 1) + lane;
+                    xa[q] = c >= 0 ? ra[c] : INFINITY;
+                    xb[q] = c >= 0 ? rb[c] : INFINITY;
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int64_t c = top - 32 * (q + 1) + lane;
+                    const bool ok = c >= 0 && xa[q] <= ed && xb[q] <= ed && u32(c) != a && u32(c) != eb;
+                    const u32 bal = __ballot_sync(0xffffffffu, ok);
+                    if (found == NOV && bal) found = u32(top - 32 * (q + 1) + (31 - __clz(bal)));
+                }
+            }
+            if (int(lane) == src && found != NOV) {
+                w = found;
+                da = ra[found];
+                db = rb[found];
+            }
+        }
+        // The cofacet's zero facet: the first, in ascending index order, of
+        // its edges with length d (tri_zero_facet's order; (a, b) is one of
+        // the three). Another edge than (a, b) only where lengths tie; the
+        // emergent probe then asks whether that facet's own first cofacet is
+        // this triangle, that is, whether no vertex above the third one fits.
+        bool apparent = false, em = false, ask = false;
+        u32 f0 = 0, f1 = 0, third = 0;
+        if (kept && w != NOV) {
+            u32 c0 = a, c1 = b, c2 = w;
+            sort3(c0, c1, c2);
+            auto len = [&](u32 u, u32 v) -> f32 {
+                if (u != w && v != w) return d;
+                return u == a || v == a ? da : db;
+            };
+            if (len(c1, c2) == d) f0 = c1, f1 = c2, third = c0;
+            else if (len(c0, c2) == d) f0 = c0, f1 = c2, third = c1;
+            else f0 = c0, f1 = c1, third = c2;
+            apparent = f0 != w && f1 != w;
+            ask = !apparent;
+            em = ask;
+        }
+        if (__any_sync(0xffffffffu, ask)) {
+            u32 c = n;   // candidates at and above c are tested
+            if (ask) {
+                const u32 stop = max(third + 1, n > kAppProbe ? n - kAppProbe : 0u);
+                while (c > stop) {
+                    --c;
+                    if (c != f0 && c != f1 && mat[u64(c) * n + f0] <= d && mat[u64(c) * n + f1] <= d) {
+                        em = false;
+                        break;
+                    }
+                }
+            }
+            const bool more = ask && em && c > third + 1;
+            for (u32 rest = __ballot_sync(0xffffffffu, more); rest; rest &= rest - 1) {
+                const int src = __ffs(rest) - 1;
+                const bool any = warp_any_above(cx, __shfl_sync(0xffffffffu, f0, src), __shfl_sync(0xffffffffu, f1, src),
+                                                __shfl_sync(0xffffffffu, d, src), __shfl_sync(0xffffffffu, third, src),
+                                                __shfl_sync(0xffffffffu, c, src));
+                if (int(lane) == src) em = !any;
+            }
+        }
+        if (kept)
+            res[u64(a) * (a - 1) / 2 + b] =
+                (w == NOV ? kAppNone : w) | (apparent ? kAppApparent : 0u) | (em ? kAppEm : 0u);
+    }
+}
+
+// (The wide key layout, more than kPackedMaxN vertices: a warp for each sorted
+// edge, results by its sorted position.)
 __global__ void k_apparent_dense(const f32* __restrict__ mat, u32 n, const u64* __restrict__ keys, EdgeFmt fmt, u64 m,
                                  u8* __restrict__ app, u32* __restrict__ emw, u8* __restrict__ emf) {
     pdl_wait();
@@ -413,53 +576,111 @@ __global__ void k_bv_flatten(const u32* __restrict__ parent, u32* __restrict__ c
 // --------------------------------------------------------------------------
 // Ordered compaction of H0 bars and columns.
 // --------------------------------------------------------------------------
-// One flag word per edge: finite H0 bar << 32 | column (m < 2^32, so one
-// scan counts both without a carry between the halves).
-__global__ void k_flags_dim0(const u64* __restrict__ keys, EdgeFmt fmt, const u8* __restrict__ tree,
-                             const u8* __restrict__ app, u64 m, int want_cols, u64* __restrict__ f) {
+// Two passes over the sorted edges: counts per run of kRun edges (one warp a
+// run), a scan of the counts, then the emit with the ranks inside a run from
+// ballots. (Per-edge flag and offset words instead cost 32 bytes an edge of
+// traffic; what bounds the pair form's count now is its 4-byte gather by
+// edge index, 1.1 ms for 43 M edges; the emit takes 0.23.)
+// PAIRS: the apparent scan's results are k_apparent_pairs' words by edge
+// index, and the count pass writes the per-edge apparent flags from them;
+// otherwise they are per-edge arrays in sorted order.
+constexpr u32 kRun = 512;
+
+// cnt[run] = finite H0 bars << 32 | columns.
+template <bool PAIRS>
+__global__ void k_count_dim0(const u64* __restrict__ keys, EdgeFmt fmt, const u8* __restrict__ tree, u8* __restrict__ app,
+                             const u32* __restrict__ res, u64 m, int want_cols, u64* __restrict__ cnt) {
     pdl_wait();
     pdl_trigger();
-    for (u64 e = u64(blockIdx.x) * blockDim.x + threadIdx.x; e < m; e += u64(gridDim.x) * blockDim.x) {
-        const bool t = tree[e];
-        f[e] = (u64(t && fmt.d(keys[e]) > 0.0f) << 32) | u64(want_cols && !t && !(app && app[e]));
+    const u32 lane = threadIdx.x & 31;
+    const u64 runs = (m + kRun - 1) / kRun;
+    const u64 warps = (u64(gridDim.x) * blockDim.x) >> 5;
+    for (u64 run = (u64(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; run < runs; run += warps) {
+        u32 h = 0, cols = 0;
+#pragma unroll 4
+        for (u32 i = 0; i < kRun; i += 32) {
+            const u64 e = run * kRun + i + lane;
+            if (e >= m) continue;
+            const u64 key = keys[e];
+            const bool t = tree[e];
+            h += t && fmt.d(key) > 0.0f;
+            if (want_cols) {
+                bool ap;
+                if constexpr (PAIRS) {
+                    ap = (res[fmt.rips(key)] & kAppApparent) != 0;
+                    app[e] = ap;
+                } else {
+                    ap = app[e];
+                }
+                cols += !t && !ap;
+            }
+        }
+        h = __reduce_add_sync(0xffffffffu, h);
+        cols = __reduce_add_sync(0xffffffffu, cols);
+        if (lane == 0) cnt[run] = (u64(h) << 32) | cols;
     }
 }
 
+// off: the exclusive scan of cnt (m < 2^32: one sum counts both without a
+// carry between the halves), tot its total.
+template <bool PAIRS>
 __global__ void k_emit_dim0(const u64* __restrict__ keys, EdgeFmt fmt, const u8* __restrict__ tree,
-                            const u8* __restrict__ app,
-                            const u32* __restrict__ emw, const u8* __restrict__ emf, u64 m, int want_cols,
-                            const u64* __restrict__ o2, const u64* __restrict__ tot,
+                            const u8* __restrict__ app, const u32* __restrict__ emw, const u8* __restrict__ emf, u64 m,
+                            int want_cols, const u64* __restrict__ off, const u64* __restrict__ tot,
                             f32* __restrict__ h0, u64* __restrict__ h0_edge, u64* __restrict__ cidx,
                             f32* __restrict__ cd, u64* __restrict__ emi, u8* __restrict__ emf_out) {
     pdl_wait();
     pdl_trigger();
+    const u32 lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
     const u64 ncols = tot[0] & 0xffffffffull;
-    for (u64 e = u64(blockIdx.x) * blockDim.x + threadIdx.x; e < m; e += u64(gridDim.x) * blockDim.x) {
-        const u64 key = keys[e];
-        const f32 d = fmt.d(key);
-        const bool t = tree[e];
-        const u64 oe = o2[e];   // exclusive counts: H0 bars << 32 | columns
-        if (t && d > 0.0f) {
-            h0[oe >> 32] = d;
-            h0_edge[oe >> 32] = fmt.rips(key);   // the bar's critical (death) edge
-        }
-        if (want_cols && !t && !(app && app[e])) {
-            const u64 o = ncols - 1 - (oe & 0xffffffffull);   // descending order (rips.hpp:867)
-            const u64 idx = fmt.rips(key);
-            cidx[o] = idx;
-            cd[o] = d;
-            const u32 w = emw[e];
-            if (w == NOV) {
-                emi[o] = kNone;
-                emf_out[o] = 0;
-            } else {
-                u32 a, b;
-                decode_edge(idx, a, b);
-                u32 c0 = a, c1 = b, c2 = w;
-                sort3(c0, c1, c2);
-                emi[o] = tri_idx(c0, c1, c2);
-                emf_out[o] = emf[e];
+    const u64 runs = (m + kRun - 1) / kRun;
+    const u64 warps = (u64(gridDim.x) * blockDim.x) >> 5;
+    for (u64 run = (u64(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; run < runs; run += warps) {
+        u64 oh = off[run] >> 32, oc = off[run] & 0xffffffffull;
+#pragma unroll 4
+        for (u32 i = 0; i < kRun; i += 32) {
+            const u64 e = run * kRun + i + lane;
+            const bool in = e < m;
+            const bool t = in && tree[e];
+            const bool col = in && want_cols && !t && !app[e];
+            const u64 key = in ? keys[e] : 0ull;
+            const f32 d = fmt.d(key);
+            const bool bar = t && d > 0.0f;
+            const u32 hb = __ballot_sync(0xffffffffu, bar), cb = __ballot_sync(0xffffffffu, col);
+            if (bar) {
+                const u64 o = oh + __popc(hb & lt);
+                h0[o] = d;
+                h0_edge[o] = fmt.rips(key);   // the bar's critical (death) edge
             }
+            if (col) {
+                const u64 o = ncols - 1 - (oc + __popc(cb & lt));   // descending order (rips.hpp:867)
+                const u64 idx = fmt.rips(key);
+                cidx[o] = idx;
+                cd[o] = d;
+                u32 w;
+                u8 em;
+                if constexpr (PAIRS) {
+                    const u32 r = emw[idx];
+                    w = (r & kAppNone) == kAppNone ? NOV : r & kAppNone;
+                    em = (r & kAppEm) != 0;
+                } else {
+                    w = emw[e];
+                    em = emf[e];
+                }
+                if (w == NOV) {
+                    emi[o] = kNone;
+                    emf_out[o] = 0;
+                } else {
+                    u32 a, b;
+                    decode_edge(idx, a, b);
+                    u32 c0 = a, c1 = b, c2 = w;
+                    sort3(c0, c1, c2);
+                    emi[o] = tri_idx(c0, c1, c2);
+                    emf_out[o] = em;
+                }
+            }
+            oh += __popc(hb);
+            oc += __popc(cb);
         }
     }
 }
@@ -487,7 +708,9 @@ inline u32 grid_for(u64 work, u32 per_block) {
 // sort takes all 31 distance bits, and a wrong count sets *err instead of
 // writing out of bounds.
 constexpr u64 kUnknownM = ~0ull;
-static u64 sorted_edge_keys(tt_ctx* c, const Complex& cx, int redzed, u64** keys_out, u64** eidx_out,
+// want_inv: S_EDGE_INV is needed (k_apparent_csr walks the edges in index
+// order); without it, packed keys are written by the fill itself.
+static u64 sorted_edge_keys(tt_ctx* c, const Complex& cx, int redzed, bool want_inv, u64** keys_out, u64** eidx_out,
                             u64 m_known = kUnknownM, u32* err = nullptr) {
     const u32 n = cx.n;
     u64 m = 0;
@@ -521,26 +744,36 @@ static u64 sorted_edge_keys(tt_ctx* c, const Complex& cx, int redzed, u64** keys
     if (m >= 0xffffffffull) invalid("gb300: more than 2^32 - 1 kept edges");
     u64* keys = c->arena.get<u64>(S_EDGE_KEYS, m + 1);
     const bool wide = n > kPackedMaxN;
+    const bool direct = !wide && !want_inv;
     *eidx_out = nullptr;
     if (m) {
-        u64* skey = c->arena.get<u64>(S_EDGE_SORT, m + 1);
-        u64* sidx = c->arena.get<u64>(S_EDGE_IDX, m + 1);
-        if (cx.mat)
-            launch_pdl(k_edge_fill<DenseRows>, g, 256, 0, c->stream, DenseRows{cx.mat, n}, n, cx.thr, off, m, redzed, skey,
-                       sidx, err);
-        else
-            launch_pdl(k_edge_fill<CsrRows>, g, 256, 0, c->stream, CsrRows{cx.rp, cx.ci, cx.w}, n, cx.thr, off, m, redzed,
-                       skey, sidx, err);
-        TT_LAUNCH("k_edge_fill");
         u64* kb = c->arena.get<u64>(S_SORT_A, m);
+        // direct: filled into whichever buffer the sort's passes bring back to `keys`
+        const bool odd = radix_passes(m, dbits) & 1;
+        u64* skey = !direct ? c->arena.get<u64>(S_EDGE_SORT, m + 1) : odd ? kb : keys;
+        u64* sidx = direct ? nullptr : c->arena.get<u64>(S_EDGE_IDX, m + 1);
+        auto fill = [&](auto rows, auto dir) {
+            launch_pdl(k_edge_fill<decltype(rows), decltype(dir)::value>, g, 256, 0, c->stream, rows, n, cx.thr, off, m,
+                       redzed, skey, sidx, err);
+        };
+        auto fill_rows = [&](auto rows) {
+            if (direct) fill(rows, std::true_type{});
+            else fill(rows, std::false_type{});
+        };
+        if (cx.mat) fill_rows(DenseRows{cx.mat, n});
+        else fill_rows(CsrRows{cx.rp, cx.ci, cx.w});
+        TT_LAUNCH("k_edge_fill");
         // a stable sort on the distance bits that differ (none: already in order)
-        const bool sw = dbits > 0 && radix_sort<u32>(c, skey, static_cast<u32*>(nullptr), m, kb,
-                                                     static_cast<u32*>(nullptr), dbits, 32);
-        u32* inv = c->arena.get<u32>(S_EDGE_INV, m + 1);
-        launch_pdl(k_edge_pack, grid_for(m, 256), 256, 0, c->stream, sw ? kb : skey, sidx, m, redzed, wide, keys, inv);
-        if (wide) *eidx_out = sidx;
-        TT_LAUNCH("k_edge_pack");
-        c->launches += 2;
+        const bool sw = dbits > 0 && radix_sort<u32>(c, skey, static_cast<u32*>(nullptr), m, direct && odd ? keys : kb,
+                                                     static_cast<u32*>(nullptr), dbits, direct ? kIdxBits : 32);
+        c->launches += 1;
+        if (!direct) {
+            u32* inv = c->arena.get<u32>(S_EDGE_INV, m + 1);
+            launch_pdl(k_edge_pack, grid_for(m, 256), 256, 0, c->stream, sw ? kb : skey, sidx, m, redzed, wide, keys, inv);
+            if (wide) *eidx_out = sidx;
+            TT_LAUNCH("k_edge_pack");
+            c->launches += 1;
+        }
     }
     *keys_out = keys;
     return m;
@@ -550,7 +783,9 @@ void dim0(tt_ctx* c, const Complex& cx, u32 maxdim, Dim0Out& out, u64 m_known) {
     out = Dim0Out{};
     u32* err = m_known != kUnknownM ? c->arena.get<u32>(S_DIM0_ERR, 4) : nullptr;
     if (err) TT_CUDA(cudaMemsetAsync(err, 0, sizeof(u32), c->stream));
-    const u64 m = sorted_edge_keys(c, cx, 0, &out.keys, &out.eidx, m_known, err);
+    // packed keys of a dense complex: the apparent scan goes by vertex pairs
+    const bool pairs = cx.mat && cx.n <= kPackedMaxN;
+    const u64 m = sorted_edge_keys(c, cx, 0, !pairs && maxdim >= 1, &out.keys, &out.eidx, m_known, err);
     const EdgeFmt fmt{out.eidx};
     out.m = m;
     if (m >= 0xffffffffull) invalid("gb300: more than 2^32 - 1 kept edges");
@@ -558,8 +793,9 @@ void dim0(tt_ctx* c, const Complex& cx, u32 maxdim, Dim0Out& out, u64 m_known) {
     // per-edge flags
     u8* app = c->arena.get<u8>(S_FLAGS, 2 * m + 16);
     u8* tree = app + m + 8;
-    u32* emw = c->arena.get<u32>(S_EDGE_TMP, m + 1);
-    u8* emf = c->arena.get<u8>(S_MISC2, m + 1);
+    // the apparent scan's results: a word a vertex pair, or arrays by sorted position
+    u32* emw = c->arena.get<u32>(S_EDGE_TMP, pairs ? u64(n) * (n - (n > 0)) / 2 + 1 : m + 1);
+    u8* emf = pairs ? nullptr : c->arena.get<u8>(S_MISC2, m + 1);
     TT_CUDA(cudaMemsetAsync(tree, 0, m + 1, c->stream));
     // The apparent/emergent scan and the spanning forest read the same sorted
     // edges and write disjoint flags. The forest's short rounds (and their
@@ -569,9 +805,11 @@ void dim0(tt_ctx* c, const Complex& cx, u32 maxdim, Dim0Out& out, u64 m_known) {
     SideScope side(c);
     const cudaStream_t fs = n ? side.fork() : c->stream;   // the forest's stream
     if (maxdim >= 1 && m) {
-        u32* inv = c->arena.get<u32>(S_EDGE_INV, m + 1);
         const cudaStream_t s = c->stream;
-        if (cx.mat)
+        if (pairs)
+            launch_pdl(k_apparent_pairs, dim3(div_up(n, 32), std::min<u32>(div_up(n, 8), 65535)), 256, 0, s, cx.mat, n,
+                       cx.thr, emw);
+        else if (cx.mat)
             launch_pdl(k_apparent_dense, grid_for(m * 32, 256), 256, 0, s, cx.mat, n, out.keys, fmt, m, app, emw, emf);
         else
             // six of the eight resident blocks an SM: the forest's short
@@ -579,7 +817,7 @@ void dim0(tt_ctx* c, const Complex& cx, u32 maxdim, Dim0Out& out, u64 m_known) {
             // wave of scan blocks to retire (measured: kNN front end of
             // 100,000 points, dim0 0.04 ms shorter than with all eight)
             launch_pdl(k_apparent_csr, std::min<u32>(grid_for(m, 256), 6 * kSMs), 256, 0, s, 
-                CsrCx{cx.rp, cx.ci, cx.w}, out.keys, fmt, inv, m, app, emw, emf);
+                CsrCx{cx.rp, cx.ci, cx.w}, out.keys, fmt, c->arena.get<u32>(S_EDGE_INV, m + 1), m, app, emw, emf);
         TT_LAUNCH("k_apparent");
         ++c->launches;
     }
@@ -644,13 +882,15 @@ void dim0(tt_ctx* c, const Complex& cx, u32 maxdim, Dim0Out& out, u64 m_known) {
     side.join();   // the forest's tree flags
     // ordered compaction of H0 deaths and columns
     const int want_cols = maxdim >= 1;
-    u64* f2 = c->arena.get<u64>(S_MISC0, 2 * m + 4);
-    u64* o2 = f2 + m + 2;
+    const u64 runs = (m + kRun - 1) / kRun;
+    u64* cnt = c->arena.get<u64>(S_MISC0, runs + 1);
     u64* tot = c->arena.get<u64>(S_COUNT, 4);
+    const u32 gr = grid_for(runs * 32, 256);
     if (m) {
-        launch_pdl(k_flags_dim0, grid_for(m, 256), 256, 0, c->stream, out.keys, fmt, tree, out.app, m, want_cols, f2);
-        TT_LAUNCH("k_flags_dim0");
-        scan_exclusive<u64>(c, f2, o2, m, tot);
+        if (pairs) launch_pdl(k_count_dim0<true>, gr, 256, 0, c->stream, out.keys, fmt, tree, app, emw, m, want_cols, cnt);
+        else launch_pdl(k_count_dim0<false>, gr, 256, 0, c->stream, out.keys, fmt, tree, app, emw, m, want_cols, cnt);
+        TT_LAUNCH("k_count_dim0");
+        scan_exclusive<u64>(c, cnt, cnt, runs, tot);
         c->launches += 1;
     } else {
         TT_CUDA(cudaMemsetAsync(tot, 0, sizeof(u64), c->stream));
@@ -666,9 +906,12 @@ void dim0(tt_ctx* c, const Complex& cx, u32 maxdim, Dim0Out& out, u64 m_known) {
         out.emf = c->arena.get<u8>(S_OUT4, ncols + 1);
         out.h0_edge = c->arena.get<u64>(S_OUT5, nh0 + 1);
         if (m) {
-            launch_pdl(k_emit_dim0, grid_for(m, 256), 256, 0, c->stream, out.keys, fmt, tree, out.app, emw, emf, m, want_cols,
-                                                                 o2, tot, out.h0, out.h0_edge, out.cidx, out.cd,
-                                                                 out.emi, out.emf);
+            auto go = [&](auto kernel) {
+                launch_pdl(kernel, gr, 256, 0, c->stream, out.keys, fmt, tree, app, emw, emf, m, want_cols, cnt, tot,
+                           out.h0, out.h0_edge, out.cidx, out.cd, out.emi, out.emf);
+            };
+            if (pairs) go(k_emit_dim0<true>);
+            else go(k_emit_dim0<false>);
             TT_LAUNCH("k_emit_dim0");
             ++c->launches;
         }
@@ -709,7 +952,7 @@ __global__ void k_emit_redzed(const u64* __restrict__ keys, EdgeFmt fmt, u64 m, 
 u64 redzed_edges(tt_ctx* c, const Complex& cx, f32* d, int32_t* verts, u64 cap) {
     u64* keys = nullptr;
     u64* eidx = nullptr;
-    const u64 m = sorted_edge_keys(c, cx, 1, &keys, &eidx);
+    const u64 m = sorted_edge_keys(c, cx, 1, false, &keys, &eidx);
     if (m && m <= cap) {
         k_emit_redzed<<<grid_for(m, 256), 256, 0, c->stream>>>(keys, EdgeFmt{eidx}, m, d, verts);
         TT_LAUNCH("k_emit_redzed");
@@ -723,7 +966,7 @@ u64 redzed_edges(tt_ctx* c, const Complex& cx, f32* d, int32_t* verts, u64 cap) 
 u64 redzed_edges_owned(tt_ctx* c, const Complex& cx, f32** d, int32_t** verts) {
     u64* keys = nullptr;
     u64* eidx = nullptr;
-    const u64 m = sorted_edge_keys(c, cx, 1, &keys, &eidx);
+    const u64 m = sorted_edge_keys(c, cx, 1, false, &keys, &eidx);
     *d = c->arena.get<f32>(S_RZ_D, m + 1);
     *verts = c->arena.get<int32_t>(S_RZ_V, 2 * m + 2);
     if (m) {

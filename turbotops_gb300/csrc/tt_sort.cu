@@ -474,6 +474,16 @@ void scan_exclusive(tt_ctx* c, const T* in, T* out, u64 n, T* total, int depth) 
 template void scan_exclusive<u64>(tt_ctx*, const u64*, u64*, u64, u64*, int);
 template void scan_exclusive<u32>(tt_ctx*, const u32*, u32*, u64, u32*, int);
 
+constexpr u64 kLocalMin = u64(1) << 22;   // keys from which the tile-local scatter pays (beyond L2)
+
+// Passes radix_sort makes over n keys for that many bits: an odd number
+// leaves the result in the other buffer.
+int radix_passes(u64 n, int bits) {
+    if (n <= 1 || bits <= 0) return 0;
+    const int maxbits = n >= kLocalMin ? RS_LBITS : RS_MAXBITS;
+    return (bits + maxbits - 1) / maxbits;
+}
+
 // Sorts keys[0..n) ascending (stable, with the optional payload). Returns the
 // buffers that hold the result: the caller's (keys, vals) or the arena
 // scratch (kbuf, vbuf) — 'swapped' tells which.
@@ -504,9 +514,8 @@ bool radix_sort(tt_ctx* c, u64* keys, V* vals, u64 n, u64* kbuf, V* vbuf, int fo
     // spread evenly over them (25 bits: 9 + 8 + 8; 11 bits: one pass). Inputs
     // far beyond L2 take digits of at most RS_LBITS bits and the local
     // scatter: more passes, each writing contiguous runs.
-    const bool local = n >= (u64(1) << 22);
-    const int maxbits = local ? RS_LBITS : RS_MAXBITS;
-    const int passes = (bits + maxbits - 1) / maxbits;
+    const bool local = n >= kLocalMin;
+    const int passes = radix_passes(n, bits);
     int shift = lo_bit;
     for (int q = 0; q < passes; ++q) {
         const int width = (lo_bit + bits - shift + (passes - q) - 1) / (passes - q);
