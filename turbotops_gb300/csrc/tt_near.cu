@@ -1,0 +1,189 @@
+// tt_near.cu — the spatial order of the ordered searches (tt_near.cuh).
+//
+// Up to 8 coordinates the points are sorted along a Morton curve: every
+// coordinate is mapped through a smooth distribution function of its sample
+// mean and deviation (so that Gaussian tails and uniform cubes both spread
+// evenly over the cells) and cut into 2^b cells, the b bits of the
+// coordinates interleaved: 22 bits in two radix passes (11 in one up to 8,192
+// points). Above 8 coordinates a few bits each no longer make compact cells;
+// the points are sorted by their nearest pivot instead (tt_knn.cu
+// pivot_order). Any order gives the same results; it only decides how many
+// tiles a query reads.
+#include "tt_near.cuh"
+
+namespace tt {
+namespace near {
+
+namespace {
+
+constexpr u32 kCodeDims = 8;
+constexpr u32 kSample = 4096;
+constexpr int kStatThreads = 256;
+
+// Mean and scale of every coordinate over at most kSample strided points:
+// st[k] = mean, st[8 + k] = 1.702 / deviation (the logistic curve with that
+// scale follows the normal distribution function within 0.01).
+__global__ void __launch_bounds__(kStatThreads) k_near_stats(const f32* __restrict__ x, u32 n, u32 dim,
+                                                            f32* __restrict__ st) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ f32 part[kStatThreads / 32][2];
+    const u32 cnt = min(n, kSample);
+    for (u32 k = 0; k < dim; ++k) {
+        const f32 c0 = x[k];   // sums relative to one point: no cancellation far from the origin
+        f32 s = 0.0f, s2 = 0.0f;
+        for (u32 i = threadIdx.x; i < cnt; i += kStatThreads) {
+            const f32 d = x[(u64(i) * n / cnt) * dim + k] - c0;
+            s += d;
+            s2 = fmaf(d, d, s2);
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            s += __shfl_xor_sync(0xffffffffu, s, o);
+            s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+        }
+        if ((threadIdx.x & 31) == 0) {
+            part[threadIdx.x >> 5][0] = s;
+            part[threadIdx.x >> 5][1] = s2;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            f32 a = 0.0f, b = 0.0f;
+            for (int w = 0; w < kStatThreads / 32; ++w) a += part[w][0], b += part[w][1];
+            const f32 m = a / f32(cnt), var = b / f32(cnt) - m * m;
+            st[k] = c0 + m;
+            st[kCodeDims + k] = var > 0.0f ? 1.702f * rsqrtf(var) : 0.0f;
+        }
+        __syncthreads();
+    }
+}
+
+// Morton code of every point, `bits` a coordinate (a non-finite coordinate
+// lands in some cell: the conversions saturate).
+__global__ void k_near_codes(const f32* __restrict__ x, u32 n, u32 dim, u32 bits, const f32* __restrict__ st,
+                             u64* __restrict__ key, u32* __restrict__ val) {
+    pdl_wait();
+    pdl_trigger();
+    const f32 cells = f32(1u << bits);
+    for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        u32 q[kCodeDims];
+#pragma unroll
+        for (u32 k = 0; k < kCodeDims; ++k) {
+            q[k] = 0;
+            if (k < dim) {
+                const f32 z = (x[u64(i) * dim + k] - st[k]) * st[kCodeDims + k];
+                const f32 u = cells / (1.0f + __expf(-z));
+                q[k] = min(__float2uint_rz(u), (1u << bits) - 1u);
+            }
+        }
+        u32 code = 0;
+        for (int b = int(bits) - 1; b >= 0; --b)
+#pragma unroll
+            for (u32 k = 0; k < kCodeDims; ++k)
+                if (k < dim) code = (code << 1) | ((q[k] >> b) & 1u);
+        key[i] = code;
+        val[i] = i;
+    }
+}
+
+// Float bits in an order that integer min / max follow (no NaN).
+__device__ __forceinline__ u32 ordered(f32 f) {
+    const u32 b = __float_as_uint(f);
+    return (b >> 31) ? ~b : b | 0x80000000u;
+}
+__device__ __forceinline__ f32 from_ordered(u32 o) { return __uint_as_float((o >> 31) ? o & 0x7fffffffu : ~o); }
+
+// Tile t: its 32 points' coordinates (coordinate-major, zero-padded to dp)
+// and ids, and its box (slots past n left out; a NaN leaves the coordinate
+// unbounded: linf's maximum drops it, so the point can be near). One warp a
+// tile.
+__global__ void __launch_bounds__(128) k_near_tiles(const f32* __restrict__ x, u32 n, u32 dim, u32 dp,
+                                                    const u32* __restrict__ perm, u32 ntiles, u32 tpad,
+                                                    f32* __restrict__ xt, u32* __restrict__ id, f32* __restrict__ box) {
+    pdl_wait();
+    pdl_trigger();
+    const u32 lane = threadIdx.x & 31, t = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (t >= ntiles) return;
+    const u32 p = t * kTile + lane;
+    const bool live = p < n;
+    const u32 src = live ? perm[p] : 0xffffffffu;
+    id[p] = src;
+    for (u32 k = 0; k < dp; ++k) {
+        const f32 v = live && k < dim ? x[u64(src) * dim + k] : 0.0f;
+        xt[(u64(t) * dp + k) * kTile + lane] = v;
+        const u32 lo = __reduce_min_sync(0xffffffffu, ordered(!live ? INFINITY : v == v ? v : -INFINITY));
+        const u32 hi = __reduce_max_sync(0xffffffffu, ordered(!live ? -INFINITY : v == v ? v : INFINITY));
+        if (lane == 0) {
+            box[u64(k) * tpad + t] = from_ordered(lo);
+            box[u64(dp + k) * tpad + t] = from_ordered(hi);
+        }
+    }
+}
+
+// Super tile s: the box of its (up to) 32 tiles' boxes. One warp each.
+__global__ void __launch_bounds__(128) k_near_super(const f32* __restrict__ tbox, u32 ntiles, u32 tpad, u32 nsup,
+                                                    u32 spad, u32 dp, f32* __restrict__ sbox) {
+    pdl_wait();
+    pdl_trigger();
+    const u32 lane = threadIdx.x & 31, s = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (s >= nsup) return;
+    const u32 t = s * 32 + lane;
+    for (u32 k = 0; k < dp; ++k) {
+        const u32 lo = __reduce_min_sync(0xffffffffu, ordered(t < ntiles ? tbox[u64(k) * tpad + t] : INFINITY));
+        const u32 hi = __reduce_max_sync(0xffffffffu, ordered(t < ntiles ? tbox[u64(dp + k) * tpad + t] : -INFINITY));
+        if (lane == 0) {
+            sbox[u64(k) * spad + s] = from_ordered(lo);
+            sbox[u64(dp + k) * spad + s] = from_ordered(hi);
+        }
+    }
+}
+
+}  // namespace
+
+// Slots: S_NEAR_X, S_NEAR_ID, S_NEAR_BOX (results); S_TC_KEYS, S_TC_VALS,
+// S_NEAR_ST and the radix sort's own while it runs.
+View near_order(tt_ctx* c, const f32* x, u32 n, u32 dim) {
+    View v;
+    const u32 dp = padded_dim(dim);
+    v.n = n;
+    v.ntiles = div_up(n, kTile);
+    v.nsup = div_up(v.ntiles, 32);
+    v.tpad = v.nsup * 32;
+    v.spad = div_up(v.nsup, 32) * 32;
+    const u32* perm;
+    if (dim <= kCodeDims) {
+        u64* key = c->arena.get<u64>(S_TC_KEYS, n);
+        u32* val = c->arena.get<u32>(S_TC_VALS, n);
+        f32* st = c->arena.get<f32>(S_NEAR_ST, 2 * kCodeDims);
+        const u32 bits = std::max<u32>(1, (n <= 8192 ? 11 : 22) / dim);
+        launch_pdl(k_near_stats, 1, kStatThreads, 0, c->stream, x, n, dim, st);
+        TT_LAUNCH("k_near_stats");
+        launch_pdl(k_near_codes, std::min<u32>(div_up(n, 256), 8 * u32(c->sms)), 256, 0, c->stream, x, n, dim, bits, st,
+                   key, val);
+        TT_LAUNCH("k_near_codes");
+        c->launches += 2;
+        u64* kb = c->arena.get<u64>(S_SORT_A, n);
+        u32* vb = c->arena.get<u32>(S_SORT_VA, n);
+        perm = radix_sort<u32>(c, key, val, n, kb, vb, int(bits * dim)) ? vb : val;
+    } else {
+        perm = pivot_order(c, x, n, dim);
+    }
+    f32* xt = c->arena.get<f32>(S_NEAR_X, u64(v.ntiles) * dp * kTile);
+    u32* id = c->arena.get<u32>(S_NEAR_ID, u64(v.ntiles) * kTile);
+    f32* tbox = c->arena.get<f32>(S_NEAR_BOX, 2 * u64(dp) * (v.tpad + v.spad));
+    f32* sbox = tbox + 2 * u64(dp) * v.tpad;
+    launch_pdl(k_near_tiles, div_up(v.ntiles, 4), 128, 0, c->stream, x, n, dim, dp, perm, v.ntiles, v.tpad, xt, id, tbox);
+    TT_LAUNCH("k_near_tiles");
+    launch_pdl(k_near_super, div_up(v.nsup, 4), 128, 0, c->stream, static_cast<const f32*>(tbox), v.ntiles, v.tpad,
+               v.nsup, v.spad, dp, sbox);
+    TT_LAUNCH("k_near_super");
+    c->launches += 2;
+    v.xt = xt;
+    v.id = id;
+    v.tbox = tbox;
+    v.sbox = sbox;
+    return v;
+}
+
+}  // namespace near
+}  // namespace tt
