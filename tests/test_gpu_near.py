@@ -92,3 +92,21 @@ def _radius_check(x, tau, metric):
     ("gauss", 1300, 3, float("inf")), ("far", 800, 3, 1.0), ("gauss", 520, 12, 4.0)])
 def test_radius(kind, n, dim, tau, metric):
     _radius_check(_cloud(kind, n, dim, n + dim), tau, metric)
+
+
+@pytest.mark.parametrize("metric", ["l2", "l1", "linf"])
+@pytest.mark.parametrize("kind,n,dim", [
+    ("gauss", 512, 3), ("gauss", 1025, 2), ("gmm", 1100, 8), ("gmm", 2100, 12), ("gmm", 4200, 16), ("gmm", 1500, 32),
+    ("gmm", 3000, 32), ("gmm", 1300, 50), ("gmm", 900, 64), ("grid", 2000, 3), ("grid", 1500, 2), ("same", 700, 3),
+    ("far", 1200, 3), ("uniform", 33000, 3)])
+def test_mst(kind, n, dim, metric):
+    """Sorted spanning-tree weights: the ordered rounds against rounds that scan every pair."""
+    x = dev(synth.uniform(n, dim, n) if kind == "uniform" else _cloud(kind, n, dim, n))
+    c = ctx()
+    a = bits(host(ops.mst_deaths(c, x, metric)))
+    c.check(c.L.tt_ctx_set_knn_mode(c.h, 1))
+    try:
+        b = bits(host(ops.mst_deaths(c, x, metric)))
+    finally:
+        c.check(c.L.tt_ctx_set_knn_mode(c.h, 0))
+    assert np.array_equal(a, b)

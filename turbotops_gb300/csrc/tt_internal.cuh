@@ -161,8 +161,10 @@ u64 assemble2(tt_ctx* c, const Complex& cx, const u64* keys, u64 m, const u64* p
               u64** cidx, f32** cd, u64* napp);
 
 // ---- tt_knn.cu
+namespace near { struct View; }
+// (order: the points' spatial order if the caller has it)
 void knn_exact(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, u32 k, u32* ids, f32* dists,
-               bool defer = false);
+               bool defer = false, const near::View* order = nullptr);
 const u32* pivot_order(tt_ctx* c, const f32* x, u32 n, u32 dim);   // the points sorted by nearest pivot
 double tc_gram_check(tt_ctx* c, u32 products, u64 seed);   // tt_knn_tc.cu
 void selftest_wait_timeout(tt_ctx* c, u32 polls);           // tt_diag.cu

@@ -343,8 +343,7 @@ static constexpr u32 kNearMin = 512;
 static bool near_applicable(u32 n, u32 dim, int kind) {
     return kind != M_LP && n >= kNearMin && dim >= 1 && dim <= near::kMaxDim;
 }
-static void near_lists(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, u32 k, u32* ids, f32* dists) {
-    const near::View v = near::near_order(c, x, n, dim);
+static void near_lists(tt_ctx* c, const near::View& v, u32 dim, int kind, u32 k, u32* ids, f32* dists) {
     switch (kind) {
         case M_L1: near::near_knn<M_L1>(c, v, dim, k, ids, dists); break;
         case M_L2: near::near_knn<M_L2>(c, v, dim, k, ids, dists); break;
@@ -352,7 +351,8 @@ static void near_lists(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, u32 k,
     }
 }
 
-void knn_exact(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, u32 k, u32* ids, f32* dists, bool defer) {
+void knn_exact(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, u32 k, u32* ids, f32* dists, bool defer,
+               const near::View* order_known) {
     if (k == 0 || n < 2) return;
     // L2 in R^32: the tensor-core Gram filter (tt_knn_tc.cu) unless the
     // context asks for the exhaustive scan; both give the same lists
@@ -361,7 +361,7 @@ void knn_exact(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, u32 k, 
         return;
     }
     if (c->knn_mode == 0 && near_applicable(n, dim, kind) && k <= 32) {
-        near_lists(c, x, n, dim, kind, k, ids, dists);
+        near_lists(c, order_known ? *order_known : near::near_order(c, x, n, dim), dim, kind, k, ids, dists);
         if (!defer) TT_CUDA(cudaStreamSynchronize(c->stream));
         return;
     }

@@ -13,8 +13,8 @@
 // after at most ceil(log2 n) rounds one tree remains. The deaths are then
 // sorted by a radix sort on their float bits.
 //
-// Above kKnnMin points the rounds start from each point's K nearest
-// neighbours (one exact kNN pass; the tensor-core filter for L2 in R^32):
+// From kOrderMin points (L1, L2, Linf; kKnnMin for Lp) the rounds start from
+// each point's K nearest neighbours (one exact kNN pass):
 // the first list entry in another component is the point's nearest foreign
 // point (the list holds the K smallest (d, j) of all points), and a point
 // whose whole list lies in its own component has no foreign edge shorter than
@@ -23,7 +23,12 @@
 // component's other points, so only those interior points are scanned (a
 // listed subset of queries) before the per-component minima are taken:
 // every round's proposals are the same as with a scan of every point.
-#include "tt_internal.cuh"
+// The scan goes through the points in spatial order (tt_near.cuh
+// k_near_foreign): it leaves out the tiles of the query's own component and
+// those whose box is farther than the component's best proposal so far.
+// 100,000 points of a 16-Gaussian mixture in R^32, L2: the scans of six
+// rounds took 82 ms as exhaustive ones (up to 35.7 ms a round, FP32 issue).
+#include "tt_near.cuh"
 
 namespace tt {
 
@@ -36,7 +41,8 @@ namespace {
 
 constexpr u32 kNoD = 0xffffffffu;   // no proposal (above every float's bits)
 constexpr u32 kKnnK = 16;           // neighbours a point keeps for the rounds
-constexpr u32 kKnnMin = 4096;       // fewer points: every round scans every point
+constexpr u32 kKnnMin = 4096;       // Lp, fewer points: every round scans every point
+constexpr u32 kOrderMin = 512;      // L1, L2, Linf, fewer points: the same (one scan costs less than the order's launches)
 
 // From each point's list (ascending (d, id), K entries): the first entry in
 // another component is its proposal, d bits << 32 | j; with none, near[i] =
@@ -80,11 +86,13 @@ __global__ void k_mst_init(u32* __restrict__ comp, u32* __restrict__ parent, u32
 }
 
 // Per component: the smallest distance bits among its points' proposals ...
-__global__ void k_mst_min_d(const u32* __restrict__ comp, const unsigned long long* __restrict__ near,
-                            u32* __restrict__ bd, u32 n) {
+__global__ void k_mst_min_d(const u32* __restrict__ comp, const unsigned long long* __restrict__ near, u32* bd, u32 n) {
     for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const u64 k = near[i];
-        if (k != ~0ull) atomicMin(&bd[comp[i]], u32(k >> 32));
+        if (k == ~0ull) continue;
+        // (most offers of a large component are above its best already: a load decides those)
+        u32* b = bd + comp[i];
+        if (*reinterpret_cast<volatile u32*>(b) > u32(k >> 32)) atomicMin(b, u32(k >> 32));
     }
 }
 
@@ -146,19 +154,28 @@ u64 mst_deaths(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, f32* de
     u64* bi = c->arena.get<u64>(S_UF_WORK, n + 1);
     u32* bd = c->arena.get<u32>(S_UF_WORK2, n + 1);
     // the lists first (the kNN stage's own scratch is free again after it)
-    const bool lists = n >= kKnnMin;
+    const bool ordered = kind != M_LP && n >= kOrderMin && dim >= 1 && dim <= near::kMaxDim && c->knn_mode != 1;
+    const bool lists = ordered || n >= kKnnMin;
     const u32 K = std::min<u32>(kKnnK, n - 1);
     u32* kid = nullptr;
     f32* kd = nullptr;
+    near::View v;
+    u32 *cpos = nullptr, *tcomp = nullptr, *scomp = nullptr;
+    if (ordered) {
+        v = near::near_order(c, x, n, dim);
+        cpos = c->arena.get<u32>(S_MST_C, u64(v.ntiles) * (near::kTile + 1) + v.nsup);
+        tcomp = cpos + u64(v.ntiles) * near::kTile;
+        scomp = tcomp + v.ntiles;
+    }
     if (lists) {
         kid = c->arena.get<u32>(S_KNN_I, u64(n) * K + 1);
         kd = c->arena.get<f32>(S_KNN_D, u64(n) * K + 1);
-        knn_exact(c, x, n, dim, kind, p, K, kid, kd, false);
+        knn_exact(c, x, n, dim, kind, p, K, kid, kd, false, ordered ? &v : nullptr);
         settle_finite(c);   // a pending check of the points: a NaN leaves a list short
     }
     u32* kb = lists ? c->arena.get<u32>(S_MST_KB, n + 1) : nullptr;
-    u32* qlist = lists ? c->arena.get<u32>(S_MST_Q, n + 2) : nullptr;
-    u32* nq = lists ? qlist + n + 1 : nullptr;
+    u32* qlist = lists ? c->arena.get<u32>(S_MST_Q, u64(n) + 2 + near::kTile) : nullptr;
+    u32* nq = lists ? qlist + n + near::kTile + 1 : nullptr;
     u32* cnt = c->arena.get<u32>(S_MISC1, 4);
     u32* err = device_error_word(c);
     k_mst_init<<<grid_for(n), 256, 0, c->stream>>>(comp, parent, bd, bi, n);
@@ -169,10 +186,22 @@ u64 mst_deaths(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, f32* de
         if (lists) {
             k_mst_knn_near<<<grid_for(n), 256, 0, c->stream>>>(kid, kd, K, comp, near, kb, n);
             k_mst_min_d<<<grid_for(n), 256, 0, c->stream>>>(comp, near, bd, n);
-            TT_CUDA(cudaMemsetAsync(nq, 0, sizeof(u32), c->stream));
-            k_mst_flag<<<grid_for(n), 256, 0, c->stream>>>(near, kb, comp, bd, qlist, nq, n);
-            c->launches += 3;
-            foreign_nearest(c, x, n, dim, kind, p, comp, near, err, qlist, nq);
+            c->launches += 2;
+            if (ordered) {
+                near::near_components(c, v, comp, cpos, tcomp, scomp);
+                near::near_queries(c, v, dim, cpos, near, kb, bd, qlist, nq);
+                auto go = [&](auto kd_) {
+                    near::near_foreign<decltype(kd_)::value>(c, v, dim, cpos, tcomp, scomp, qlist, nq, bd, near);
+                };
+                if (kind == M_L1) go(std::integral_constant<int, M_L1>{});
+                else if (kind == M_L2) go(std::integral_constant<int, M_L2>{});
+                else go(std::integral_constant<int, M_LINF>{});
+            } else {
+                TT_CUDA(cudaMemsetAsync(nq, 0, sizeof(u32), c->stream));
+                k_mst_flag<<<grid_for(n), 256, 0, c->stream>>>(near, kb, comp, bd, qlist, nq, n);
+                c->launches += 1;
+                foreign_nearest(c, x, n, dim, kind, p, comp, near, err, qlist, nq);
+            }
         } else {
             foreign_nearest(c, x, n, dim, kind, p, comp, near, err);
         }

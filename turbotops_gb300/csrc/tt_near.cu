@@ -138,7 +138,72 @@ __global__ void __launch_bounds__(128) k_near_super(const f32* __restrict__ tbox
     }
 }
 
+// A block takes a super tile, a warp a tile of it.
+__global__ void __launch_bounds__(1024) k_near_components(const u32* __restrict__ id, u32 ntiles,
+                                                          const u32* __restrict__ comp, u32* __restrict__ cpos,
+                                                          u32* __restrict__ tcomp, u32* __restrict__ scomp) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ u32 lo[32], hi[32];
+    const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5, t = blockIdx.x * 32 + w;
+    u32 a = 0xffffffffu, b = 0;   // smallest and largest component of the tile
+    if (t < ntiles) {
+        const u32 i = id[t * kTile + lane];
+        const u32 cc = i != 0xffffffffu ? comp[i] : 0xffffffffu;
+        cpos[t * kTile + lane] = cc;
+        a = __reduce_min_sync(0xffffffffu, cc);
+        b = __reduce_max_sync(0xffffffffu, i != 0xffffffffu ? cc : 0u);
+        if (lane == 0) tcomp[t] = a == b ? a : 0xfffffffeu;
+    }
+    if (lane == 0) lo[w] = a, hi[w] = b;
+    __syncthreads();
+    if (w == 0) {
+        a = __reduce_min_sync(0xffffffffu, lo[lane]);
+        b = __reduce_max_sync(0xffffffffu, hi[lane]);
+        if (lane == 0) scomp[blockIdx.x] = a == b ? a : 0xfffffffeu;
+    }
+}
+
+__global__ void __launch_bounds__(256) k_near_queries(const u32* __restrict__ id, u32 ntiles,
+                                                      const u32* __restrict__ cpos,
+                                                      const unsigned long long* __restrict__ near,
+                                                      const u32* __restrict__ kb, const u32* __restrict__ bd, u32 qw,
+                                                      u32* __restrict__ qlist, u32* __restrict__ nq) {
+    pdl_wait();
+    pdl_trigger();
+    const u32 lane = threadIdx.x & 31;
+    const u32 warps = (gridDim.x * blockDim.x) >> 5;
+    for (u32 t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < ntiles; t += warps) {
+        const u32 p = t * kTile + lane, i = id[p];
+        const bool ask = i != 0xffffffffu && (!kb || (near[i] == ~0ull && kb[i] <= bd[cpos[p]]));
+        const u32 m = __ballot_sync(0xffffffffu, ask);
+        if (!m) continue;
+        const u32 cnt = __popc(m), room = (cnt + qw - 1) / qw * qw;
+        u32 base = 0;
+        if (lane == 0) base = atomicAdd(nq, room);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        const u32 o = __popc(m & ((1u << lane) - 1u));
+        if (ask) qlist[base + o] = p;
+        if (lane >= cnt && lane < room) qlist[base + lane] = 0xffffffffu;
+    }
+}
+
 }  // namespace
+
+void near_components(tt_ctx* c, const View& v, const u32* comp, u32* cpos, u32* tcomp, u32* scomp) {
+    launch_pdl(k_near_components, v.nsup, 1024, 0, c->stream, v.id, v.ntiles, comp, cpos, tcomp, scomp);
+    TT_LAUNCH("k_near_components");
+    ++c->launches;
+}
+
+void near_queries(tt_ctx* c, const View& v, u32 dim, const u32* cpos, const unsigned long long* near, const u32* kb,
+                  const u32* bd, u32* qlist, u32* nq) {
+    TT_CUDA(cudaMemsetAsync(nq, 0, sizeof(u32), c->stream));
+    launch_pdl(k_near_queries, std::min<u32>(div_up(v.ntiles, 8), 8 * u32(c->sms)), 256, 0, c->stream, v.id, v.ntiles,
+               cpos, near, kb, bd, queries_per_warp(padded_dim(dim)), qlist, nq);
+    TT_LAUNCH("k_near_queries");
+    ++c->launches;
+}
 
 // Slots: S_NEAR_X, S_NEAR_ID, S_NEAR_BOX (results); S_TC_KEYS, S_TC_VALS,
 // S_NEAR_ST and the radix sort's own while it runs.

@@ -57,6 +57,9 @@ inline u32 padded_dim(u32 dim) {
     return dim <= 4 ? (dim < 2 ? 2 : dim) : dim <= 8 ? 8 : dim <= 16 ? 16 : dim <= 32 ? 32 : dim <= 48 ? 48 : 64;
 }
 
+// Queries a warp takes at once (tt_near.cuh's header).
+constexpr u32 queries_per_warp(u32 dp) { return dp <= 4 ? 1 : dp <= 8 ? 2 : dp <= 16 ? 4 : 8; }
+
 // tt_near.cu
 View near_order(tt_ctx* c, const f32* x, u32 n, u32 dim);
 
@@ -68,6 +71,19 @@ void near_radius_count(tt_ctx* c, const View& v, u32 dim, f32 tau, u64* cnt, u32
 template <int KIND>
 void near_radius_fill(tt_ctx* c, const View& v, u32 dim, f32 tau, const u64* rp, u32* ci, f32* w);
 constexpr u32 kRadiusRow = 1024;   // longest row the fill sorts
+// One round's proposals of the listed queries (k_near_foreign).
+template <int KIND>
+void near_foreign(tt_ctx* c, const View& v, u32 dim, const u32* cpos, const u32* tcomp, const u32* scomp,
+                  const u32* qlist, const u32* nq, u32* bd, unsigned long long* near);
+// Components in the points' order: cpos[position], and the component a tile
+// or a super tile shares (tt_near.cu).
+void near_components(tt_ctx* c, const View& v, const u32* comp, u32* cpos, u32* tcomp, u32* scomp);
+// The queries of a round, listed by position in whole groups of
+// queries_per_warp (~0 fills a group up), *nq the list's length: the points
+// without a proposal whose kb (K-th neighbour's distance bits; null: every
+// point) does not exceed their component's best so far.
+void near_queries(tt_ctx* c, const View& v, u32 dim, const u32* cpos, const unsigned long long* near, const u32* kb,
+                  const u32* bd, u32* qlist, u32* nq);
 
 #ifdef TT_NEAR_IMPL
 
@@ -138,10 +154,16 @@ __device__ __forceinline__ f32 box_bound(const f32* __restrict__ box, u32 pad, u
     });
 }
 
+// No tile is left out beforehand.
+struct SkipNone {
+    __device__ __forceinline__ bool tile(u32) const { return false; }
+    __device__ __forceinline__ bool super(u32) const { return false; }
+};
+
 // Walks the tiles in reach of the warp's queries; visit(tile, coordinates,
 // candidate id) tests one tile and returns whether a bound may have dropped.
-template <int KIND, int DP, int CH, int QW, typename Visit>
-__device__ __forceinline__ void walk(const View& v, WarpQ<DP, QW>& W, u32 home, Visit&& visit) {
+template <int KIND, int DP, int CH, int QW, typename Visit, typename Skip = SkipNone>
+__device__ __forceinline__ void walk(const View& v, WarpQ<DP, QW>& W, u32 home, Visit&& visit, Skip skip = Skip{}) {
     const u32 lane = threadIdx.x & 31;
     auto group_thr = [&]() -> f32 {   // the largest bound (-1: none)
         f32 m = -1.0f;
@@ -162,7 +184,7 @@ __device__ __forceinline__ void walk(const View& v, WarpQ<DP, QW>& W, u32 home, 
         return visit(tile, c, __ldg(v.id + tile * kTile + lane));
     };
     f32 thr = group_thr();
-    if (load_visit(home)) thr = group_thr();
+    if (!skip.tile(home) && load_visit(home)) thr = group_thr();
     const u32 s0 = home / 32;
     // The closest open box of 32 held one a lane (bound bits; ~0: done). The
     // bounds are >= +0, so their bits order like them.
@@ -175,20 +197,22 @@ __device__ __forceinline__ void walk(const View& v, WarpQ<DP, QW>& W, u32 home, 
     auto descend = [&](u32 s) {
         const u32 t = s * 32 + lane;
         u32 b = 0xffffffffu;
-        if (t < v.ntiles && t != home) b = __float_as_uint(box_bound<KIND, DP, CH, QW>(v.tbox, v.tpad, t, W));
+        if (t < v.ntiles && t != home && !skip.tile(t))
+            b = __float_as_uint(box_bound<KIND, DP, CH, QW>(v.tbox, v.tpad, t, W));
         u32 src;
         while (closest(b, src)) {
             if (lane == src) b = 0xffffffffu;
             if (load_visit(s * 32 + src)) thr = group_thr();
         }
     };
-    descend(s0);
+    if (!skip.super(s0)) descend(s0);
     const u32 rounds = (v.nsup + 31) / 32, r0 = s0 / 32;
     for (u32 r = 0; r < rounds; ++r) {   // the home round first
         const u32 base = (r == 0 ? r0 : r <= r0 ? r - 1 : r) * 32;
         const u32 s = base + lane;
         u32 b = 0xffffffffu;
-        if (s < v.nsup && s != s0) b = __float_as_uint(box_bound<KIND, DP, CH, QW>(v.sbox, v.spad, s, W));
+        if (s < v.nsup && s != s0 && !skip.super(s))
+            b = __float_as_uint(box_bound<KIND, DP, CH, QW>(v.sbox, v.spad, s, W));
         u32 src;
         while (closest(b, src)) {
             if (lane == src) b = 0xffffffffu;
@@ -329,6 +353,114 @@ __global__ void __launch_bounds__(32 * kWarps)
     }
 }
 
+// ---- nearest point of another component -------------------------------------
+// One Borůvka round's proposals (tt_mst.cu): for every listed query (positions
+// in the order, `qlist`, ~0 entries skipped) its minimum (distance, id) over
+// the points of other components, near[id] = distance bits << 32 | id. A
+// tile, or a super tile, whose points all share the queries' component is left
+// out (tcomp, scomp: the shared component, or kMixed).
+// Only a component's best proposal counts, so a query starts from the bound
+// bd[component], the best its component has so far (distance bits), takes up
+// what other warps find meanwhile and publishes its own: candidates above the
+// bound cannot be the component's minimum, those at the bound still compete by
+// edge index. A query without a candidate within the bound leaves ~0.
+constexpr u32 kMixed = 0xfffffffeu, kNoComp = 0xffffffffu;
+
+struct SkipComp {
+    const u32* tcomp;
+    const u32* scomp;
+    u32 comp;   // the queries' shared component, or kNoComp
+    __device__ __forceinline__ bool tile(u32 t) const { return __ldg(tcomp + t) == comp; }
+    __device__ __forceinline__ bool super(u32 s) const { return __ldg(scomp + s) == comp; }
+};
+
+template <int KIND, int DP, int CH, int QW>
+__global__ void __launch_bounds__(32 * kWarps)
+    k_near_foreign(View v, const u32* __restrict__ cpos, const u32* __restrict__ tcomp, const u32* __restrict__ scomp,
+                   const u32* __restrict__ qlist, const u32* __restrict__ nq, u32* bd,
+                   unsigned long long* __restrict__ near) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ WarpQ<DP, QW> sw[kWarps];
+    __shared__ u64 sbest[kWarps][QW];
+    __shared__ u32 scq[kWarps][QW];
+    const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const u32 g0 = (blockIdx.x * kWarps + w) * QW;
+    if (g0 >= *nq) return;
+    WarpQ<DP, QW>& W = sw[w];
+    u64(&best)[QW] = sbest[w];
+    u32(&cq)[QW] = scq[w];
+    u32 mypos = 0xffffffffu, mycomp = kNoComp;
+    if (lane < QW) {
+        mypos = qlist[g0 + lane];   // (the list is padded to whole groups)
+        const bool in = mypos != 0xffffffffu;
+        mycomp = in ? cpos[mypos] : kNoComp;
+        const u32 b = in ? *reinterpret_cast<volatile u32*>(bd + mycomp) : 0u;
+        cq[lane] = mycomp;
+        best[lane] = in ? (u64(b) << 32) | 0xffffffffu : 0ull;
+        W.own[lane] = in ? v.id[mypos] : 0xffffffffu;
+        W.thr[lane] = !in ? -1.0f : b == 0xffffffffu ? INFINITY : bound_of<KIND>(__uint_as_float(b));
+    }
+    __syncwarp();
+    const u32 first = __ballot_sync(0xffffffffu, mypos != 0xffffffffu);   // never empty: lists start groups with a query
+    const u32 p_home = __shfl_sync(0xffffffffu, mypos, __ffs(first) - 1);
+    const u32 c_home = __shfl_sync(0xffffffffu, mycomp, __ffs(first) - 1);
+    const bool one = __all_sync(0xffffffffu, mypos == 0xffffffffu || mycomp == c_home);
+#pragma unroll 1
+    for (u32 e = lane; e < QW * DP; e += 32) {
+        const u32 q = e / DP, k = e % DP;
+        const u32 p = W.own[q] != 0xffffffffu ? qlist[g0 + q] : p_home;   // (a missing query repeats the first)
+        W.q[q][k] = v.xt[u64(p / kTile) * (DP * kTile) + k * kTile + p % kTile];
+    }
+    __syncwarp();
+    for (u32 k = lane; k < DP; k += 32) {
+        f32 lo = INFINITY, hi = -INFINITY;
+#pragma unroll
+        for (u32 q = 0; q < QW; ++q) {
+            const f32 x = W.q[q][k];
+            lo = x == x ? fminf(lo, x) : -INFINITY;
+            hi = x == x ? fmaxf(hi, x) : INFINITY;
+        }
+        W.lo[k] = lo;
+        W.hi[k] = hi;
+    }
+    __syncwarp();
+    const SkipComp skip{tcomp, scomp, one ? c_home : kNoComp};
+    walk<KIND, DP, CH, QW>(
+        v, W, p_home / kTile,
+        [&](u32 tile, const f32(&c)[DP], u32 cid) -> bool {
+            const u32 cc = __ldg(cpos + tile * kTile + lane);   // kNoComp past the points
+            bool dropped = false;
+#pragma unroll 1
+            for (u32 q = 0; q < QW; ++q) {
+                const f32 s = eval<KIND, DP, CH>(RegDiff<DP>{W.q[q], c});
+                const bool pass = cid != 0xffffffffu && cc != cq[q] && !(s > W.thr[q]);
+                if (!__any_sync(0xffffffffu, pass)) continue;
+                const f32 d = KIND == M_L2 ? __fsqrt_rn(s) : s;
+                const u64 old = best[q];
+                const u64 key = (u64(__float_as_uint(d)) << 32) | cid;
+                const bool take = pass && key < old;
+                const u32 dm = __reduce_min_sync(0xffffffffu, take ? u32(key >> 32) : 0xffffffffu);
+                const u32 im = __reduce_min_sync(0xffffffffu, take && u32(key >> 32) == dm ? cid : 0xffffffffu);
+                if (im == 0xffffffffu) continue;
+                if (lane == 0) {
+                    best[q] = (u64(dm) << 32) | im;
+                    // the component's bound: ours, or a smaller one found meanwhile
+                    const u32 seen = atomicMin(bd + cq[q], dm);
+                    W.thr[q] = bound_of<KIND>(__uint_as_float(min(seen, dm)));
+                }
+                __syncwarp();
+                dropped = true;
+            }
+            return dropped;
+        },
+        skip);
+    if (lane < QW && mypos != 0xffffffffu) {
+        const u64 k = best[lane];
+        near[W.own[lane]] = u32(k) == 0xffffffffu ? ~0ull : k;
+    }
+}
+
 // ---- radius graph -----------------------------------------------------------
 // Row lengths (cnt by original id) and the longest row, then the rows: a
 // warp collects a row's entries (id << 32 | distance bits) in shared memory,
@@ -415,7 +547,7 @@ __global__ void __launch_bounds__(32 * kWarps)
 
 template <int KIND, int DP, int CH>
 void launch_knn(tt_ctx* c, const View& v, u32 k, u32* ids, f32* dists) {
-    constexpr int QW = DP <= 4 ? 1 : DP <= 8 ? 2 : DP <= 16 ? 4 : 8;
+    constexpr int QW = queries_per_warp(DP);
     launch_pdl(k_near_knn<KIND, DP, CH, QW>, div_up(div_up(v.n, QW), kWarps), 32 * kWarps, 0, c->stream, v, k, ids, dists);
     TT_LAUNCH("k_near_knn");
     ++c->launches;
@@ -452,6 +584,19 @@ void near_knn(tt_ctx* c, const View& v, u32 dim, u32 k, u32* ids, f32* dists) {
     });
 }
 
+template <int KIND>
+void near_foreign(tt_ctx* c, const View& v, u32 dim, const u32* cpos, const u32* tcomp, const u32* scomp,
+                  const u32* qlist, const u32* nq, u32* bd, unsigned long long* near) {
+    with_dim<KIND>(dim, [&](auto dp, auto ch) {
+        constexpr int QW = queries_per_warp(decltype(dp)::value);
+        launch_pdl(k_near_foreign<KIND, decltype(dp)::value, decltype(ch)::value, QW>,
+                   div_up(u64(v.ntiles) * kTile, QW * kWarps), 32 * kWarps, 0, c->stream, v, cpos, tcomp, scomp, qlist,
+                   nq, bd, near);
+        TT_LAUNCH("k_near_foreign");
+        ++c->launches;
+    });
+}
+
 template <int KIND, bool FILL>
 void radius_pass(tt_ctx* c, const View& v, u32 dim, f32 tau, u64* cnt, u32* longest, const u64* rp, u32* ci, f32* w) {
     // the largest eval value a kept pair can have (host copy of bound_of)
@@ -481,6 +626,8 @@ void near_radius_fill(tt_ctx* c, const View& v, u32 dim, f32 tau, const u64* rp,
 
 #define TT_NEAR_INSTANTIATE(KIND)                                                     \
     template void near_knn<KIND>(tt_ctx*, const View&, u32, u32, u32*, f32*);         \
+    template void near_foreign<KIND>(tt_ctx*, const View&, u32, const u32*, const u32*, const u32*, const u32*, \
+                                     const u32*, u32*, unsigned long long*);          \
     template void near_radius_count<KIND>(tt_ctx*, const View&, u32, f32, u64*, u32*); \
     template void near_radius_fill<KIND>(tt_ctx*, const View&, u32, f32, const u64*, u32*, f32*);
 

@@ -203,7 +203,7 @@ void persistence_points(tt_ctx* c, const f32* x_h, u32 n, u32 dim, int kind, f32
         out.threshold = thr;
         out.edges = n ? n - 1 : 0;
         if (n == 0) return;
-        f32* deaths = c->arena.get<f32>(S_MISC0, n);
+        f32* deaths = c->arena.get<f32>(S_MST_OUT, n);
         mst_deaths(c, x, n, dim, kind, p, deaths);
         const auto d = to_host(c, deaths, n - 1);
         sync(c);
