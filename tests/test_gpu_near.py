@@ -65,6 +65,27 @@ def test_knn_hard_clouds(kind, n, dim, k):
         assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
 
 
+@pytest.mark.parametrize("metric", ["lp:1.1", "lp:1.5", "lp:2.5", "lp:3", "lp:4", "lp:7.3", "lp:12", "lp:64"])
+@pytest.mark.parametrize("kind,n,dim,k", [("gauss", 600, 2, 15), ("grid", 1025, 3, 16), ("gmm", 700, 8, 10),
+                                          ("gauss", 640, 13, 7), ("gmm", 1500, 32, 15), ("gmm", 520, 50, 32),
+                                          ("same", 530, 4, 5), ("far", 800, 5, 12), ("nonfinite", 700, 9, 8)])
+def test_knn_lp(kind, n, dim, k, metric):
+    """The Lp lists' power-sum filter and queue (exponents with and without a
+    closed power, below and above 8 coordinates)."""
+    x = _cloud(kind, n, dim, n)
+    a, b = _lists(x, k, metric, 0), _lists(x, k, metric, 1)
+    assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+
+
+@pytest.mark.parametrize("scale", [1e-30, 1e-12, 1e12, 1e25])
+def test_knn_lp_scales(scale):
+    """Powers that under- or overflow must filter nothing."""
+    x = (synth.gauss(600, 10, 3) * np.float32(scale)).astype(np.float32)
+    for metric in ("lp:1.5", "lp:3", "lp:9.5"):
+        a, b = _lists(x, 12, metric, 0), _lists(x, 12, metric, 1)
+        assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+
+
 @pytest.mark.parametrize("metric", ["l2", "l1", "linf"])
 def test_knn_large_with_ties(metric):
     x = np.concatenate([synth.grid(20000, 3, 30, 4), synth.uniform(13000, 3, 5) * np.float32(30)])   # past 1,024 tiles

@@ -28,8 +28,8 @@ __global__ void __launch_bounds__(kStatThreads) k_near_stats(const f32* __restri
     pdl_wait();
     pdl_trigger();
     __shared__ f32 part[kStatThreads / 32][2];
-    const u32 cnt = min(n, kSample);
-    for (u32 k = 0; k < dim; ++k) {
+    const u32 cnt = min(n, kSample), k = blockIdx.x;   // one block a coordinate
+    {
         const f32 c0 = x[k];   // sums relative to one point: no cancellation far from the origin
         f32 s = 0.0f, s2 = 0.0f;
         for (u32 i = threadIdx.x; i < cnt; i += kStatThreads) {
@@ -54,7 +54,6 @@ __global__ void __launch_bounds__(kStatThreads) k_near_stats(const f32* __restri
             st[k] = c0 + m;
             st[kCodeDims + k] = var > 0.0f ? 1.702f * rsqrtf(var) : 0.0f;
         }
-        __syncthreads();
     }
 }
 
@@ -99,7 +98,8 @@ __device__ __forceinline__ f32 from_ordered(u32 o) { return __uint_as_float((o >
 // tile.
 __global__ void __launch_bounds__(128) k_near_tiles(const f32* __restrict__ x, u32 n, u32 dim, u32 dp,
                                                     const u32* __restrict__ perm, u32 ntiles, u32 tpad,
-                                                    f32* __restrict__ xt, u32* __restrict__ id, f32* __restrict__ box) {
+                                                    f32* __restrict__ xt, u32* __restrict__ id, f32* __restrict__ box,
+                                                    f32* __restrict__ abox) {
     pdl_wait();
     pdl_trigger();
     const u32 lane = threadIdx.x & 31, t = blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -116,6 +116,10 @@ __global__ void __launch_bounds__(128) k_near_tiles(const f32* __restrict__ x, u
         if (lane == 0) {
             box[u64(k) * tpad + t] = from_ordered(lo);
             box[u64(dp + k) * tpad + t] = from_ordered(hi);
+            if (abox) {
+                abox[(u64(t) * 2) * dp + k] = from_ordered(lo);
+                abox[(u64(t) * 2 + 1) * dp + k] = from_ordered(hi);
+            }
         }
     }
 }
@@ -221,7 +225,7 @@ View near_order(tt_ctx* c, const f32* x, u32 n, u32 dim) {
         u32* val = c->arena.get<u32>(S_TC_VALS, n);
         f32* st = c->arena.get<f32>(S_NEAR_ST, 2 * kCodeDims);
         const u32 bits = std::max<u32>(1, (n <= 8192 ? 11 : 22) / dim);
-        launch_pdl(k_near_stats, 1, kStatThreads, 0, c->stream, x, n, dim, st);
+        launch_pdl(k_near_stats, dim, kStatThreads, 0, c->stream, x, n, dim, st);
         TT_LAUNCH("k_near_stats");
         launch_pdl(k_near_codes, std::min<u32>(div_up(n, 256), 8 * u32(c->sms)), 256, 0, c->stream, x, n, dim, bits, st,
                    key, val);
@@ -235,9 +239,12 @@ View near_order(tt_ctx* c, const f32* x, u32 n, u32 dim) {
     }
     f32* xt = c->arena.get<f32>(S_NEAR_X, u64(v.ntiles) * dp * kTile);
     u32* id = c->arena.get<u32>(S_NEAR_ID, u64(v.ntiles) * kTile);
-    f32* tbox = c->arena.get<f32>(S_NEAR_BOX, 2 * u64(dp) * (v.tpad + v.spad));
+    const bool directions = dp >= kProjectDim;
+    f32* tbox = c->arena.get<f32>(S_NEAR_BOX, 2 * u64(dp) * (v.tpad + v.spad + (directions ? v.ntiles : 0)));
     f32* sbox = tbox + 2 * u64(dp) * v.tpad;
-    launch_pdl(k_near_tiles, div_up(v.ntiles, 4), 128, 0, c->stream, x, n, dim, dp, perm, v.ntiles, v.tpad, xt, id, tbox);
+    f32* abox = directions ? sbox + 2 * u64(dp) * v.spad : nullptr;
+    launch_pdl(k_near_tiles, div_up(v.ntiles, 4), 128, 0, c->stream, x, n, dim, dp, perm, v.ntiles, v.tpad, xt, id, tbox,
+               abox);
     TT_LAUNCH("k_near_tiles");
     launch_pdl(k_near_super, div_up(v.nsup, 4), 128, 0, c->stream, static_cast<const f32*>(tbox), v.ntiles, v.tpad,
                v.nsup, v.spad, dp, sbox);
@@ -247,6 +254,7 @@ View near_order(tt_ctx* c, const f32* x, u32 n, u32 dim) {
     v.id = id;
     v.tbox = tbox;
     v.sbox = sbox;
+    v.abox = abox;
     return v;
 }
 

@@ -13,10 +13,11 @@
 // tiles at a time, then the 32 tiles of the super tile, one a lane, always
 // going on with the closest box, and stops where the closest one is farther
 // than every query's current bound. The candidates of a tile are held in
-// registers and tested against the QW queries in turn (their coordinates
-// broadcast from shared memory), so more queries a warp reuse the tile's
-// loads at the price of a larger common box: 1 up to four dimensions, 8 from
-// 32 on.
+// registers and tested against the queries that still need it, in turn (their
+// coordinates broadcast from shared memory), so more queries a warp reuse the
+// tile's loads: 1 up to four dimensions, 8 from 32 on. Every query is tested
+// against every box on its own (a common box of 8 points in R^32 reaches into
+// every cluster: 100,000 mixture points' foreign searches took 70 ms with it).
 //
 // Why no result changes. The lower bound of a box is the metric's own
 // lane-ordered float evaluation (tt_metric.cuh) of the gap vector
@@ -27,9 +28,11 @@
 // bit, with no margin. A box is skipped only when its bound exceeds the
 // query's bound strictly, the same test that drops a candidate, and all lists
 // compare (distance, id), so the visiting order does not matter.
-// (Non-integer and integer Lp have no such evaluation: they stay with the
-// exhaustive scan.) Coordinates padded with zeros beyond the dimension add
-// exact zeros to the sums, in the same lane order.
+// Coordinates padded with zeros beyond the dimension add exact zeros to the
+// sums, in the same lane order. Lp's own evaluation is long (a power series a
+// coordinate, a root in double precision) and not monotone in its last bits:
+// there boxes and candidates are tested on a fast power sum with a margin for
+// every error (below, k_near_knn_lp), and only the survivors are evaluated.
 #pragma once
 #include "tt_internal.cuh"
 #include "tt_metric.cuh"
@@ -40,6 +43,7 @@ namespace near {
 constexpr u32 kTile = 32;
 constexpr u32 kWarps = 4;          // warps a block
 constexpr u32 kMaxDim = 64;
+constexpr u32 kProjectDim = 16;    // padded dimensions from which tiles are also tested along a direction
 
 // The points in order. Boxes: lower corners, then upper ones, coordinate by
 // coordinate (row k: the tiles' values, padded to `tpad` / `spad` columns).
@@ -48,7 +52,9 @@ struct View {
     const u32* id = nullptr;   // [ntiles * 32]: original ids, ~0 past n
     const f32* tbox = nullptr;   // [2 * dp][tpad]
     const f32* sbox = nullptr;   // [2 * dp][spad]
+    const f32* abox = nullptr;   // [ntiles][2][dp]: the tiles' corners again (dp >= kProjectDim; else null)
     u32 n = 0, ntiles = 0, nsup = 0, tpad = 0, spad = 0;
+    f32 p = 2.0f;    // Lp: the exponent
 };
 
 // Coordinates held for `dim` (zero-padded) and 16-coordinate chunks in the
@@ -70,6 +76,8 @@ template <int KIND>
 void near_radius_count(tt_ctx* c, const View& v, u32 dim, f32 tau, u64* cnt, u32* longest);
 template <int KIND>
 void near_radius_fill(tt_ctx* c, const View& v, u32 dim, f32 tau, const u64* rp, u32* ci, f32* w);
+void near_knn_lp(tt_ctx* c, View v, u32 dim, f32 p, u32 k, u32* ids, f32* dists);   // p <= kLpMax
+constexpr f32 kLpMax = 64.0f;
 constexpr u32 kRadiusRow = 1024;   // longest row the fill sorts
 // One round's proposals of the listed queries (k_near_foreign).
 template <int KIND>
@@ -87,13 +95,48 @@ void near_queries(tt_ctx* c, const View& v, u32 dim, const u32* cpos, const unsi
 
 #ifdef TT_NEAR_IMPL
 
+// |d|^p, fast: exponents whose power is a product with at most one square root
+// (cls 1, 2), or exp2(p log2 |d|) on the special-function unit. 0 and
+// subnormal |d| give 0, NaN stays NaN.
+__device__ __forceinline__ f32 sqrt_fast(f32 x) {
+    f32 r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+template <int CLS>
+__device__ __forceinline__ f32 pow_abs(f32 d, f32 p) {
+    const f32 a = fabsf(d);
+    if constexpr (CLS == 1) return a * sqrt_fast(a);                // 1.5
+    else if constexpr (CLS == 2) return a * a * a;                  // 3
+    else {
+        f32 l, r;
+        asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(a));
+        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(p * l));
+        return r;
+    }
+}
+inline int pow_class(f32 p) { return p == 1.5f ? 1 : p == 3.0f ? 2 : 0; }
+// The kernels' kind for Lp names the class too: M_LP + 16 cls (a class for
+// each kernel: with a switch at every power the code outgrew the instruction
+// cache, and a fetch stall took 40 % of the cycles).
+constexpr bool is_lp(int kind) { return (kind & 15) == M_LP; }
+template <int KIND, int DP, typename Diff>
+__device__ __forceinline__ f32 pow_sum(const Diff& diff, f32 p) {
+    f32 t[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int k = 0; k < DP; ++k) t[k & 3] += pow_abs<(KIND >> 4)>(diff(k), p);
+    return (t[0] + t[1]) + (t[2] + t[3]);
+}
+
 // The metric's evaluation before its final root (L2: the squared sum), of
 // d[k] = q[k] - c[k], the query's coordinates in shared memory, the
 // candidate's (or the gap's) in registers; the lane order of tt_metric.cuh
 // for dim coordinates with CH = dim / 16 chunks, zero-padded to DP.
 template <int KIND, int DP, int CH, typename Diff>
-__device__ __forceinline__ f32 eval(const Diff& diff) {
-    if constexpr (KIND == M_LINF) {
+__device__ __forceinline__ f32 eval(const Diff& diff, f32 p = 2.0f) {
+    if constexpr (is_lp(KIND)) {
+        return pow_sum<KIND, DP>(diff, p);
+    } else if constexpr (KIND == M_LINF) {
         f32 m = 0.0f;
 #pragma unroll
         for (int k = 0; k < DP; ++k) m = fmaxf(m, fabsf(diff(k)));
@@ -132,6 +175,11 @@ __device__ __forceinline__ f32 bound_of(f32 d) {
     else return d;
 }
 
+// A distance that every point whose computed distance is at most d lies
+// within: the evaluations err by less than 2^-15 (L1, L2: 66 roundings of
+// 2^-24; Lp: k_near_knn_lp).
+__device__ __forceinline__ f32 bound_margin(f32 d) { return d * (1.0f + 0x1p-10f); }
+
 template <int DP>
 constexpr int row_floats() { return (DP + 3) / 4 * 4; }
 
@@ -139,19 +187,172 @@ constexpr int row_floats() { return (DP + 3) / 4 * 4; }
 template <int DP, int QW>
 struct WarpQ {
     alignas(16) f32 q[QW][row_floats<DP>()];
-    f32 lo[DP], hi[DP];
+    alignas(16) f32 qt[DP][QW];   // the same, coordinate-major
     f32 thr[QW];   // eval values above it cannot matter (negative: no query)
+    f32 bnd[QW];   // distances above it cannot matter (bound_margin)
     u32 own[QW];
 };
 
-// Lower bound of box column t against the warp's box.
+// The queries that box column t may matter to (a bit each), and the smallest
+// of their lower bounds in b (float bits; ~0: none). One query: its bound is
+// the metric's lane-ordered evaluation of the gaps. More: the sums run over
+// the coordinates for all queries at once (a box's corners are read once),
+// rounded down, and the margin 2^-16 covers the candidate sums' own rounding
+// (at most 66 operations, each within 2^-24).
 template <int KIND, int DP, int CH, int QW>
-__device__ __forceinline__ f32 box_bound(const f32* __restrict__ box, u32 pad, u32 t, const WarpQ<DP, QW>& W) {
-    return eval<KIND, DP, CH>([&](int k) -> f32 {
-        const f32 lo = __ldg(box + u64(k) * pad + t), hi = __ldg(box + u64(DP + k) * pad + t);
-        // (infinities that cancel leave a NaN, which fmaxf drops: a gap of 0)
-        return fmaxf(fmaxf(__fsub_rn(lo, W.hi[k]), __fsub_rn(W.lo[k], hi)), 0.0f);
-    });
+__device__ __forceinline__ u32 box_needs(const f32* __restrict__ box, u32 pad, u32 t, const WarpQ<DP, QW>& W, f32 p,
+                                         u32& b) {
+    // (infinities that cancel leave a NaN, which fmaxf drops: a gap of 0)
+    auto gap = [](f32 lo, f32 hi, f32 q) -> f32 { return fmaxf(fmaxf(__fsub_rn(lo, q), __fsub_rn(q, hi)), 0.0f); };
+    if constexpr (QW == 1) {
+        const f32 s = eval<KIND, DP, CH>(
+            [&](int k) -> f32 { return gap(__ldg(box + u64(k) * pad + t), __ldg(box + u64(DP + k) * pad + t), W.qt[k][0]); },
+            p);
+        b = __float_as_uint(s);
+        if (!(s > W.thr[0])) return 1u;
+        b = 0xffffffffu;
+        return 0u;
+    } else {
+        f32 s[QW];
+#pragma unroll
+        for (int q = 0; q < QW; ++q) s[q] = 0.0f;
+        auto add = [&](auto&& term) {
+#pragma unroll 4
+            for (int k = 0; k < DP; ++k) {
+                const f32 lo = __ldg(box + u64(k) * pad + t), hi = __ldg(box + u64(DP + k) * pad + t);
+#pragma unroll
+                for (int q = 0; q < QW; ++q) s[q] = term(gap(lo, hi, W.qt[k][q]), s[q]);
+            }
+        };
+        if constexpr (is_lp(KIND)) add([&](f32 g, f32 a) -> f32 { return a + pow_abs<(KIND >> 4)>(g, p); });
+        else if constexpr (KIND == M_LINF) add([](f32 g, f32 a) -> f32 { return fmaxf(a, g); });
+        else if constexpr (KIND == M_L2) add([](f32 g, f32 a) -> f32 { return __fmaf_rd(g, g, a); });
+        else add([](f32 g, f32 a) -> f32 { return __fadd_rd(a, g); });
+        u32 need = 0;
+        b = 0xffffffffu;
+#pragma unroll
+        for (int q = 0; q < QW; ++q) {
+            const f32 v = KIND == M_L2 || KIND == M_L1 ? s[q] * (1.0f - 0x1p-16f) : s[q];
+            if (!(v > W.thr[q])) {
+                need |= 1u << q;
+                b = min(b, __float_as_uint(s[q]));
+            }
+        }
+        return need;
+    }
+}
+
+// A box in many dimensions is a loose bound: 32 points of a Gaussian in R^32
+// spread over +-2 deviations along every axis, so the gaps between two
+// clusters nearly vanish one by one. Along the direction from the queries to
+// the tile the same points take up a tenth of the distance. For any u,
+// |u . (x - q)| <= |u|_p' |x - q|_p (Hoelder, 1/p + 1/p' = 1), so a tile whose
+// smallest u . x exceeds u . q by more than |u|_p' times a query's bound holds
+// nothing for it. u is the gradient of the distance at the vector D between
+// the centres (L2: D; L1: its signs; Lp: sign(D) |D|^(p-1)).
+// Rounding: u is what it is, as computed. The projections are sums relative
+// to the queries' centre g; each errs by at most (DP + 2) 2^-24 of
+// sum |u_k| |x_k - g_k|, which the box corners bound (err: 2^-17 times
+// both sides' sums); |u|_p' is taken 2^-9 up.
+// (100,000 mixture points in R^32: the foreign searches of a spanning tree 45
+// ms with the boxes alone, 30 ms with the directions; L1.5 lists: 20 % of the
+// tiles pass the boxes of 8 queries, 6 % are their own cluster's.)
+template <int DP>
+struct Direction {
+    alignas(16) f32 g[DP];     // the queries' centre
+    alignas(16) f32 u[DP];
+    f32 qy[DP][8];             // the queries relative to it, coordinate-major
+    f32 ext[DP];               // their largest |q_k - g_k|
+};
+struct NoDirection {};
+template <int KIND, int DP>
+constexpr bool projects() { return DP >= int(kProjectDim) && KIND != M_LINF; }
+template <int KIND, int DP>
+using DirectionOf = typename std::conditional<projects<KIND, DP>(), Direction<DP>, NoDirection>::type;
+
+template <int DP, int QW>
+__device__ __forceinline__ void init_direction(const WarpQ<DP, QW>& W, Direction<DP>& D) {
+    const u32 lane = threadIdx.x & 31;
+    for (u32 k = lane; k < DP; k += 32) {
+        f32 lo = W.qt[k][0], hi = lo;
+#pragma unroll
+        for (int q = 1; q < QW; ++q) lo = fminf(lo, W.qt[k][q]), hi = fmaxf(hi, W.qt[k][q]);
+        const f32 g = 0.5f * lo + 0.5f * hi;
+        f32 e = 0.0f;
+        D.g[k] = g;
+#pragma unroll
+        for (int q = 0; q < QW; ++q) {
+            const f32 y = __fsub_rn(W.qt[k][q], g);
+            D.qy[k][q] = y;
+            e = fmaxf(e, fabsf(y));
+        }
+        D.ext[k] = e;
+    }
+    __syncwarp();
+}
+
+__device__ __forceinline__ f32 warp_sum(f32 x) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
+
+// The queries of `need` that the tile (candidates c, one a lane; `live`: a
+// point) may still matter to.
+template <int KIND, int DP, int QW>
+__device__ __forceinline__ u32 project(const View& v, const WarpQ<DP, QW>& W, Direction<DP>& D, u32 tile,
+                                       const f32 (&c)[DP], bool live, u32 need) {
+    const u32 lane = threadIdx.x & 31;
+    f32 nrm = 0.0f, mag = 0.0f;
+#pragma unroll
+    for (int h = 0; h < (DP + 31) / 32; ++h) {
+        const u32 k = lane + 32 * h;
+        if (k < DP) {
+            const f32 lo = __ldg(v.abox + (u64(tile) * 2) * DP + k), hi = __ldg(v.abox + (u64(tile) * 2 + 1) * DP + k);
+            const f32 g = D.g[k];
+            const f32 d = (0.5f * lo + 0.5f * hi) - g;
+            f32 u, t;   // the direction, its term of |u|_p'
+            if constexpr (KIND == M_L2) {
+                u = d;
+                t = d * d;
+            } else if constexpr (KIND == M_L1) {
+                u = d < 0.0f ? -1.0f : 1.0f;
+                t = 0.0f;
+            } else {
+                u = copysignf(pow_abs<0>(d, v.p - 1.0f), d);
+                t = pow_abs<0>(u, v.p / (v.p - 1.0f));
+            }
+            D.u[k] = u;
+            nrm += t;
+            mag += fabsf(u) * (fmaxf(fabsf(lo - g), fabsf(hi - g)) + D.ext[k]);
+        }
+    }
+    nrm = warp_sum(nrm);
+    mag = warp_sum(mag);
+    if constexpr (KIND != M_L1)   // terms lost to underflow (each below 2^-126) must not matter
+        if (!(nrm >= 0x1p-100f)) return need;
+    if constexpr (KIND == M_L2) nrm = sqrtf(nrm);
+    else if constexpr (KIND == M_L1) nrm = 1.0f;
+    else nrm = pow_abs<0>(nrm, (v.p - 1.0f) / v.p);
+    nrm *= 1.0f + 0x1p-9f;
+    __syncwarp();
+    f32 pc[2] = {0.0f, 0.0f}, pq[2] = {0.0f, 0.0f};
+    const u32 ql = lane & 7u;
+#pragma unroll
+    for (int k = 0; k < DP; ++k) {
+        const f32 u = D.u[k];
+        pc[k & 1] = fmaf(u, __fsub_rn(c[k], D.g[k]), pc[k & 1]);
+        pq[k & 1] = fmaf(u, D.qy[k][ql], pq[k & 1]);
+    }
+    f32 m = pc[0] + pc[1];
+    m = live ? m : INFINITY;   // (a NaN candidate: kept below, the difference is NaN or too small)
+    const bool odd = __any_sync(0xffffffffu, live && !(m == m));
+#pragma unroll
+    for (int o = 16; o; o >>= 1) m = fminf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const f32 lead = (m - (pq[0] + pq[1])) - 0x1p-16f * mag;
+    const bool out = lane < QW && !odd && lead > nrm * W.bnd[lane < QW ? lane : 0] && lead < INFINITY;
+    __syncwarp();
+    return need & ~__ballot_sync(0xffffffffu, out);
 }
 
 // No tile is left out beforehand.
@@ -161,10 +362,13 @@ struct SkipNone {
 };
 
 // Walks the tiles in reach of the warp's queries; visit(tile, coordinates,
-// candidate id) tests one tile and returns whether a bound may have dropped.
+// candidate id, queries) tests one tile against the queries of a bit mask and
+// returns whether a bound may have dropped.
 template <int KIND, int DP, int CH, int QW, typename Visit, typename Skip = SkipNone>
-__device__ __forceinline__ void walk(const View& v, WarpQ<DP, QW>& W, u32 home, Visit&& visit, Skip skip = Skip{}) {
+__device__ __forceinline__ void walk(const View& v, WarpQ<DP, QW>& W, DirectionOf<KIND, DP>& D, u32 home, Visit&& visit,
+                                     Skip skip = Skip{}) {
     const u32 lane = threadIdx.x & 31;
+    if constexpr (projects<KIND, DP>()) init_direction<DP, QW>(W, D);
     auto group_thr = [&]() -> f32 {   // the largest bound (-1: none)
         f32 m = -1.0f;
         if constexpr (QW == 1) {
@@ -176,33 +380,40 @@ __device__ __forceinline__ void walk(const View& v, WarpQ<DP, QW>& W, u32 home, 
         }
         return m;
     };
-    auto load_visit = [&](u32 tile) -> bool {
+    auto load_visit = [&](u32 tile, u32 need) -> bool {
         f32 c[DP];
         const f32* xt = v.xt + u64(tile) * (DP * kTile) + lane;
 #pragma unroll
         for (int k = 0; k < DP; ++k) c[k] = __ldg(xt + k * kTile);
-        return visit(tile, c, __ldg(v.id + tile * kTile + lane));
+        const u32 cid = __ldg(v.id + tile * kTile + lane);
+        if constexpr (projects<KIND, DP>()) {
+            if (tile != home) {
+                need = project<KIND, DP, QW>(v, W, D, tile, c, cid != 0xffffffffu, need);
+                if (!need) return false;
+            }
+        }
+        return visit(tile, c, cid, need);
     };
     f32 thr = group_thr();
-    if (!skip.tile(home) && load_visit(home)) thr = group_thr();
+    if (!skip.tile(home) && load_visit(home, (1u << QW) - 1u)) thr = group_thr();
     const u32 s0 = home / 32;
     // The closest open box of 32 held one a lane (bound bits; ~0: done). The
     // bounds are >= +0, so their bits order like them.
     auto closest = [&](u32 b, u32& src) -> bool {
         const u32 m = __reduce_min_sync(0xffffffffu, b);
-        if (m == 0xffffffffu || __uint_as_float(m) > thr) return false;
+        if (m == 0xffffffffu || __uint_as_float(m) * (QW == 1 ? 1.0f : 1.0f - 0x1p-16f) > thr) return false;
         src = u32(__ffs(__ballot_sync(0xffffffffu, b == m)) - 1);
         return true;
     };
     auto descend = [&](u32 s) {
         const u32 t = s * 32 + lane;
-        u32 b = 0xffffffffu;
+        u32 b = 0xffffffffu, need = 0;
         if (t < v.ntiles && t != home && !skip.tile(t))
-            b = __float_as_uint(box_bound<KIND, DP, CH, QW>(v.tbox, v.tpad, t, W));
+            need = box_needs<KIND, DP, CH, QW>(v.tbox, v.tpad, t, W, v.p, b);
         u32 src;
         while (closest(b, src)) {
             if (lane == src) b = 0xffffffffu;
-            if (load_visit(s * 32 + src)) thr = group_thr();
+            if (load_visit(s * 32 + src, QW == 1 ? 1u : __shfl_sync(0xffffffffu, need, src))) thr = group_thr();
         }
     };
     if (!skip.super(s0)) descend(s0);
@@ -212,7 +423,7 @@ __device__ __forceinline__ void walk(const View& v, WarpQ<DP, QW>& W, u32 home, 
         const u32 s = base + lane;
         u32 b = 0xffffffffu;
         if (s < v.nsup && s != s0 && !skip.super(s))
-            b = __float_as_uint(box_bound<KIND, DP, CH, QW>(v.sbox, v.spad, s, W));
+            box_needs<KIND, DP, CH, QW>(v.sbox, v.spad, s, W, v.p, b);
         u32 src;
         while (closest(b, src)) {
             if (lane == src) b = 0xffffffffu;
@@ -228,25 +439,13 @@ __device__ __forceinline__ void load_queries(const View& v, u32 p0, f32 thr0, Wa
     const u32 lane = threadIdx.x & 31;
     for (u32 e = lane; e < QW * DP; e += 32) {
         const u32 q = e / DP, k = e % DP, p = p0 + q;
-        W.q[q][k] = p < v.n ? v.xt[u64(p / kTile) * (DP * kTile) + k * kTile + p % kTile] : 0.0f;
+        W.q[q][k] = W.qt[k][q] = p < v.n ? v.xt[u64(p / kTile) * (DP * kTile) + k * kTile + p % kTile] : 0.0f;
     }
     if (lane < QW) {
         const u32 p = p0 + lane;
         W.thr[lane] = p < v.n ? thr0 : -1.0f;
+        W.bnd[lane] = p < v.n ? INFINITY : 0.0f;
         W.own[lane] = p < v.n ? v.id[p] : 0xffffffffu;
-    }
-    __syncwarp();
-    for (u32 k = lane; k < DP; k += 32) {
-        f32 lo = INFINITY, hi = -INFINITY;
-#pragma unroll
-        for (u32 q = 0; q < QW; ++q)
-            if (p0 + q < v.n) {
-                const f32 x = W.q[q][k];
-                lo = x == x ? fminf(lo, x) : -INFINITY;   // (a NaN: unbounded, as in a tile's box)
-                hi = x == x ? fmaxf(hi, x) : INFINITY;
-            }
-        W.lo[k] = lo;
-        W.hi[k] = hi;
     }
     __syncwarp();
 }
@@ -302,12 +501,16 @@ __device__ __forceinline__ void merge_keys(u64& L, u64& kth, u32 k, u64 key, u32
     }
 }
 
+// 100,000 uniform points in R^3, k = 15, L2: 0.225 ms (exhaustive scan 31.55
+// ms); 20,011 x 8 Gaussian points, Linf, k = 10: 0.36 ms (2.9 ms). Latency
+// bound: the walk's loads and shuffles follow each other.
 template <int KIND, int DP, int CH, int QW>
 __global__ void __launch_bounds__(32 * kWarps)
     k_near_knn(View v, u32 k, u32* __restrict__ ids, f32* __restrict__ dists) {
     pdl_wait();
     pdl_trigger();
     __shared__ WarpQ<DP, QW> sw[kWarps];
+    __shared__ DirectionOf<KIND, DP> sd[projects<KIND, DP>() ? kWarps : 1];
     __shared__ u64 slist[kWarps][QW][32];
     const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const u32 p0 = (blockIdx.x * kWarps + w) * QW;
@@ -318,10 +521,11 @@ __global__ void __launch_bounds__(32 * kWarps)
 #pragma unroll
     for (int q = 0; q < QW; ++q) list[q][lane] = kEmpty;
     __syncwarp();
-    walk<KIND, DP, CH, QW>(v, W, p0 / kTile, [&](u32, const f32(&c)[DP], u32 cid) -> bool {
+    walk<KIND, DP, CH, QW>(v, W, sd[projects<KIND, DP>() ? w : 0], p0 / kTile, [&](u32, const f32(&c)[DP], u32 cid, u32 need) -> bool {
         bool dropped = false;
 #pragma unroll 1
-        for (u32 q = 0; q < QW; ++q) {
+        for (; need; need &= need - 1) {
+            const u32 q = QW == 1 ? 0u : u32(__ffs(need) - 1);
             const f32 s = eval<KIND, DP, CH>(RegDiff<DP>{W.q[q], c});
             const f32 tq = W.thr[q];
             // (past the points: id ~0; past the queries: bound -1)
@@ -335,12 +539,135 @@ __global__ void __launch_bounds__(32 * kWarps)
             if (!mask) continue;
             merge_keys(L, kth, k, key, mask);
             list[q][lane] = L;
-            if (lane == 0) W.thr[q] = bound_of<KIND>(__uint_as_float(u32(kth >> 32)));
+            if (lane == 0) {
+                const f32 dk = __uint_as_float(u32(kth >> 32));
+                W.thr[q] = bound_of<KIND>(dk);
+                if constexpr (projects<KIND, DP>()) W.bnd[q] = bound_margin(dk);
+            }
             __syncwarp();
             dropped = true;
         }
         return dropped;
     });
+#pragma unroll 1
+    for (u32 q = 0; q < QW; ++q) {
+        if (p0 + q >= v.n) break;
+        const u64 L = list[q][lane];
+        const u64 o = u64(W.own[q]) * k + lane;
+        if (lane < k) {
+            ids[o] = u32(L);
+            if (dists) dists[o] = __uint_as_float(u32(L >> 32));
+        }
+    }
+}
+
+// Lp lists. A candidate of a query with k-th distance B is evaluated exactly
+// when its power sum F = sum |d_k|^p (fast) is at most
+//   T = B^p (fast) (1 + (p + 1) 2^-12).
+// The reference's distance (lp_parts, lp_root) is M powf(s, 1/p) with s the
+// sum of its power series of |d_k| / M: the series' log2 (arguments above
+// 1e-30) errs by less than 2^-16, so a term by a factor within
+// 1 +- (p 2^-16 + 2^-18), the terms it clamps by less than 2^-126 of a sum
+// that is at least about 1, and the root by p 2^-22 of the power. F and T err by
+// p 2^-15 each (lg2.approx within 2^-22 of a logarithm below 128, ex2.approx
+// 2^-22, sums of 64 terms 2^-18). Together below p 2^-13.6 + 2^-16 for p <= kLpMax, a
+// third of the margin. T outside [2^-100, 2^100], where powers
+// under- or overflow, filters nothing. The gap vector of a box goes through the same sum: the power sums of the
+// coordinate differences, as rounded, are at least the gap's.
+// Survivors are queued and evaluated 32 at a time, one a lane, so that the
+// long exact path runs in full warps.
+// 100,000 x 32 mixture points, L1.5, k = 15: 13.5 ms, 2.1 instructions a cycle
+// (exhaustive scan with early exits: 390 ms). Bound by issue and the
+// special-function unit (one square root a coordinate).
+template <int KIND>
+__device__ __forceinline__ f32 lp_thr(f32 d, f32 p) {
+    if (!(d < INFINITY)) return INFINITY;
+    const f32 t = pow_abs<(KIND >> 4)>(d, p) * (1.0f + (p + 1.0f) * 0x1p-12f);
+    return t >= 0x1p-100f && t <= 0x1p100f ? t : INFINITY;
+}
+
+struct TileCol {   // coordinate k of one candidate
+    const f32* x;
+    __device__ __forceinline__ f32 operator()(u32 k) const { return __ldg(x + k * kTile); }
+};
+
+template <int KIND, int DP, int QW>
+__global__ void __launch_bounds__(32 * kWarps)
+    k_near_knn_lp(View v, u32 dim, u32 k, u32* __restrict__ ids, f32* __restrict__ dists) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ WarpQ<DP, QW> sw[kWarps];
+    __shared__ DirectionOf<KIND, DP> sd[projects<KIND, DP>() ? kWarps : 1];
+    __shared__ u64 slist[kWarps][QW][32];
+    __shared__ u32 spos[kWarps][64];   // survivors: position in the order, query (a ring)
+    __shared__ u8 sq[kWarps][64];
+    const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+    const u32 p0 = (blockIdx.x * kWarps + w) * QW;
+    if (p0 >= v.n) return;
+    WarpQ<DP, QW>& W = sw[w];
+    load_queries<DP, QW>(v, p0, INFINITY, W);
+    u64(&list)[QW][32] = slist[w];
+#pragma unroll
+    for (int q = 0; q < QW; ++q) list[q][lane] = kEmpty;
+    __syncwarp();
+    u32 head = 0, count = 0;
+    // evaluates the first `cnt` (at most 32) survivors
+    auto flush = [&](u32 cnt) {
+        __syncwarp();
+        const bool in = lane < cnt;
+        const u32 pos = in ? spos[w][(head + lane) & 63] : 0, q = in ? sq[w][(head + lane) & 63] : 0;
+        u64 key = ~0ull;
+        if (in) {
+            f32 M, sum;
+            lp_parts(Row{W.q[q]}, TileCol{v.xt + u64(pos / kTile) * (DP * kTile) + pos % kTile}, dim, v.p, M, sum);
+            const f32 bd = __uint_as_float(u32(list[q][k - 1] >> 32));
+            if (!(lp_root_lower(M, sum, v.p) > bd))
+                key = (u64(__float_as_uint(lp_root(M, sum, v.p))) << 32) | v.id[pos];
+        }
+        for (u32 open = __ballot_sync(0xffffffffu, key != ~0ull); open;) {
+            const u32 qq = __shfl_sync(0xffffffffu, q, __ffs(open) - 1);
+            const u32 all = __ballot_sync(0xffffffffu, q == qq) & open;
+            open &= ~all;
+            u64 L = list[qq][lane];
+            u64 kth = shfl64(L, k - 1);
+            const u32 mask = __ballot_sync(0xffffffffu, key < kth) & all;
+            if (!mask) continue;
+            merge_keys(L, kth, k, key, mask);
+            list[qq][lane] = L;
+            if (lane == 0) {
+                const f32 dk = __uint_as_float(u32(kth >> 32));
+                W.thr[qq] = lp_thr<KIND>(dk, v.p);
+                if constexpr (projects<KIND, DP>()) W.bnd[qq] = bound_margin(dk);
+            }
+            __syncwarp();
+        }
+        head += cnt;
+        count -= cnt;
+        __syncwarp();
+    };
+    walk<KIND, DP, 0, QW>(v, W, sd[projects<KIND, DP>() ? w : 0], p0 / kTile, [&](u32 tile, const f32(&c)[DP], u32 cid, u32 need) -> bool {
+        bool dropped = false;
+#pragma unroll 1
+        for (; need; need &= need - 1) {
+            const u32 q = QW == 1 ? 0u : u32(__ffs(need) - 1);
+            const f32 s = eval<KIND, DP, 0>(RegDiff<DP>{W.q[q], c}, v.p);
+            const bool pass = cid != W.own[q] && cid != 0xffffffffu && !(s > W.thr[q]);
+            const u32 m = __ballot_sync(0xffffffffu, pass);
+            if (!m) continue;
+            if (pass) {
+                const u32 o = (head + count + __popc(m & lt)) & 63;
+                spos[w][o] = tile * kTile + lane;
+                sq[w][o] = u8(q);
+            }
+            count += __popc(m);
+            if (count >= 32) {
+                flush(32);
+                dropped = true;
+            }
+        }
+        return dropped;
+    });
+    if (count) flush(count);
 #pragma unroll 1
     for (u32 q = 0; q < QW; ++q) {
         if (p0 + q >= v.n) break;
@@ -382,6 +709,7 @@ __global__ void __launch_bounds__(32 * kWarps)
     pdl_wait();
     pdl_trigger();
     __shared__ WarpQ<DP, QW> sw[kWarps];
+    __shared__ DirectionOf<KIND, DP> sd[projects<KIND, DP>() ? kWarps : 1];
     __shared__ u64 sbest[kWarps][QW];
     __shared__ u32 scq[kWarps][QW];
     const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -400,6 +728,7 @@ __global__ void __launch_bounds__(32 * kWarps)
         best[lane] = in ? (u64(b) << 32) | 0xffffffffu : 0ull;
         W.own[lane] = in ? v.id[mypos] : 0xffffffffu;
         W.thr[lane] = !in ? -1.0f : b == 0xffffffffu ? INFINITY : bound_of<KIND>(__uint_as_float(b));
+        W.bnd[lane] = !in ? 0.0f : b == 0xffffffffu ? INFINITY : bound_margin(__uint_as_float(b));
     }
     __syncwarp();
     const u32 first = __ballot_sync(0xffffffffu, mypos != 0xffffffffu);   // never empty: lists start groups with a query
@@ -410,29 +739,18 @@ __global__ void __launch_bounds__(32 * kWarps)
     for (u32 e = lane; e < QW * DP; e += 32) {
         const u32 q = e / DP, k = e % DP;
         const u32 p = W.own[q] != 0xffffffffu ? qlist[g0 + q] : p_home;   // (a missing query repeats the first)
-        W.q[q][k] = v.xt[u64(p / kTile) * (DP * kTile) + k * kTile + p % kTile];
-    }
-    __syncwarp();
-    for (u32 k = lane; k < DP; k += 32) {
-        f32 lo = INFINITY, hi = -INFINITY;
-#pragma unroll
-        for (u32 q = 0; q < QW; ++q) {
-            const f32 x = W.q[q][k];
-            lo = x == x ? fminf(lo, x) : -INFINITY;
-            hi = x == x ? fmaxf(hi, x) : INFINITY;
-        }
-        W.lo[k] = lo;
-        W.hi[k] = hi;
+        W.q[q][k] = W.qt[k][q] = v.xt[u64(p / kTile) * (DP * kTile) + k * kTile + p % kTile];
     }
     __syncwarp();
     const SkipComp skip{tcomp, scomp, one ? c_home : kNoComp};
     walk<KIND, DP, CH, QW>(
-        v, W, p_home / kTile,
-        [&](u32 tile, const f32(&c)[DP], u32 cid) -> bool {
+        v, W, sd[projects<KIND, DP>() ? w : 0], p_home / kTile,
+        [&](u32 tile, const f32(&c)[DP], u32 cid, u32 need) -> bool {
             const u32 cc = __ldg(cpos + tile * kTile + lane);   // kNoComp past the points
             bool dropped = false;
 #pragma unroll 1
-            for (u32 q = 0; q < QW; ++q) {
+            for (; need; need &= need - 1) {
+                const u32 q = QW == 1 ? 0u : u32(__ffs(need) - 1);
                 const f32 s = eval<KIND, DP, CH>(RegDiff<DP>{W.q[q], c});
                 const bool pass = cid != 0xffffffffu && cc != cq[q] && !(s > W.thr[q]);
                 if (!__any_sync(0xffffffffu, pass)) continue;
@@ -448,6 +766,7 @@ __global__ void __launch_bounds__(32 * kWarps)
                     // the component's bound: ours, or a smaller one found meanwhile
                     const u32 seen = atomicMin(bd + cq[q], dm);
                     W.thr[q] = bound_of<KIND>(__uint_as_float(min(seen, dm)));
+                    W.bnd[q] = bound_margin(__uint_as_float(min(seen, dm)));
                 }
                 __syncwarp();
                 dropped = true;
@@ -464,7 +783,9 @@ __global__ void __launch_bounds__(32 * kWarps)
 // ---- radius graph -----------------------------------------------------------
 // Row lengths (cnt by original id) and the longest row, then the rows: a
 // warp collects a row's entries (id << 32 | distance bits) in shared memory,
-// sorts them by id and writes the row.
+// sorts them by id and writes the row. 50,000 uniform points in R^3, 240
+// neighbours: count 0.14 ms, fill 0.48 ms (exhaustive scans 4.2 and 4.05 ms);
+// the fill is bound by its sort in shared memory.
 template <int KIND, int DP, int CH, bool FILL>
 __global__ void __launch_bounds__(32 * kWarps)
     k_near_radius(View v, f32 tau, f32 bound, u64* __restrict__ cnt, u32* __restrict__ longest,
@@ -472,6 +793,7 @@ __global__ void __launch_bounds__(32 * kWarps)
     pdl_wait();
     pdl_trigger();
     __shared__ WarpQ<DP, 1> sw[kWarps];
+    __shared__ DirectionOf<KIND, DP> sd[projects<KIND, DP>() ? kWarps : 1];
     __shared__ u64 srow[FILL ? kWarps : 1][FILL ? kRadiusRow : 1];
     const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const u32 p0 = blockIdx.x * kWarps + w;
@@ -480,7 +802,7 @@ __global__ void __launch_bounds__(32 * kWarps)
     load_queries<DP, 1>(v, p0, bound, W);
     u64* row = srow[FILL ? w : 0];
     u32 len = 0;
-    walk<KIND, DP, CH, 1>(v, W, p0 / kTile, [&](u32, const f32(&c)[DP], u32 cid) -> bool {
+    walk<KIND, DP, CH, 1>(v, W, sd[projects<KIND, DP>() ? w : 0], p0 / kTile, [&](u32, const f32(&c)[DP], u32 cid, u32) -> bool {
         const f32 s = eval<KIND, DP, CH>(RegDiff<DP>{W.q[0], c});
         bool pass = cid != W.own[0] && cid != 0xffffffffu && s <= bound;
         if (!__any_sync(0xffffffffu, pass)) return false;
@@ -558,7 +880,8 @@ template <int KIND, typename F>
 void with_dim(u32 dim, F&& f) {
     using std::integral_constant;
     auto go = [&](auto dp, auto ch) {
-        if constexpr (KIND == M_LINF) f(dp, integral_constant<int, 0>{});   // a max: no lane order
+        // (a max, and Lp's filter: no lane order)
+        if constexpr (KIND == M_LINF || is_lp(KIND)) f(dp, integral_constant<int, 0>{});
         else f(dp, ch);
     };
 #define TT_D(DP, CH) go(integral_constant<int, DP>{}, integral_constant<int, CH>{})
