@@ -26,6 +26,7 @@ def _clumps(n, seed):
 CASES = [("gauss", n, "inf") for n in (2, 3, 31, 32, 33, 64, 65, 72, 73, 129)]
 CASES += [("clumps", n, t) for n in (33, 97, 200, 400) for t in ("inf", "2.5")]
 CASES += [("grid", n, "inf") for n in (34, 100, 300)]        # ties: emergent probes past 32 candidates
+CASES += [("gauss", 2048, "inf"), ("clumps", 2048, "60"), ("gauss", 2049, "inf"), ("clumps", 2100, "60")]   # one block's forest, separate rounds
 CASES += [("same", 70, "inf"), ("gauss", 700, "0.35"), ("clumps", 700, "30")]   # m below and above 16 n
 
 

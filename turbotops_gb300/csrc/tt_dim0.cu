@@ -145,13 +145,15 @@ __global__ void k_edge_count(Rows rows, u32 n, f32 thr, u64* __restrict__ cnt, u
 // for the RedZeD order, idx ascending) gets its filtration key (DIRECT:
 // packed layout), or sort key dbits << 32 | q and, beside it, idx. A stable
 // sort on the dbits then yields (d, idx) in the filtration order: the ties
-// keep the order of q. DIRECT saves k_edge_pack's gather and scatter by q
+// keep the order of q. (m == kCountOnDevice: the count is off[n].) DIRECT saves k_edge_pack's gather and scatter by q
 // (43 M edges of 12,000 points: 3.9 ms) where nothing needs the positions q.
+constexpr u64 kCountOnDevice = ~0ull;
 template <typename Rows, bool DIRECT>
 __global__ void k_edge_fill(Rows rows, u32 n, f32 thr, const u64* __restrict__ off, u64 m, int redzed,
                             u64* __restrict__ skey, u64* __restrict__ sidx, u32* __restrict__ err) {
     pdl_wait();
     pdl_trigger();
+    if (m == kCountOnDevice) m = off[n];
     const int lane = threadIdx.x & 31;
     const u32 warps = (gridDim.x * blockDim.x) >> 5;
     for (u32 v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += warps) {
@@ -589,13 +591,20 @@ constexpr u32 kRun = 512;
 // cnt[run] = finite H0 bars << 32 | columns.
 template <bool PAIRS>
 __global__ void k_count_dim0(const u64* __restrict__ keys, EdgeFmt fmt, const u8* __restrict__ tree, u8* __restrict__ app,
-                             const u32* __restrict__ res, u64 m, int want_cols, u64* __restrict__ cnt) {
+                             const u32* __restrict__ res, u64 m, const u64* __restrict__ mdev, int want_cols,
+                             u64* __restrict__ cnt) {
     pdl_wait();
     pdl_trigger();
     const u32 lane = threadIdx.x & 31;
+    const u64 cap_runs = (m + kRun - 1) / kRun;   // runs past the count get zeros (the scan covers the capacity)
+    if (mdev) m = *mdev;
     const u64 runs = (m + kRun - 1) / kRun;
     const u64 warps = (u64(gridDim.x) * blockDim.x) >> 5;
-    for (u64 run = (u64(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; run < runs; run += warps) {
+    for (u64 run = (u64(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; run < cap_runs; run += warps) {
+        if (run >= runs) {
+            if (lane == 0) cnt[run] = 0;
+            continue;
+        }
         u32 h = 0, cols = 0;
 #pragma unroll 4
         for (u32 i = 0; i < kRun; i += 32) {
@@ -626,12 +635,13 @@ __global__ void k_count_dim0(const u64* __restrict__ keys, EdgeFmt fmt, const u8
 template <bool PAIRS>
 __global__ void k_emit_dim0(const u64* __restrict__ keys, EdgeFmt fmt, const u8* __restrict__ tree,
                             const u8* __restrict__ app, const u32* __restrict__ emw, const u8* __restrict__ emf, u64 m,
-                            int want_cols, const u64* __restrict__ off, const u64* __restrict__ tot,
+                            const u64* __restrict__ mdev, int want_cols, const u64* __restrict__ off, const u64* __restrict__ tot,
                             f32* __restrict__ h0, u64* __restrict__ h0_edge, u64* __restrict__ cidx,
                             f32* __restrict__ cd, u64* __restrict__ emi, u8* __restrict__ emf_out) {
     pdl_wait();
     pdl_trigger();
     const u32 lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
+    if (mdev) m = *mdev;
     const u64 ncols = tot[0] & 0xffffffffull;
     const u64 runs = (m + kRun - 1) / kRun;
     const u64 warps = (u64(gridDim.x) * blockDim.x) >> 5;
@@ -685,6 +695,109 @@ __global__ void k_emit_dim0(const u64* __restrict__ keys, EdgeFmt fmt, const u8*
     }
 }
 
+
+// --------------------------------------------------------------------------
+// The spanning forest of a small dense complex (n <= kSmallN) without a host
+// round trip: one block runs the Boruvka rounds on the shortest edges with
+// the components in shared memory, a filter keeps the later edges that still
+// join two components (usually none: the forest is complete), and the block
+// finishes with those. (The rounds of separate kernels cost three launches
+// and a share of a round trip each, whatever the size.)
+// --------------------------------------------------------------------------
+constexpr u32 kSmallN = 2048;
+constexpr u32 kForestThreads = 1024;
+
+// Edges: the ranks [0, min(*m, first)) when `first`, else list[0, *count).
+// st[0] = hooks so far, st[1] = live edges (the filter's list).
+__global__ void __launch_bounds__(kForestThreads) k_forest_block(const u64* __restrict__ keys, const u64* __restrict__ m,
+                                                                u32 first, const u32* __restrict__ list, u32 n,
+                                                                u32* __restrict__ comp_g, u8* __restrict__ tree,
+                                                                u32* __restrict__ st) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ u32 comp[kSmallN], parent[kSmallN], best[kSmallN];
+    __shared__ u32 hooked;
+    const u32 tid = threadIdx.x;
+    const u32 before = first ? 0u : st[0];
+    const u32 cnt = first ? u32(min(*m, u64(first))) : st[1];
+    if (!first && cnt == 0) return;
+    for (u32 v = tid; v < n; v += kForestThreads) {
+        const u32 c = first ? v : comp_g[v];
+        comp[v] = parent[v] = c;
+        best[v] = NOV;
+    }
+    if (tid == 0) hooked = 0;
+    __syncthreads();
+    const EdgeFmt fmt{};
+    for (;;) {
+        bool any = false;
+        for (u32 e = tid; e < cnt; e += kForestThreads) {
+            const u32 r = first ? e : list[e];
+            u32 a, b;
+            decode_edge(fmt.rips(keys[r]), a, b);
+            const u32 ca = comp[a], cb = comp[b];
+            if (ca == cb) continue;
+            any = true;
+            if (*reinterpret_cast<volatile u32*>(&best[ca]) > r) atomicMin(&best[ca], r);
+            if (*reinterpret_cast<volatile u32*>(&best[cb]) > r) atomicMin(&best[cb], r);
+        }
+        if (!__syncthreads_or(any)) break;
+        for (u32 c = tid; c < n; c += kForestThreads) {
+            const u32 r = best[c];
+            if (comp[c] != c || r == NOV) continue;
+            u32 a, b;
+            decode_edge(fmt.rips(keys[r]), a, b);
+            const u32 o = comp[a] == c ? comp[b] : comp[a];
+            tree[r] = 1;
+            if (best[o] == r && c < o) continue;   // mutual: o hooks onto c
+            parent[c] = o;
+            atomicAdd(&hooked, 1u);
+        }
+        __syncthreads();
+        for (u32 v = tid; v < n; v += kForestThreads) {
+            u32 r = parent[comp[v]];
+            for (u32 q = 0; parent[r] != r && q < n; ++q) r = parent[r];
+            comp[v] = r;
+        }
+        __syncthreads();
+        for (u32 v = tid; v < n; v += kForestThreads) {
+            parent[v] = comp[v];
+            best[v] = NOV;
+        }
+        __syncthreads();
+        if (before + hooked == n - 1) break;   // (shared, read after a barrier and next written after one)
+    }
+    __syncthreads();
+    for (u32 v = tid; v < n; v += kForestThreads) comp_g[v] = comp[v];
+    if (tid == 0) st[0] = before + hooked;
+}
+
+// The edges [first, *m) that join two components, unless the forest is
+// complete: list[0, st[1]).
+__global__ void k_forest_filter(const u64* __restrict__ keys, const u64* __restrict__ m, u32 first, u32 n,
+                                const u32* __restrict__ comp, u32* __restrict__ list, u32* __restrict__ st) {
+    pdl_wait();
+    pdl_trigger();
+    if (st[0] == n - 1) return;
+    const u32 lane = threadIdx.x & 31;
+    const u64 total = *m;
+    const EdgeFmt fmt{};
+    for (u64 base = first + u64(blockIdx.x) * blockDim.x; base < total; base += u64(gridDim.x) * blockDim.x) {
+        const u64 r = base + threadIdx.x;   // whole warps iterate together
+        bool keep = false;
+        if (r < total) {
+            u32 a, b;
+            decode_edge(fmt.rips(keys[r]), a, b);
+            keep = comp[a] != comp[b];
+        }
+        const u32 bal = __ballot_sync(0xffffffffu, keep);
+        if (!bal) continue;
+        u32 pos = 0;
+        if (lane == 0) pos = atomicAdd(st + 1, u32(__popc(bal)));
+        pos = __shfl_sync(0xffffffffu, pos, 0);
+        if (keep) list[pos + __popc(bal & ((1u << lane) - 1u))] = u32(r);
+    }
+}
 
 inline u32 grid_for(u64 work, u32 per_block) {
     const u64 g = (work + per_block - 1) / per_block;
@@ -779,8 +892,98 @@ static u64 sorted_edge_keys(tt_ctx* c, const Complex& cx, int redzed, bool want_
     return m;
 }
 
+// dim0 of a dense complex of at most kSmallN vertices: the same stages, every
+// buffer at its largest size and every count left on the device, so that the
+// host waits once, at the end (sizes of a few hundred points spent most of
+// their time in round trips and launches).
+static void dim0_small(tt_ctx* c, const Complex& cx, u32 maxdim, Dim0Out& out) {
+    const u32 n = cx.n;
+    const u64 cap = u64(n) * (n - 1) / 2;
+    const int want_cols = maxdim >= 1;
+    const cudaStream_t s = c->stream;
+    u64* off = c->arena.get<u64>(S_EDGE_CNT, u64(n) + 2);
+    const u64* mdev = off + n;
+    u32* dmm = reinterpret_cast<u32*>(off + n + 1);
+    u64* keys = c->arena.get<u64>(S_EDGE_KEYS, cap + 1);
+    u64* kb = c->arena.get<u64>(S_SORT_A, cap);
+    u8* app = c->arena.get<u8>(S_FLAGS, 2 * cap + 16);
+    u8* tree = app + cap + 8;
+    u32* res = c->arena.get<u32>(S_EDGE_TMP, cap + 1);
+    u32* comp = c->arena.get<u32>(S_UF_PARENT, n);
+    u32* list = c->arena.get<u32>(S_UF_WORK, cap + 1);
+    const u64 runs = (cap + kRun - 1) / kRun;
+    u64* cnt = c->arena.get<u64>(S_MISC0, runs + 1);
+    u64* tot = c->arena.get<u64>(S_COUNT, 4);
+    u32* st = reinterpret_cast<u32*>(tot + 1);
+    out.keys = keys;
+    out.app = want_cols ? app : nullptr;
+    out.tree = tree;
+    out.h0 = c->arena.get<f32>(S_OUT0, n + 1);
+    out.cidx = c->arena.get<u64>(S_OUT1, (want_cols ? cap : 0) + 1);
+    out.cd = c->arena.get<f32>(S_OUT2, (want_cols ? cap : 0) + 1);
+    out.emi = c->arena.get<u64>(S_OUT3, (want_cols ? cap : 0) + 1);
+    out.emf = c->arena.get<u8>(S_OUT4, (want_cols ? cap : 0) + 1);
+    out.h0_edge = c->arena.get<u64>(S_OUT5, n + 1);
+    const EdgeFmt fmt{};
+    TT_CUDA(cudaMemsetAsync(tot, 0, 4 * sizeof(u64), s));
+    TT_CUDA(cudaMemsetAsync(tree, 0, cap + 1, s));
+    // the apparent scan beside the sort and the forest, once it is long enough
+    // to pay for the fork
+    SideScope side(c);
+    if (want_cols) {
+        const cudaStream_t as = n > 512 ? side.fork() : s;
+        launch_pdl(k_apparent_pairs, dim3(div_up(n, 32), div_up(n, 8)), 256, 0, as, cx.mat, n, cx.thr, res);
+        TT_LAUNCH("k_apparent");
+        ++c->launches;
+    }
+    const u32 g = grid_for(u64(n) * 32, 256);
+    launch_pdl(k_edge_count<DenseRows>, g, 256, 0, s, DenseRows{cx.mat, n}, n, cx.thr, off, dmm);
+    TT_LAUNCH("k_edge_count");
+    scan_exclusive<u64>(c, off, off, n, off + n);
+    constexpr int kBits = 31;   // every bit of a non-negative float: as many passes as 23 bits
+    const bool odd = radix_passes(cap, kBits) & 1;
+    launch_pdl(k_edge_fill<DenseRows, true>, g, 256, 0, s, DenseRows{cx.mat, n}, n, cx.thr, off, kCountOnDevice, 0,
+               odd ? kb : keys, static_cast<u64*>(nullptr), static_cast<u32*>(nullptr));
+    TT_LAUNCH("k_edge_fill");
+    radix_sort<u32>(c, odd ? kb : keys, static_cast<u32*>(nullptr), cap, odd ? keys : kb, static_cast<u32*>(nullptr),
+                    kBits, kIdxBits, reinterpret_cast<const unsigned long long*>(mdev));
+    const u32 first = std::max<u32>(8 * n, 4 * kForestThreads);
+    launch_pdl(k_forest_block, 1, kForestThreads, 0, s, keys, mdev, first, list, n, comp, tree, st);
+    TT_LAUNCH("k_forest_block");
+    c->launches += 3;
+    if (cap > first) {
+        launch_pdl(k_forest_filter, grid_for(cap - first, 256), 256, 0, s, keys, mdev, first, n,
+                   static_cast<const u32*>(comp), list, st);
+        TT_LAUNCH("k_forest_filter");
+        launch_pdl(k_forest_block, 1, kForestThreads, 0, s, keys, mdev, 0u, list, n, comp, tree, st);
+        TT_LAUNCH("k_forest_block");
+        c->launches += 2;
+    }
+    side.join();
+    const u32 gr = grid_for(runs * 32, 256);
+    launch_pdl(k_count_dim0<true>, gr, 256, 0, s, keys, fmt, tree, app, res, cap, mdev, want_cols, cnt);
+    TT_LAUNCH("k_count_dim0");
+    scan_exclusive<u64>(c, cnt, cnt, runs, tot);
+    launch_pdl(k_emit_dim0<true>, gr, 256, 0, s, keys, fmt, tree, app, res, static_cast<const u8*>(nullptr), cap, mdev,
+               want_cols, cnt, tot, out.h0, out.h0_edge, out.cidx, out.cd, out.emi, out.emf);
+    TT_LAUNCH("k_emit_dim0");
+    c->launches += 2;
+    u64* h = static_cast<u64*>(c->pinned.get(4 * sizeof(u64)));
+    TT_CUDA(cudaMemcpyAsync(h, tot, 2 * sizeof(u64), cudaMemcpyDeviceToHost, s));
+    TT_CUDA(cudaMemcpyAsync(h + 2, mdev, sizeof(u64), cudaMemcpyDeviceToHost, s));
+    TT_CUDA(cudaStreamSynchronize(s));
+    out.m = h[2];
+    out.nh0 = h[0] >> 32;
+    out.ncols = h[0] & 0xffffffffull;
+    out.essential = n - u32(h[1]);
+}
+
 void dim0(tt_ctx* c, const Complex& cx, u32 maxdim, Dim0Out& out, u64 m_known) {
     out = Dim0Out{};
+    if (cx.mat && cx.n >= 2 && cx.n <= kSmallN) {
+        dim0_small(c, cx, maxdim, out);
+        return;
+    }
     u32* err = m_known != kUnknownM ? c->arena.get<u32>(S_DIM0_ERR, 4) : nullptr;
     if (err) TT_CUDA(cudaMemsetAsync(err, 0, sizeof(u32), c->stream));
     // packed keys of a dense complex: the apparent scan goes by vertex pairs
@@ -847,10 +1050,10 @@ void dim0(tt_ctx* c, const Complex& cx, u32 maxdim, Dim0Out& out, u64 m_known) {
         // few edges a point connect nearly everything: by the time the long
         // ones join, one pass finds them inside a component (or the forest
         // is complete and they are never read). Groups of 8 n, then 64 n
-        // edges, then the rest; with fewer than 16 n edges (kNN graphs) the
-        // extra trips would cost more than the passes they save, and all
-        // join at once.
-        const u64 group[3] = {m < 16 * u64(n) ? m : 8 * u64(n), std::min<u64>(m, 72 * u64(n)), m};
+        // edges, then the rest; with fewer than 16 n edges (kNN graphs), or
+        // fewer than 2^17 in all, the extra trips would cost more than the
+        // passes they save, and all join at once.
+        const u64 group[3] = {m < std::max<u64>(16 * u64(n), 1 << 17) ? m : 8 * u64(n), std::min<u64>(m, 72 * u64(n)), m};
         u32 known = 0, joined = 0;
         for (int round = 0, trip = 0; round < kRounds; ++trip) {
             const u32 upto = u32(trip < 3 ? group[trip] : m);
@@ -887,8 +1090,8 @@ void dim0(tt_ctx* c, const Complex& cx, u32 maxdim, Dim0Out& out, u64 m_known) {
     u64* tot = c->arena.get<u64>(S_COUNT, 4);
     const u32 gr = grid_for(runs * 32, 256);
     if (m) {
-        if (pairs) launch_pdl(k_count_dim0<true>, gr, 256, 0, c->stream, out.keys, fmt, tree, app, emw, m, want_cols, cnt);
-        else launch_pdl(k_count_dim0<false>, gr, 256, 0, c->stream, out.keys, fmt, tree, app, emw, m, want_cols, cnt);
+        if (pairs) launch_pdl(k_count_dim0<true>, gr, 256, 0, c->stream, out.keys, fmt, tree, app, emw, m, static_cast<const u64*>(nullptr), want_cols, cnt);
+        else launch_pdl(k_count_dim0<false>, gr, 256, 0, c->stream, out.keys, fmt, tree, app, emw, m, static_cast<const u64*>(nullptr), want_cols, cnt);
         TT_LAUNCH("k_count_dim0");
         scan_exclusive<u64>(c, cnt, cnt, runs, tot);
         c->launches += 1;
@@ -907,7 +1110,7 @@ void dim0(tt_ctx* c, const Complex& cx, u32 maxdim, Dim0Out& out, u64 m_known) {
         out.h0_edge = c->arena.get<u64>(S_OUT5, nh0 + 1);
         if (m) {
             auto go = [&](auto kernel) {
-                launch_pdl(kernel, gr, 256, 0, c->stream, out.keys, fmt, tree, app, emw, emf, m, want_cols, cnt, tot,
+                launch_pdl(kernel, gr, 256, 0, c->stream, out.keys, fmt, tree, app, emw, emf, m, static_cast<const u64*>(nullptr), want_cols, cnt, tot,
                            out.h0, out.h0_edge, out.cidx, out.cd, out.emi, out.emf);
             };
             if (pairs) go(k_emit_dim0<true>);
