@@ -12,16 +12,27 @@
 //                   from one work list (uneven clouds balance themselves) and
 //                   fold row maxima
 //   k_batch_radius  per-cloud minimum of the row maxima
-//   k_batch_rowcount + scan   kept pairs per row and their offsets (the
-//                   total kept count stays on the device)
-//   k_batch_edges   the kept edges of every cloud, compacted, as 64-bit keys
-//                     cloud << (31 + ib) | d bits << ib | index
-//                   in (cloud, index) order, so one stable radix sort of the
-//                   bits above the index field (cloud and d: 40 bits for 512
-//                   clouds, four passes) orders all clouds at once by
-//                   (cloud, d, index); the sort reads its key count from the
-//                   device and skips the tiles beyond it
-//   k_batch_emit    EdgeList (diameter, vertex pair) + per-cloud offsets
+//   k_batch_hist    kept pairs per row, and every cloud's histogram of its kept
+//                   distances over bins linear in the distance
+//   scan            of the row counts: per-cloud offsets, the total
+//   k_batch_bins    bin offsets per cloud; consecutive bins grouped into items
+//                   of at most kItemCap edges, or, where one bin holds more
+//                   than kBinMax (ties, tight clusters), the cloud marked for
+//                   the radix sort
+//   k_batch_part    the kept edges as keys (d bits << 32 | index) into their
+//                   bins, in no particular order inside a bin
+//   k_batch_items   each item ordered in shared memory and written out as
+//                   EdgeList (diameter, vertex pair)
+// A distance is moved twice that way (into its bin, and out in order), where
+// the four 8-bit passes of a radix sort read it eight times and wrote it four
+// (512 clouds, 312 M kept edges: 13.6 ms with the edge lists, now 7.0). The bin
+// of a distance is floor(d * bins / radius) in floats: monotone in d, so the
+// bins partition the filtration order whatever the rounding.
+// The marked clouds go through
+//   k_batch_edges   keys cloud << (31 + ib) | d bits << ib | index, compacted
+//                   in (cloud, index) order, a segmented stable radix sort on
+//                   the distance bits, and k_batch_emit
+// whose kernels return at once when no cloud is marked.
 // Buffers are sized for the worst case (every pair kept), so no step reads a
 // count back to the host and the whole sequence is captured into a CUDA
 // graph once and replayed.
@@ -94,42 +105,383 @@ __global__ void k_batch_radius(const u32* __restrict__ rowmax, const u32* __rest
     }
 }
 
-// Kept pairs (j < i, d <= the cloud's radius) per row: one warp per row of
-// one cloud (rows listed globally), the count into row_cnt.
-__global__ void k_batch_rowcount(const f32* __restrict__ mats, const u64* __restrict__ mat_off,
-                                 const u32* __restrict__ sizes, const u64* __restrict__ pt_off,
-                                 const u32* __restrict__ row_cloud, u64 rows, const u32* __restrict__ radius,
-                                 u64* __restrict__ row_cnt) {
-    const int lane = threadIdx.x & 31;
-    const u64 warps = (u64(gridDim.x) * blockDim.x) >> 5;
-    for (u64 r = (u64(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; r < rows; r += warps) {
-        const u32 c = row_cloud[r];
-        const u32 n = sizes[c];
-        const u32 i = u32(r - pt_off[c]);
-        const f32 thr = __uint_as_float(radius[c]);
-        const f32* row = mats + mat_off[c] + u64(i) * n;
-        u64 kept = 0;
-#pragma unroll 4
-        for (u32 j0 = 0; j0 < i; j0 += 32) {   // (unrolled: several row loads in flight)
-            const u32 j = j0 + lane;
-            kept += __popc(__ballot_sync(0xffffffffu, j < i && row[j] <= thr));
+// A run of a cloud's rows holding about kChunkPairs pairs.
+struct Chunk {
+    u32 cloud, row0, row1;
+    u32 pad;
+    u64 rank;   // its place in `ranks`: per bin, the cloud's edges of earlier-counted chunks
+};
+constexpr u64 kChunkPairs = 64 * 1024;
+constexpr u32 kMaxBins = 8192;
+constexpr int kPartThreads = 1024;
+// One block an SM (by its shared memory): the blocks then write into the bins
+// of about ten million edges at a time, which L2 holds until their lines are
+// full. With four blocks an SM on runs twice as long, partly written sectors
+// went out to memory and came back (8.2 ms for 312 M edges; now 3.4, bound by
+// the scattered 8-byte stores).
+constexpr size_t kPartSmem = 120 * 1024;
+constexpr u32 kItemCap = 4096;                 // edges an item orders at once
+constexpr u32 kItemStep = 2560;                // an item: the bins that start in one step of this many edges ...
+constexpr u32 kBinMax = kItemCap - kItemStep;  // ... and no bin longer than this
+constexpr int kItemThreads = 256;
+constexpr u32 kSlots = 2048;                   // linear slots an item's keys are placed by
+struct Item {
+    u32 begin, end;   // edges of the cloud, relative to its first
+};
+
+// What the sort stages know of a cloud (device arrays indexed by cloud).
+struct CloudTable {
+    const u64* pt_off;
+    const u64* mat_off;
+    const u32* sizes;
+    const u32* bin_off;    // first bin; the next cloud's ends them
+    const u32* item_off;   // first item slot
+};
+
+__device__ __forceinline__ u32 bin_of(f32 d, f32 scale, u32 bins) {
+    return min(bins - 1u, __float2uint_rz(__fmul_rn(d, scale)));   // (a NaN product, 0 * inf, is bin 0)
+}
+
+// The kept entries of a row (j < i, d <= thr), a warp a row: f(d, j) for each,
+// with kRowLoads loads in flight (a row's entries are used once, so the loads'
+// latency is what a warp waits for).
+constexpr int kRowLoads = 8;
+template <typename F>
+__device__ __forceinline__ void for_row(const f32* __restrict__ row, u32 i, f32 thr, F&& f) {
+    const u32 lane = threadIdx.x & 31;
+    for (u32 j0 = 0; j0 < i; j0 += 32 * kRowLoads) {
+        f32 d[kRowLoads];
+#pragma unroll
+        for (int q = 0; q < kRowLoads; ++q) {
+            const u32 j = j0 + 32 * q + lane;
+            d[q] = j < i ? row[j] : INFINITY;
         }
-        if (lane == 0) row_cnt[r] = kept;
+        f(d, j0 + lane);
     }
 }
 
-// The kept pairs written compacted, at row_off[row] + rank in the row: the
-// array runs over (cloud, index) ascending (rows ascending, j ascending in a
-// row), so a stable sort on the bits above the index field alone orders it
-// by (cloud, d, index). Key: cloud << (31 + ib) | d bits << ib | index.
+// Row counts and the cloud's histogram, one block a chunk: the bins counted in
+// shared memory first (one global atomic a bin and chunk; its old value is
+// where the chunk's edges go within the bin).
+constexpr int kHistThreads = 512;
+__global__ void __launch_bounds__(kHistThreads)
+    k_batch_hist(const f32* __restrict__ mats, CloudTable T, const Chunk* __restrict__ chunks,
+                 const u32* __restrict__ radius, u64* __restrict__ row_cnt, u32* __restrict__ hist,
+                 u32* __restrict__ ranks) {
+    __shared__ u32 h[kMaxBins];
+    const Chunk ck = chunks[blockIdx.x];
+    const u32 c = ck.cloud, n = T.sizes[c], b0 = T.bin_off[c], bins = T.bin_off[c + 1] - b0;
+    const f32 thr = __uint_as_float(radius[c]), scale = __fdiv_rn(f32(bins), thr);
+    for (u32 b = threadIdx.x; b < bins; b += kHistThreads) h[b] = 0;
+    __syncthreads();
+    const u32 lane = threadIdx.x & 31;
+    for (u32 i = ck.row0 + (threadIdx.x >> 5); i < ck.row1; i += kHistThreads / 32) {
+        u32 kept = 0;
+        for_row(mats + T.mat_off[c] + u64(i) * n, i, thr, [&](const f32(&d)[kRowLoads], u32 j) {
+#pragma unroll
+            for (int q = 0; q < kRowLoads; ++q) {
+                const bool keep = j + 32 * q < i && d[q] <= thr;
+                if (keep) atomicAdd(&h[bin_of(d[q], scale, bins)], 1u);
+                kept += keep;
+            }
+        });
+        kept = __reduce_add_sync(0xffffffffu, kept);
+        if (lane == 0) row_cnt[T.pt_off[c] + i] = kept;
+    }
+    __syncthreads();
+    for (u32 b = threadIdx.x; b < bins; b += kHistThreads) ranks[ck.rank + b] = h[b] ? atomicAdd(&hist[b0 + b], h[b]) : 0u;
+}
+
+// Exclusive scan over the 1,024 threads of the block (u32).
+__device__ __forceinline__ u32 block_scan1024(u32 v, u32* warp_tot, u32& total) {
+    const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    u32 inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const u32 y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= u32(o)) inc += y;
+    }
+    __syncthreads();   // warp_tot free again
+    if (lane == 31) warp_tot[w] = inc;
+    __syncthreads();
+    u32 pre = 0, tot = 0;
+#pragma unroll
+    for (u32 q = 0; q < 32; ++q) {
+        const u32 t = warp_tot[q];
+        pre += q < w ? t : 0u;
+        tot += t;
+    }
+    total = tot;
+    return pre + inc - v;
+}
+
+// One block a cloud: its bins' starts (hist becomes the cursors of the
+// partition), its items, and whether it is left to the radix sort; edge_off
+// from the scanned row counts (the last block adds the total).
+__global__ void __launch_bounds__(1024) k_batch_bins(CloudTable T, u32 clouds, const u64* __restrict__ row_off,
+                                                     const unsigned long long* __restrict__ total,
+                                                     u32* __restrict__ hist, Item* __restrict__ items,
+                                                     u32* __restrict__ radix, u64* __restrict__ edge_off) {
+    __shared__ u32 wt[32];
+    const u32 c = blockIdx.x, b0 = T.bin_off[c], bins = T.bin_off[c + 1] - b0;
+    const u32 per = (bins + 1023) / 1024;   // bins a thread: at most kMaxBins / 1024
+    u32 v[kMaxBins / 1024];
+    u32 sum = 0, mx = 0;
+#pragma unroll
+    for (u32 q = 0; q < kMaxBins / 1024; ++q) {
+        const u32 b = threadIdx.x * per + q;
+        v[q] = q < per && b < bins ? hist[b0 + b] : 0u;
+        sum += v[q];
+        mx = max(mx, v[q]);
+    }
+    u32 all;
+    const u32 start = block_scan1024(sum, wt, all);
+    const u32 s0 = T.item_off[c], cap = T.item_off[c + 1] - s0;
+    const bool rad = __syncthreads_or(mx > kBinMax) || cap == 0;
+    if (threadIdx.x == 0) {
+        radix[c] = rad;
+        edge_off[c] = row_off[T.pt_off[c]];
+        if (c == clouds - 1) edge_off[clouds] = *total;
+    }
+    // items: bin b opens one when its start lies in another step than the
+    // start of the bin before it
+    u32 opens = 0, run = start;
+    u32 prev = threadIdx.x == 0 ? 0xffffffffu : 0u;   // the previous bin's step
+    // the previous bin (another thread's last) starts at start - its count; its step:
+    __shared__ u32 last_step[1024];
+#pragma unroll
+    for (u32 q = 0, r = start; q < kMaxBins / 1024; ++q) {
+        if (q < per) last_step[threadIdx.x] = r / kItemStep;
+        r += v[q];
+    }
+    __syncthreads();
+    if (threadIdx.x > 0) prev = last_step[threadIdx.x - 1];
+#pragma unroll
+    for (u32 q = 0, r = start, p = prev; q < kMaxBins / 1024; ++q) {
+        const u32 b = threadIdx.x * per + q;
+        if (q < per && b < bins) {
+            const u32 st = r / kItemStep;
+            opens += st != p;
+            p = st;
+        }
+        r += v[q];
+    }
+    u32 nitems;
+    u32 slot = block_scan1024(opens, wt, nitems);
+    u32 p = prev;
+#pragma unroll
+    for (u32 q = 0; q < kMaxBins / 1024; ++q) {
+        const u32 b = threadIdx.x * per + q;
+        if (q < per && b < bins) {
+            const u32 st = run / kItemStep;
+            if (st != p && !rad) {
+                items[s0 + slot].begin = run;
+                if (slot) items[s0 + slot - 1].end = run;
+            }
+            slot += st != p;
+            p = st;
+            hist[b0 + b] = run;
+        }
+        run += v[q];
+    }
+    if (rad) nitems = 0;
+    else if (threadIdx.x == 0 && nitems) items[s0 + nitems - 1].end = all;
+    for (u32 q = nitems + threadIdx.x; q < cap; q += blockDim.x) items[s0 + q] = Item{0, 0};
+}
+
+// The kept edges of a chunk into their bins, one block a chunk.
+__global__ void __launch_bounds__(kPartThreads)
+    k_batch_part(const f32* __restrict__ mats, CloudTable T, const Chunk* __restrict__ chunks,
+                 const u32* __restrict__ radius, const u32* __restrict__ radix, const u64* __restrict__ edge_off,
+                 const u32* __restrict__ bin_start, const u32* __restrict__ ranks, u64* __restrict__ keys) {
+    extern __shared__ u32 h[];   // [kMaxBins] (of kPartSmem bytes): the next free place of every bin
+    const Chunk ck = chunks[blockIdx.x];
+    const u32 c = ck.cloud;
+    if (radix[c]) return;
+    const u32 n = T.sizes[c], b0 = T.bin_off[c], bins = T.bin_off[c + 1] - b0;
+    const f32 thr = __uint_as_float(radius[c]), scale = __fdiv_rn(f32(bins), thr);
+    for (u32 b = threadIdx.x; b < bins; b += kPartThreads) h[b] = bin_start[b0 + b] + ranks[ck.rank + b];
+    __syncthreads();
+    const f32* mat = mats + T.mat_off[c];
+    u64* out = keys + edge_off[c];
+    for (u32 i = ck.row0 + (threadIdx.x >> 5); i < ck.row1; i += kPartThreads / 32) {
+        const u32 rbase = u32(u64(i) * (i - 1) / 2);
+        for_row(mat + u64(i) * n, i, thr, [&](const f32(&d)[kRowLoads], u32 j) {
+            u32 pos[kRowLoads];
+#pragma unroll
+            for (int q = 0; q < kRowLoads; ++q)
+                if (j + 32 * q < i && d[q] <= thr) pos[q] = atomicAdd(&h[bin_of(d[q], scale, bins)], 1u);
+#pragma unroll
+            for (int q = 0; q < kRowLoads; ++q)
+                if (j + 32 * q < i && d[q] <= thr)
+                    out[pos[q]] = (u64(__float_as_uint(d[q])) << 32) | (rbase + j + 32 * q);
+        });
+    }
+}
+
+// decode_edge for idx < 2^31 in 32-bit arithmetic (v <= 65,536, so v (v - 1)
+// fits; the closed form in FP32 is within one of the answer).
+__device__ __forceinline__ void decode_edge31(u32 idx, u32& a, u32& b) {
+    u32 v = u32((1.0f + sqrtf(fmaf(8.0f, f32(idx), 1.0f))) * 0.5f);
+    u32 t = v * (v - 1u) / 2u;
+    if (t > idx) {
+        --v;
+        t -= v;
+    }
+    if (t + v <= idx) {
+        t += v;
+        ++v;
+    }
+    a = v;
+    b = idx - t;
+}
+
+// One item: its keys counted into kSlots linear slots of its distance range
+// (about one key a slot), placed slot by slot in shared memory, and the few
+// keys of a slot put in order by insertion. An item whose distances crowd (a
+// slot of more than kSlotMax keys: ties) is ordered by a bitonic sort instead.
+// Then written out in order. 312 M edges: 3.1 ms, 1.9 instructions a cycle,
+// bound by shared-memory latency at 23 warps an SM.
+constexpr u32 kSlotMax = 24;
+__global__ void __launch_bounds__(kItemThreads)
+    k_batch_items(const Item* __restrict__ items, const u32* __restrict__ item_cloud, const u64* __restrict__ edge_off,
+                  const u64* __restrict__ keys, f32* __restrict__ ed, int32_t* __restrict__ ev) {
+    __shared__ u64 sk[kItemCap];
+    __shared__ u32 cnt[kSlots];
+    __shared__ u32 red[2][kItemThreads / 32];
+    __shared__ u32 wt[kItemThreads / 32];
+    const Item it = items[blockIdx.x];
+    const u32 m = it.end - it.begin;
+    if (m == 0) return;
+    const u64 base = edge_off[item_cloud[blockIdx.x]] + it.begin;
+    const u32 tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    constexpr u32 kPer = kItemCap / kItemThreads;
+    u64 k[kPer];
+    u32 lo = 0xffffffffu, hi = 0;
+#pragma unroll
+    for (u32 q = 0; q < kPer; ++q) {
+        const u32 e = q * kItemThreads + tid;
+        k[q] = e < m ? keys[base + e] : ~0ull;
+        if (e < m) {
+            lo = min(lo, u32(k[q] >> 32));
+            hi = max(hi, u32(k[q] >> 32));
+        }
+        if (e < kSlots) cnt[e] = 0;
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (lane == 0) red[0][w] = lo, red[1][w] = hi;
+    __syncthreads();
+#pragma unroll
+    for (u32 q = 0; q < kItemThreads / 32; ++q) lo = min(lo, red[0][q]), hi = max(hi, red[1][q]);
+    // slots linear in the distance: (d - dmin) * (kSlots / (dmax - dmin)), monotone in d
+    const f32 dmin = __uint_as_float(lo), range = __fsub_rn(__uint_as_float(hi), dmin);
+    const f32 scale = range > 0.0f ? __fdiv_rn(f32(kSlots), range) : 0.0f;
+    u32 at[kPer];
+#pragma unroll
+    for (u32 q = 0; q < kPer; ++q) {
+        const u32 e = q * kItemThreads + tid;
+        if (e < m) {
+            const f32 d = __uint_as_float(u32(k[q] >> 32));
+            const u32 s = bin_of(__fsub_rn(d, dmin), scale, kSlots);
+            at[q] = (s << 16) | atomicAdd(&cnt[s], 1u);   // slot, place in it (both below 2^13)
+        }
+    }
+    __syncthreads();
+    // exclusive scan of the slots, kSlotPer consecutive ones a thread
+    constexpr u32 kSlotPer = kSlots / kItemThreads;
+    u32 c[kSlotPer], sum = 0, most = 0;
+#pragma unroll
+    for (u32 q = 0; q < kSlotPer; ++q) {
+        c[q] = cnt[tid * kSlotPer + q];
+        sum += c[q];
+        most = max(most, c[q]);
+    }
+    u32 inc = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const u32 y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= u32(o)) inc += y;
+    }
+    if (lane == 31) wt[w] = inc;
+    const bool crowded = __syncthreads_or(most > kSlotMax);
+    u32 pre = inc - sum;
+#pragma unroll
+    for (u32 q = 0; q < kItemThreads / 32; ++q) pre += q < w ? wt[q] : 0u;
+    {
+        u32 run = pre;
+#pragma unroll
+        for (u32 q = 0; q < kSlotPer; ++q) {
+            cnt[tid * kSlotPer + q] = run;
+            run += c[q];
+        }
+    }
+    __syncthreads();
+    if (!crowded) {
+#pragma unroll
+        for (u32 q = 0; q < kPer; ++q) {
+            const u32 e = q * kItemThreads + tid;
+            if (e < m) sk[cnt[at[q] >> 16] + (at[q] & 0xffffu)] = k[q];
+        }
+        __syncthreads();
+        u32 run = pre;
+#pragma unroll
+        for (u32 q = 0; q < kSlotPer; ++q) {
+            const u32 len = c[q];
+            for (u32 x = 1; x < len; ++x) {   // insertion by the whole key
+                const u64 key = sk[run + x];
+                u32 y = x;
+                while (y > 0 && sk[run + y - 1] > key) {
+                    sk[run + y] = sk[run + y - 1];
+                    --y;
+                }
+                sk[run + y] = key;
+            }
+            run += len;
+        }
+    } else {
+        u32 P = 2;
+        while (P < m) P <<= 1;
+#pragma unroll
+        for (u32 q = 0; q < kPer; ++q) sk[q * kItemThreads + tid] = k[q];   // (past m: ~0)
+        __syncthreads();
+        for (u32 size = 2; size <= P; size <<= 1)
+            for (u32 stride = size >> 1; stride; stride >>= 1) {
+                for (u32 i = tid; i < P / 2; i += kItemThreads) {
+                    const u32 a = 2 * i - (i & (stride - 1)), b = a + stride;
+                    const u64 x = sk[a], y = sk[b];
+                    if ((x > y) == ((a & size) == 0)) {
+                        sk[a] = y;
+                        sk[b] = x;
+                    }
+                }
+                __syncthreads();
+            }
+    }
+    __syncthreads();
+    for (u32 e = tid; e < m; e += kItemThreads) {
+        const u64 key = sk[e];
+        u32 a, b;
+        decode_edge31(u32(key), a, b);
+        ed[base + e] = __uint_as_float(u32(key >> 32));
+        reinterpret_cast<int2*>(ev)[base + e] = make_int2(int(b), int(a));
+    }
+}
+
+// The marked clouds' kept pairs written compacted, at row_off[row] + rank in
+// the row: their keys run over (cloud, index) ascending (rows ascending, j
+// ascending in a row), so a stable sort on the bits above the index field
+// alone orders them by (cloud, d, index). Key: cloud << (31 + ib) | d bits << ib | index.
 __global__ void k_batch_edges(const f32* __restrict__ mats, const u64* __restrict__ mat_off,
                               const u32* __restrict__ sizes, const u64* __restrict__ pt_off,
-                              const u32* __restrict__ row_cloud, u64 rows, const u32* __restrict__ radius, int ib,
-                              const u64* __restrict__ row_off, u64* __restrict__ keys, u64* __restrict__ per_cloud) {
+                              const u32* __restrict__ row_cloud, u64 rows, const u32* __restrict__ radius,
+                              const u32* __restrict__ radix, int ib, const u64* __restrict__ row_off,
+                              u64* __restrict__ keys) {
     const int lane = threadIdx.x & 31;
     const u64 warps = (u64(gridDim.x) * blockDim.x) >> 5;
     for (u64 r = (u64(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; r < rows; r += warps) {
         const u32 c = row_cloud[r];
+        if (!radix[c]) continue;
         const u32 n = sizes[c];
         const u32 i = u32(r - pt_off[c]);
         const f32 thr = __uint_as_float(radius[c]);
@@ -147,69 +499,51 @@ __global__ void k_batch_edges(const f32* __restrict__ mats, const u64* __restric
                     (u64(c) << (31 + ib)) | (u64(__float_as_uint(d)) << ib) | (rbase + j);
             pos += __popc(bal);
         }
-        const u64 kept = pos - row_off[r];
-        if (lane == 0 && kept) atomicAdd((unsigned long long*)&per_cloud[c], (unsigned long long)kept);
     }
 }
 
-// Exclusive scan of the per-cloud edge counts (one CTA; clouds <= 65536),
-// and the segmented sort's tiles of the kept keys: cloud c's ceil(count /
-// kSegTileKeys) tiles after the previous clouds', their digit counts at 256
-// per tile in the same order; *ntiles = the list's length.
-__global__ void k_batch_offsets(const u64* __restrict__ per_cloud, u32 clouds, u64* __restrict__ off,
-                                SegTile* __restrict__ tiles, u32* __restrict__ ntiles) {
-    __shared__ u64 part[1024];
-    __shared__ u32 tpart[1024];
-    const u32 t = threadIdx.x;
-    const u32 per = (clouds + blockDim.x - 1) / blockDim.x;
-    u64 s = 0;
-    u32 ts = 0;
+// The segmented sort's tiles of the marked clouds' keys: cloud c's
+// ceil(count / kSegTileKeys) tiles after the previous ones', their digit
+// counts at 256 per tile in the same order; *ntiles = the list's length. One
+// block; clouds <= 65536.
+__global__ void __launch_bounds__(1024) k_batch_tiles(const u64* __restrict__ off, const u32* __restrict__ radix,
+                                                      u32 clouds, SegTile* __restrict__ tiles,
+                                                      u32* __restrict__ ntiles) {
+    __shared__ u32 wt[32];
+    const u32 t = threadIdx.x, per = (clouds + blockDim.x - 1) / blockDim.x;
+    auto keys_of = [&](u32 c) -> u32 { return radix[c] ? u32(off[c + 1] - off[c]) : 0u; };
+    u32 sum = 0, ksum = 0;
     for (u32 c = t * per; c < min(clouds, (t + 1) * per); ++c) {
-        s += per_cloud[c];
-        ts += u32((per_cloud[c] + kSegTileKeys - 1) / kSegTileKeys);
+        sum += (keys_of(c) + kSegTileKeys - 1) / kSegTileKeys;
+        ksum += keys_of(c);
     }
-    part[t] = s;
-    tpart[t] = ts;
-    __syncthreads();
-    if (t == 0) {
-        u64 run = 0;
-        u32 trun = 0;
-        for (u32 q = 0; q < blockDim.x; ++q) {
-            const u64 v = part[q];
-            const u32 tv = tpart[q];
-            part[q] = run;
-            tpart[q] = trun;
-            run += v;
-            trun += tv;
-        }
-    }
-    __syncthreads();
-    u64 run = part[t];
-    u32 trun = tpart[t];
+    u32 total, ktotal;
+    u32 run = block_scan1024(sum, wt, total), krun = block_scan1024(ksum, wt, ktotal);
     for (u32 c = t * per; c < min(clouds, (t + 1) * per); ++c) {
-        off[c] = run;
-        run += per_cloud[c];
-        const u32 tc = u32((per_cloud[c] + kSegTileKeys - 1) / kSegTileKeys);
-        for (u32 q = 0; q < tc; ++q) tiles[trun + q] = SegTile{c, q, 256u * trun, tc};
-        trun += tc;
+        const u32 tc = (keys_of(c) + kSegTileKeys - 1) / kSegTileKeys;
+        for (u32 q = 0; q < tc; ++q) tiles[run + q] = SegTile{c, q, 256u * run, tc, u32(off[c]) - krun};
+        run += tc;
+        krun += keys_of(c);
     }
-    if (t == blockDim.x - 1) {
-        off[clouds] = run;
-        *ntiles = trun;
-    }
+    if (t == 0) *ntiles = total;
 }
 
-__global__ void k_batch_emit(const u64* __restrict__ keys, const unsigned long long* __restrict__ count, int ib,
+__global__ void k_batch_emit(const u64* __restrict__ keys, const u64* __restrict__ off,
+                             const SegTile* __restrict__ tiles, const u32* __restrict__ ntiles, int ib,
                              f32* __restrict__ d, int32_t* __restrict__ verts) {
-    const u64 m = *count;
     const u64 imask = (1ull << ib) - 1;
-    for (u64 e = u64(blockIdx.x) * blockDim.x + threadIdx.x; e < m; e += u64(gridDim.x) * blockDim.x) {
-        const u64 k = keys[e];
-        u32 a, b;
-        decode_edge(k & imask, a, b);
-        d[e] = __uint_as_float(u32((k >> ib) & 0x7fffffffu));
-        verts[2 * e] = int32_t(b);
-        verts[2 * e + 1] = int32_t(a);
+    const u32 nt = *ntiles;
+    for (u32 q = blockIdx.x; q < nt; q += gridDim.x) {
+        const SegTile tl = tiles[q];
+        const u64 lo = off[tl.seg] + u64(tl.t) * kSegTileKeys, hi = min(lo + kSegTileKeys, off[tl.seg + 1]);
+        for (u64 e = lo + threadIdx.x; e < hi; e += blockDim.x) {
+            const u64 k = keys[e];
+            u32 a, b;
+            decode_edge(k & imask, a, b);
+            d[e] = __uint_as_float(u32((k >> ib) & 0x7fffffffu));
+            verts[2 * e] = int32_t(b);
+            verts[2 * e + 1] = int32_t(a);
+        }
     }
 }
 
@@ -244,7 +578,17 @@ struct Batch {
     u64* row_cnt = nullptr;    // kept pairs per row, then their exclusive scan
     u64* row_off = nullptr;
     unsigned long long* count = nullptr;
-    u64* per_cloud = nullptr;
+    Chunk* chunks = nullptr;        // row runs of the histogram and the partition
+    u32 nchunks = 0;
+    u32* bin_off = nullptr;         // first bin of every cloud
+    u32 total_bins = 0;
+    u32* hist = nullptr;            // bin counts, then the bins' starts
+    u32* ranks = nullptr;           // per chunk and bin (Chunk::rank)
+    u32* item_off = nullptr;        // first item slot of every cloud
+    u32 total_items = 0;
+    Item* items = nullptr;
+    u32* item_cloud = nullptr;
+    u32* radix = nullptr;           // clouds left to the radix sort
     u64* edge_off = nullptr;
     SegTile* seg_tiles = nullptr;   // the segmented sort's tiles of the kept keys (built on the device)
     u32* seg_ntiles = nullptr;      // ... their number
@@ -352,30 +696,39 @@ struct Batch {
         TT_CUDA(cudaMemsetAsync(radius, 0xff, clouds * sizeof(u32), s));
         TT_CUDA(cudaMemsetAsync(next, 0, sizeof(u32), s));
         TT_CUDA(cudaMemsetAsync(count, 0, sizeof(unsigned long long), s));
-        TT_CUDA(cudaMemsetAsync(per_cloud, 0, clouds * sizeof(u64), s));
+        TT_CUDA(cudaMemsetAsync(hist, 0, total_bins * sizeof(u32), s));
         launch_dense(shape, s);
 
         const u32 g2 = u32(std::min<u64>((total_pts + 255) / 256, u64(owner->sms) * 16));
         k_batch_radius<<<g2, 256, 0, s>>>(rowmax, row_cloud, total_pts, radius);
         TT_LAUNCH("k_batch_radius");
-        const u32 g3 = u32(std::min<u64>((total_pts * 32 + 255) / 256, u64(owner->sms) * 32));
-        k_batch_rowcount<<<g3, 256, 0, s>>>(mats, mat_off, sizes, pt_off, row_cloud, total_pts, radius, row_cnt);
-        TT_LAUNCH("k_batch_rowcount");
+        const CloudTable T{pt_off, mat_off, sizes, bin_off, item_off};
+        k_batch_hist<<<nchunks, kHistThreads, 0, s>>>(mats, T, chunks, radius, row_cnt, hist, ranks);
+        TT_LAUNCH("k_batch_hist");
         scan_exclusive<u64>(&sctx, row_cnt, row_off, total_pts, reinterpret_cast<u64*>(count), 0);
-        k_batch_edges<<<g3, 256, 0, s>>>(mats, mat_off, sizes, pt_off, row_cloud, total_pts, radius, ib, row_off,
-                                         keys, per_cloud);
+        k_batch_bins<<<clouds, 1024, 0, s>>>(T, clouds, row_off, count, hist, items, radix, edge_off);
+        TT_LAUNCH("k_batch_bins");
+        k_batch_part<<<nchunks, kPartThreads, kPartSmem, s>>>(mats, T, chunks, radius, radix, edge_off, hist,
+                                                              ranks, keys);
+        TT_LAUNCH("k_batch_part");
+        if (total_items)
+            k_batch_items<<<total_items, kItemThreads, 0, s>>>(items, item_cloud, edge_off, keys, ed, ev);
+        TT_LAUNCH("k_batch_items");
+        // the marked clouds, each on its own (their keys are contiguous), by
+        // the distance bits alone (stable: ties keep the index order): four
+        // 8-bit passes
+        const u32 g3 = u32(std::min<u64>((total_pts * 32 + 255) / 256, u64(owner->sms) * 32));
+        k_batch_tiles<<<1, 1024, 0, s>>>(edge_off, radix, clouds, seg_tiles, seg_ntiles);
+        TT_LAUNCH("k_batch_tiles");
+        k_batch_edges<<<g3, 256, 0, s>>>(mats, mat_off, sizes, pt_off, row_cloud, total_pts, radius, radix, ib, row_off,
+                                         keys);
         TT_LAUNCH("k_batch_edges");
-        k_batch_offsets<<<1, 1024, 0, s>>>(per_cloud, clouds, edge_off, seg_tiles, seg_ntiles);
-        TT_LAUNCH("k_batch_offsets");
-        // every cloud's kept keys on their own (they are contiguous, clouds
-        // in order), by the distance bits alone (stable: ties keep the index
-        // order): four 8-bit passes, the cloud bits need none
         const bool swapped =
             radix_sort_segments(&sctx, keys, kbuf, edge_off, seg_tiles, seg_ntiles, nseg_tiles, seg_hist, 31, ib);
-        const u32 g4 = u32(std::min<u64>((total_pairs + 255) / 256, u64(owner->sms) * 32));
-        k_batch_emit<<<g4, 256, 0, s>>>(swapped ? kbuf : keys, count, ib, ed, ev);
+        const u32 g4 = std::min<u32>(std::max<u32>(nseg_tiles, 1), u32(owner->sms) * 8);
+        k_batch_emit<<<g4, 256, 0, s>>>(swapped ? kbuf : keys, edge_off, seg_tiles, seg_ntiles, ib, ed, ev);
         TT_LAUNCH("k_batch_emit");
-        sctx.launches += 6;
+        sctx.launches += 9;
     }
 
     static int bits_for(u64 v) {
@@ -411,10 +764,14 @@ Batch* batch_create(tt_ctx* c, const u32* sizes_h, u32 clouds, u32 dim, int kind
         b->sctx.device = c->device;
         b->sctx.sms = c->sms;
         TT_CUDA(cudaStreamCreateWithFlags(&b->sctx.stream, cudaStreamNonBlocking));
+        TT_CUDA(cudaFuncSetAttribute(k_batch_part, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPartSmem)));
         std::vector<u64> pt_off(clouds + 1, 0), mat_off(clouds + 1, 0), pair_off(clouds + 1, 0);
         std::vector<Tile> tiles[kNumShapes];
         std::vector<u32> row_cloud;
         u64 pairs = 0;
+        std::vector<Chunk> chunks;
+        u64 nranks = 0;
+        std::vector<u32> bin_off(clouds + 1, 0), item_off(clouds + 1, 0), item_cloud;
         for (u32 q = 0; q < clouds; ++q) {
             const u32 n = sizes_h[q];
             if (n < 1) invalid("gb300: every cloud needs at least one point");
@@ -427,6 +784,23 @@ Batch* batch_create(tt_ctx* c, const u32* sizes_h, u32 clouds, u32 dim, int kind
                 for (u32 i0 = 0; i0 < n; i0 += u32(kShapes[si].r))
                     for (u32 j0 = i0; j0 < n; j0 += u32(kShapes[si].c)) tiles[si].push_back(Tile{q, i0, j0});
             for (u32 i = 0; i < n; ++i) row_cloud.push_back(q);
+            // chunks of rows; bins of about 256 pairs (a power of two); items
+            // (a cloud beyond 32-bit edge positions goes to the radix sort: one
+            // bin, which then overflows)
+            const u64 cp = u64(n) * (n - 1) / 2;
+            u32 bins = cp < (1ull << 31) ? 64 : 1;
+            while (bins > 1 && bins < kMaxBins && u64(bins) * 256 < cp) bins *= 2;
+            for (u32 i0 = 0; i0 < n;) {
+                u32 i1 = i0;
+                for (u64 held = 0; i1 < n && held < kChunkPairs; ++i1) held += i1;
+                chunks.push_back(Chunk{q, i0, i1, 0, nranks});
+                nranks += bins;
+                i0 = i1;
+            }
+            bin_off[q + 1] = bin_off[q] + bins;
+            const u32 cap = bins > 1 ? u32(cp / kItemStep) + 1 : 0;
+            item_off[q + 1] = item_off[q] + cap;
+            item_cloud.insert(item_cloud.end(), cap, q);
         }
         // the segmented sort's capacity: every cloud's largest key count
         // (every pair kept) in tiles of kSegTileKeys, 256 digit counts a tile
@@ -458,7 +832,17 @@ Batch* batch_create(tt_ctx* c, const u32* sizes_h, u32 clouds, u32 dim, int kind
         b->row_cnt = b->alloc<u64>(b->total_pts);
         b->row_off = b->alloc<u64>(b->total_pts);
         b->count = b->alloc<unsigned long long>(1);
-        b->per_cloud = b->alloc<u64>(clouds);
+        b->nchunks = u32(chunks.size());
+        b->chunks = b->alloc<Chunk>(chunks.size());
+        b->total_bins = bin_off[clouds];
+        b->bin_off = b->alloc<u32>(clouds + 1);
+        b->hist = b->alloc<u32>(b->total_bins);
+        b->ranks = b->alloc<u32>(nranks);
+        b->total_items = item_off[clouds];
+        b->item_off = b->alloc<u32>(clouds + 1);
+        b->items = b->alloc<Item>(b->total_items);
+        b->item_cloud = b->alloc<u32>(b->total_items);
+        b->radix = b->alloc<u32>(clouds);
         b->edge_off = b->alloc<u64>(clouds + 1);
         b->nseg_tiles = u32(seg_cap);
         b->seg_hist = 256 * seg_cap;
@@ -471,6 +855,11 @@ Batch* batch_create(tt_ctx* c, const u32* sizes_h, u32 clouds, u32 dim, int kind
         TT_CUDA(cudaMemcpyAsync(b->mat_off, mat_off.data(), 8 * (clouds + 1), cudaMemcpyHostToDevice, s));
         TT_CUDA(cudaMemcpyAsync(b->pair_off, pair_off.data(), 8 * (clouds + 1), cudaMemcpyHostToDevice, s));
         TT_CUDA(cudaMemcpyAsync(b->sizes, sizes_h, 4 * clouds, cudaMemcpyHostToDevice, s));
+        TT_CUDA(cudaMemcpyAsync(b->chunks, chunks.data(), sizeof(Chunk) * chunks.size(), cudaMemcpyHostToDevice, s));
+        TT_CUDA(cudaMemcpyAsync(b->bin_off, bin_off.data(), 4 * (clouds + 1), cudaMemcpyHostToDevice, s));
+        TT_CUDA(cudaMemcpyAsync(b->item_off, item_off.data(), 4 * (clouds + 1), cudaMemcpyHostToDevice, s));
+        if (!item_cloud.empty())
+            TT_CUDA(cudaMemcpyAsync(b->item_cloud, item_cloud.data(), 4 * item_cloud.size(), cudaMemcpyHostToDevice, s));
         for (int si = 0; si < kNumShapes; ++si)
             TT_CUDA(cudaMemcpyAsync(b->tiles[si], tiles[si].data(), sizeof(Tile) * tiles[si].size(),
                                     cudaMemcpyHostToDevice, s));

@@ -103,9 +103,11 @@ void radix_reserve(tt_ctx* c, u64 n);   // every slot radix_sort of n keys may g
 void radix_reserve_entries(tt_ctx* c, u64 entries);   // ... a sort whose histogram has that many entries
 // A tile of the segmented sort: tile t (of tcount) of segment seg; its digit
 // counts at hbase + digit * tcount + t (segments' count blocks in segment
-// order, each 256 * tcount entries).
+// order, each 256 * tcount entries). shift: the segment's first key less the
+// number of keys of the listed segments before it (the scan of the counts
+// sees the listed segments only).
 struct SegTile {
-    u32 seg, t, hbase, tcount;
+    u32 seg, t, hbase, tcount, shift;
 };
 constexpr u32 kSegTileKeys = 4096;   // keys a tile of the segmented sort
 bool radix_sort_segments(tt_ctx* c, u64* keys, u64* kbuf, const u64* seg_off, const SegTile* tl,

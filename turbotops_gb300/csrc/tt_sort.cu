@@ -58,10 +58,18 @@ __device__ T block_exclusive_scan(T v, T* warp_tot, T* total) {
     return r;
 }
 
+// (limit, optional: *limit * unit entries hold counts; the tiles past them
+// return at once.)
+struct ScanLimit {
+    const u32* limit = nullptr;
+    u32 unit = 0;
+    __device__ __forceinline__ bool past(u64 base) const { return limit && base >= u64(*limit) * unit; }
+};
 template <typename T>
-__global__ void k_tile_sums(const T* __restrict__ in, u64 n, T* __restrict__ sums) {
+__global__ void k_tile_sums(const T* __restrict__ in, u64 n, T* __restrict__ sums, ScanLimit lim) {
     pdl_wait();
     pdl_trigger();
+    if (lim.past(u64(blockIdx.x) * SCAN_TILE)) return;
     __shared__ T wt[32];
     __shared__ T tot;
     const u64 base = u64(blockIdx.x) * SCAN_TILE;
@@ -77,9 +85,10 @@ __global__ void k_tile_sums(const T* __restrict__ in, u64 n, T* __restrict__ sum
 
 template <typename T>
 __global__ void k_tile_scan(const T* __restrict__ in, u64 n, const T* __restrict__ offs,
-                            T* __restrict__ out, T* __restrict__ total) {
+                            T* __restrict__ out, T* __restrict__ total, ScanLimit lim) {
     pdl_wait();
     pdl_trigger();
+    if (lim.past(u64(blockIdx.x) * SCAN_TILE)) return;
     __shared__ T wt[32];
     __shared__ T tot;
     const u64 base = u64(blockIdx.x) * SCAN_TILE + u64(threadIdx.x) * SCAN_ITEMS;
@@ -107,14 +116,16 @@ __global__ void k_tile_scan(const T* __restrict__ in, u64 n, const T* __restrict
 // device), counts digit-major over the tiles. SegTiles: the segmented sort,
 // tile b = keys [seg_off[s] + t RS_TILE, ...) of segment s (tiles never
 // straddle segments), counts at hbase + digit * tcount + t, so that one
-// exclusive scan of all segments' counts in order gives every key's final
-// position (segment s's counts sum to its key count).
+// exclusive scan of the listed segments' counts in order gives every key's
+// position among their keys (segment s's counts sum to its key count), and
+// the tile's shift its final position.
 // kAllBins: the count layout reserves every bin of the widest digit for
 // every tile (a segment's block of counts does not depend on the pass), so
 // a pass with narrower digits writes zeros into the bins it does not use;
 // the flat layout scans only the bins of the pass.
 struct FlatTiles {
     static constexpr bool kAllBins = false;
+    static constexpr bool kLoop = false;   // one tile a block
     u64 n;
     const unsigned long long* ndev;
     u32 tiles;
@@ -125,12 +136,14 @@ struct FlatTiles {
         hi = lo < nn ? min(lo + RS_TILE, nn) : lo;
     }
     __device__ __forceinline__ u64 hidx(u32 b, u32 d) const { return u64(d) * tiles + b; }
+    __device__ __forceinline__ u32 shift(u32) const { return 0; }
 };
 struct SegTiles {
     static constexpr bool kAllBins = true;
+    static constexpr bool kLoop = true;   // a block takes every gridDim-th tile: an empty list costs a launch
     const SegTile* tl;
     const u64* seg_off;
-    const u32* ntiles;   // tiles in the list (the grid covers its capacity)
+    const u32* ntiles;   // tiles in the list
     __device__ __forceinline__ bool valid(u32 b) const { return b < *ntiles; }
     __device__ __forceinline__ void range(u32 b, u64& lo, u64& hi) const {
         const SegTile e = tl[b];
@@ -142,6 +155,7 @@ struct SegTiles {
         const SegTile e = tl[b];
         return e.hbase + u64(d) * e.tcount + e.t;
     }
+    __device__ __forceinline__ u32 shift(u32 b) const { return tl[b].shift; }
 };
 // The lanes holding the same digit as this lane (a sentinel digit marks an
 // empty slot). A warp whose 32 digits agree, the common case once the later
@@ -160,9 +174,9 @@ k_rs_upsweep(const u64* __restrict__ keys, TM tm, int shift, u32 width, u32* __r
     pdl_wait();
     pdl_trigger();
     __shared__ u32 h[RS_WARPS][BINS];
-    if (!tm.valid(blockIdx.x)) return;   // past the list: no keys, no counts
+    for (u32 b = blockIdx.x; tm.valid(b); b += gridDim.x) {
     u64 tlo, n;   // this tile's keys: [tlo, n)
-    tm.range(blockIdx.x, tlo, n);
+    tm.range(b, tlo, n);
     const u32 nd = 1u << width, mask = nd - 1u;
     for (u32 t = threadIdx.x; t < RS_WARPS * nd; t += RS_THREADS) h[t / nd][t % nd] = 0;
     __syncthreads();
@@ -221,7 +235,10 @@ k_rs_upsweep(const u64* __restrict__ keys, TM tm, int shift, u32 width, u32* __r
 #pragma unroll
             for (int q = 0; q < RS_WARPS; ++q) s += h[q][d];
         }
-        hist[tm.hidx(blockIdx.x, d)] = s;
+        hist[tm.hidx(b, d)] = s;
+    }
+    if (!TM::kLoop) break;
+    __syncthreads();   // the counters are free again
     }
 }
 
@@ -310,16 +327,19 @@ k_rs_scatter_local(const u64* __restrict__ kin, u64* __restrict__ kout, const V*
     __shared__ u32 tstart[RS_LBINS];          // the digit's first position in the ordered tile
     __shared__ u32 wsum[RS_WARPS];
     __shared__ u32 mbins[RS_WARPS][RS_LBINS]; // per-warp lane masks by digit (the ranking below)
-    if (!tm.valid(blockIdx.x)) return;
+    for (u32 b = blockIdx.x; tm.valid(b); b += gridDim.x) {
     u64 tbase, n;   // this tile's keys: [tbase, n)
-    tm.range(blockIdx.x, tbase, n);
-    if (tbase >= n) return;
+    tm.range(b, tbase, n);
+    if (tbase >= n) {   // (block-uniform)
+        if (!TM::kLoop) break;
+        continue;
+    }
     const u32 nd = 1u << width, mask = nd - 1u;
     for (u32 t = threadIdx.x; t < RS_WARPS * RS_LBINS; t += RS_THREADS) {
         cnt[t / RS_LBINS][t % RS_LBINS] = 0;
         mbins[t / RS_LBINS][t % RS_LBINS] = 0;
     }
-    for (u32 d = threadIdx.x; d < nd; d += RS_THREADS) gbase[d] = offs[tm.hidx(blockIdx.x, d)];
+    for (u32 d = threadIdx.x; d < nd; d += RS_THREADS) gbase[d] = offs[tm.hidx(b, d)] + tm.shift(b);
     __syncthreads();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const u32 lt = (1u << lane) - 1u;
@@ -414,6 +434,9 @@ k_rs_scatter_local(const u64* __restrict__ kin, u64* __restrict__ kout, const V*
         kout[pos] = kk;
         if constexpr (VALS) vout[pos] = sval[j];
     }
+    if (!TM::kLoop) break;
+    __syncthreads();   // the shared tile is free again
+    }
 }
 static_assert(RS_LBINS == RS_THREADS, "one digit a thread in the local scatter's scan");
 static_assert(RS_TILE == int(kSegTileKeys), "the segmented sort's tiles are the radix tiles");
@@ -439,14 +462,15 @@ __global__ void k_minmax(const u64* __restrict__ keys, u64 n, unsigned long long
 }  // namespace
 
 template <typename T>
-void scan_exclusive(tt_ctx* c, const T* in, T* out, u64 n, T* total, int depth) {
+static void scan_limited(tt_ctx* c, const T* in, T* out, u64 n, T* total, int depth, ScanLimit lim) {
     if (n == 0) {
         if (total) TT_CUDA(cudaMemsetAsync(total, 0, sizeof(T), c->stream));
         return;
     }
     const u64 tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
     if (tiles == 1) {
-        launch_pdl(k_tile_scan<T>, 1, SCAN_THREADS, 0, c->stream, in, n, static_cast<const T*>(nullptr), out, total);
+        launch_pdl(k_tile_scan<T>, 1, SCAN_THREADS, 0, c->stream, in, n, static_cast<const T*>(nullptr), out, total,
+                   lim);
         TT_LAUNCH("k_tile_scan");
         c->launches += 1;
         return;
@@ -455,20 +479,25 @@ void scan_exclusive(tt_ctx* c, const T* in, T* out, u64 n, T* total, int depth) 
     // sums[0..tiles) tile totals, sums[tiles..2 tiles) their exclusive scan;
     // each recursion level has its own scratch slot
     T* sums = c->arena.get<T>(depth == 0 ? S_SCAN : depth == 1 ? S_SCAN2 : S_SCAN3, 2 * tiles + 2);
-    launch_pdl(k_tile_sums<T>, u32(tiles), SCAN_THREADS, 0, c->stream, in, n, sums);
+    launch_pdl(k_tile_sums<T>, u32(tiles), SCAN_THREADS, 0, c->stream, in, n, sums, lim);
     TT_LAUNCH("k_tile_sums");
     if (tiles <= SCAN_TILE) {
         launch_pdl(k_tile_scan<T>, 1, SCAN_THREADS, 0, c->stream, static_cast<const T*>(sums), tiles,
-                   static_cast<const T*>(nullptr), sums + tiles, static_cast<T*>(nullptr));
+                   static_cast<const T*>(nullptr), sums + tiles, static_cast<T*>(nullptr), ScanLimit{});
         TT_LAUNCH("k_tile_scan");
         c->launches += 1;
     } else {
         scan_exclusive<T>(c, sums, sums + tiles, tiles, nullptr, depth + 1);
     }
     launch_pdl(k_tile_scan<T>, u32(tiles), SCAN_THREADS, 0, c->stream, in, n, static_cast<const T*>(sums + tiles), out,
-               total);
+               total, lim);
     TT_LAUNCH("k_tile_scan");
     c->launches += 2;
+}
+
+template <typename T>
+void scan_exclusive(tt_ctx* c, const T* in, T* out, u64 n, T* total, int depth) {
+    scan_limited<T>(c, in, out, n, total, depth, ScanLimit{});
 }
 
 template void scan_exclusive<u64>(tt_ctx*, const u64*, u64*, u64, u64*, int);
@@ -558,13 +587,13 @@ template bool radix_sort<u64>(tt_ctx*, u64*, u64*, u64, u64*, u64*, int, int, co
 // scatter (runs of one digit leave a tile together); the tiles and their
 // count offsets come from the caller (SegTile), the segment bounds from the
 // device. The list's length is on the device (ntiles_dev); max_tiles and
-// hist_entries bound it and its counts (the grids and the scan cover them:
-// counts past the list's only shift prefixes past its keys). Returns whether
-// the result is in kbuf.
+// hist_entries bound it and its counts (blocks loop over the listed tiles and
+// the scan stops after their counts, so an empty list costs the launches
+// alone). Returns whether the result is in kbuf.
 bool radix_sort_segments(tt_ctx* c, u64* keys, u64* kbuf, const u64* seg_off, const SegTile* tl,
                          const u32* ntiles_dev, u32 max_tiles, u64 hist_entries, int bits, int lo_bit) {
-    const u32 ntiles = max_tiles;
-    if (ntiles == 0 || bits <= 0) return false;
+    if (max_tiles == 0 || bits <= 0) return false;
+    const u32 ntiles = std::min<u32>(max_tiles, 8 * u32(kSMs));   // blocks (they loop over the listed tiles)
     u32* hist = c->arena.get<u32>(S_SORT_HIST, hist_entries + 1);
     u64 *ka = keys, *kb = kbuf;
     bool swapped = false;
@@ -576,7 +605,7 @@ bool radix_sort_segments(tt_ctx* c, u64* keys, u64* kbuf, const u64* seg_off, co
         launch_pdl(k_rs_upsweep<RS_LBINS, SegTiles>, ntiles, RS_THREADS, 0, c->stream, static_cast<const u64*>(ka), tm, shift,
                    u32(width), hist);
         TT_LAUNCH("k_rs_upsweep");
-        scan_exclusive<u32>(c, hist, hist, hist_entries, nullptr, 0);
+        scan_limited<u32>(c, hist, hist, hist_entries, nullptr, 0, ScanLimit{ntiles_dev, 256});
         launch_pdl(k_rs_scatter_local<u32, false, SegTiles>, ntiles, RS_THREADS, 0, c->stream,
                    static_cast<const u64*>(ka), kb, static_cast<const u32*>(nullptr), static_cast<u32*>(nullptr), tm,
                    shift, u32(width), static_cast<const u32*>(hist));
