@@ -138,7 +138,7 @@ enum Slot : int {
     S_TXT, S_TXT_CNT, S_TXT_LINES, S_TXT_TOK, S_TXT_HOST,          // text ingestion
     S_DIM0_ERR,                                                    // dim0's announced-count check
     S_MST_KB, S_MST_Q, S_MST_C, S_MST_OUT,                         // MST: interior bounds, scanned points, components, deaths
-    S_NEAR_X, S_NEAR_ID, S_NEAR_BOX, S_NEAR_ST,                    // points in spatial order (tt_near.cuh)
+    S_NEAR_X, S_NEAR_ID, S_NEAR_BOX, S_NEAR_ST, S_NEAR_SEP,                    // points in spatial order (tt_near.cuh)
     S_NSLOTS
 };
 

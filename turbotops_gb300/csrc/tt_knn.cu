@@ -290,46 +290,64 @@ void knn_tc(tt_ctx* c, const f32* x, u32 n, u32 k, u32* ids, f32* dists, bool de
 void knn_tc_settle(tt_ctx* c);
 
 namespace {
-// rank[p] = position of pivot p (point floor(p n / P)) when the pivots are
-// sorted by the nearest of the first C of C strided ones among them, so that
-// neighbouring cells of the order lie close together. One block, P <= 256.
-__global__ void __launch_bounds__(256) k_pivot_rank(const f32* __restrict__ x, u32 n, u32 dim, u32 P, u32 C,
-                                                    u32* __restrict__ rank) {
+// Squared distances between the pivots (points floor(p n / P)): a block a row.
+constexpr u32 kMaxPivots = 192;
+__global__ void __launch_bounds__(256) k_pivot_dist(const f32* __restrict__ x, u32 n, u32 dim, u32 P,
+                                                    f32* __restrict__ dist) {
     pdl_wait();
     pdl_trigger();
-    __shared__ u32 group[256];
-    const u32 p = threadIdx.x;
-    const f32* a = x + (u64(p) * n / P) * dim;
-    u32 best = 0;
-    if (p < P) {
-        f32 bd = INFINITY;
-        for (u32 c = 0; c < C; ++c) {
-            const f32* b = x + (u64(c * P / C) * n / P) * dim;
-            f32 s = 0.0f;
-            for (u32 k = 0; k < dim; ++k) {
-                const f32 u = a[k] - b[k];
-                s = fmaf(u, u, s);
-            }
-            if (s < bd) bd = s, best = c;
-        }
-        group[p] = best;
+    const u32 a = blockIdx.x, b = threadIdx.x;
+    if (b >= P) return;
+    const f32 *xa = x + (u64(a) * n / P) * dim, *xb = x + (u64(b) * n / P) * dim;
+    f32 s = 0.0f;
+#pragma unroll 8
+    for (u32 k = 0; k < dim; ++k) {
+        const f32 u = __ldg(xa + k) - __ldg(xb + k);
+        s = fmaf(u, u, s);
     }
-    __syncthreads();
-    if (p >= P) return;
-    u32 r = 0;
-    for (u32 q = 0; q < P; ++q) r += group[q] < best || (group[q] == best && q < p);
-    rank[p] = r;
+    dist[a * P + b] = s;
 }
 
-// Each point's cell: the rank of the nearest of P strided pivot points
+// rank[p] = position of pivot p on a nearest-first chain from pivot 0 (ties to
+// the lower index), so that neighbouring cells of the order lie close together
+// (sorting the pivots by a coarser set of 16 left cells of different clusters
+// side by side, and a quarter of the 128-point blocks straddled two). One
+// block: the distances into shared memory, then one warp walks the chain.
+__global__ void __launch_bounds__(1024) k_pivot_rank(const f32* __restrict__ dist, u32 P, u32* __restrict__ rank) {
+    pdl_wait();
+    pdl_trigger();
+    extern __shared__ f32 dm[];   // P x P
+    for (u32 t = threadIdx.x; t < P * P; t += blockDim.x) dm[t] = dist[t];
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    const u32 lane = threadIdx.x;
+    u32 visited = lane == 0 ? 1u : 0u;   // bit i: pivot lane + 32 i is on the chain
+    if (lane == 0) rank[0] = 0;
+    u32 cur = 0;
+    for (u32 step = 1; step < P; ++step) {
+        u32 bd = 0xffffffffu, bp = 0xffffffffu;   // this lane's nearest unvisited pivot
+        for (u32 i = 0, p = lane; p < P; ++i, p += 32) {
+            const u32 db = fbits(dm[cur * P + p]);
+            if (!((visited >> i) & 1u) && (bp == 0xffffffffu || db < bd)) {
+                bd = db;
+                bp = p;
+            }
+        }
+        const u32 md = __reduce_min_sync(0xffffffffu, bd);
+        cur = __reduce_min_sync(0xffffffffu, bp != 0xffffffffu && bd == md ? bp : 0xffffffffu);
+        if (lane == 0) rank[cur] = step;
+        if ((cur & 31u) == lane) visited |= 1u << (cur >> 5);
+    }
+}
+
+// Each point's cell: the index of the nearest of P strided pivot points
 // (squared L2 from |p|^2 - 2 x.p; ties to the lower pivot), the pivots' rows
 // in shared memory (zero-padded to DP, a multiple of 4), the point's
-// coordinates in registers. 100,000 x 32: 195 pivots in 87 us (65 pivots took
+// coordinates in registers. 100,000 x 32: 192 pivots in 84 us (65 pivots took
 // 837 us with the coordinates read from memory for every pivot).
 template <int DP>
 __global__ void __launch_bounds__(128) k_pivot_cell(const f32* __restrict__ x, u32 n, u32 dim, u32 P,
-                                                    const u32* __restrict__ rank, u64* __restrict__ key,
-                                                    u32* __restrict__ val) {
+                                                    u64* __restrict__ key, u32* __restrict__ val) {
     pdl_wait();
     pdl_trigger();
     extern __shared__ float4 pv4[];   // P x DP / 4, then the norms
@@ -365,11 +383,16 @@ __global__ void __launch_bounds__(128) k_pivot_cell(const f32* __restrict__ x, u
             const f32 e = fmaf(-2.0f, (s[0] + s[1]) + (s[2] + s[3]), pn[q]);
             if (e < bd) bd = e, best = q;
         }
-        key[i] = rank[best];
+        key[i] = best;
         val[i] = i;
     }
 }
 }  // namespace
+
+// key[i] = the rank of point i's pivot.
+__global__ void k_pivot_key(const u32* __restrict__ rank, u32 n, u64* __restrict__ key) {
+    for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) key[i] = rank[u32(key[i])];
+}
 
 // The points sorted by cell, the cells of neighbouring pivots next to each
 // other: about n / 512 cells (as many as 48 KB of shared memory hold).
@@ -379,16 +402,22 @@ __global__ void __launch_bounds__(128) k_pivot_cell(const f32* __restrict__ x, u
 // points.
 const u32* pivot_order(tt_ctx* c, const f32* x, u32 n, u32 dim) {
     const u32 dp = dim <= 4 ? 4 : near::padded_dim(dim);
-    const u32 P = std::max<u32>(2, std::min<u32>({256u, 12000u / (dp + 1), n / 512}));
+    const u32 P = std::max<u32>(2, std::min<u32>({kMaxPivots, 12000u / (dp + 1), n / 512}));
     u64* key = c->arena.get<u64>(S_TC_KEYS, n);
     u32* val = c->arena.get<u32>(S_TC_VALS, n);
-    u32* rank = c->arena.get<u32>(S_TC_PIV, P);
-    launch_pdl(k_pivot_rank, 1, 256, 0, c->stream, x, n, dim, P, std::min<u32>(P, 16), rank);
+    f32* dist = c->arena.get<f32>(S_TC_PIV, u64(P) * P + P);
+    u32* rank = reinterpret_cast<u32*>(dist + u64(P) * P);
+    SideScope side(c);   // the chain (one block) beside the assignment
+    const cudaStream_t ps = side.fork();
+    k_pivot_dist<<<P, 256, 0, ps>>>(x, n, dim, P, dist);
+    TT_CUDA(cudaFuncSetAttribute(k_pivot_rank, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 int(kMaxPivots * kMaxPivots * sizeof(f32))));
+    k_pivot_rank<<<1, 1024, P * P * sizeof(f32), ps>>>(dist, P, rank);
     TT_LAUNCH("k_pivot_rank");
     auto cell = [&](auto d) {
         constexpr int DP = decltype(d)::value;
         launch_pdl(k_pivot_cell<DP>, std::min<u32>(div_up(n, 128), 8 * u32(c->sms)), 128, sizeof(f32) * P * (DP + 1),
-                   c->stream, x, n, dim, P, static_cast<const u32*>(rank), key, val);
+                   c->stream, x, n, dim, P, key, val);
     };
     switch (dp) {
         case 4: cell(std::integral_constant<int, 4>{}); break;
@@ -399,7 +428,10 @@ const u32* pivot_order(tt_ctx* c, const f32* x, u32 n, u32 dim) {
         default: cell(std::integral_constant<int, 64>{}); break;
     }
     TT_LAUNCH("k_pivot_cell");
-    c->launches += 2;
+    side.join();
+    k_pivot_key<<<std::min<u32>(div_up(n, 256), 4 * u32(c->sms)), 256, 0, c->stream>>>(rank, n, key);
+    TT_LAUNCH("k_pivot_key");
+    c->launches += 4;
     u64* kb = c->arena.get<u64>(S_SORT_A, n);
     u32* vb = c->arena.get<u32>(S_SORT_VA, n);
     return radix_sort<u32>(c, key, val, n, kb, vb, 32 - __builtin_clz(P - 1)) ? vb : val;
@@ -416,7 +448,7 @@ static bool near_applicable(u32 n, u32 dim, int kind) {
     return kind != M_LP && n >= kNearMin && dim >= 1 && dim <= near::kMaxDim;
 }
 // Lp lists: up to exponent kLpMax, where the filter's margin is derived
-// (100,000 x 32 mixture points, L1.5: exhaustive 390 ms, ordered 13.5 ms).
+// (100,000 x 32 mixture points, L1.5: exhaustive 390 ms, ordered 6.7 ms).
 static bool near_lp_applicable(u32 n, u32 dim, int kind, f32 p) {
     return kind == M_LP && p <= near::kLpMax && n >= kNearMin && dim >= 1 && dim <= near::kMaxDim;
 }
@@ -438,12 +470,21 @@ void knn_exact(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, u32 k, 
         return;
     }
     if (c->knn_mode == 0 && near_applicable(n, dim, kind) && k <= 32) {
-        near_lists(c, order_known ? *order_known : near::near_order(c, x, n, dim), dim, kind, k, ids, dists);
+        near::View v;
+        if (order_known) {
+            v = *order_known;
+        } else {
+            v = near::near_order(c, x, n, dim);
+            near::near_separations(c, v, dim, kind, p);
+        }
+        near_lists(c, v, dim, kind, k, ids, dists);
         if (!defer) TT_CUDA(cudaStreamSynchronize(c->stream));
         return;
     }
     if (c->knn_mode == 0 && near_lp_applicable(n, dim, kind, p) && k <= 32) {
-        near::near_knn_lp(c, near::near_order(c, x, n, dim), dim, p, k, ids, dists);
+        near::View v = near::near_order(c, x, n, dim);
+        near::near_separations(c, v, dim, kind, p);
+        near::near_knn_lp(c, v, dim, p, k, ids, dists);
         if (!defer) TT_CUDA(cudaStreamSynchronize(c->stream));
         return;
     }

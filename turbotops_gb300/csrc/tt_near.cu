@@ -142,6 +142,112 @@ __global__ void __launch_bounds__(128) k_near_super(const f32* __restrict__ tbox
     }
 }
 
+// ---- separations between blocks ---------------------------------------------
+// For blocks A and B of 128 points (4 tiles): with u = u_AB the gradient of
+// the distance at D = c_B - c_A (tt_near.cuh, project) and x in B, q in A,
+// |x - q|_p |u|_p' >= u . (x - q) >= min over B of u . x - max over A of u . q,
+// and u_BA = -u_AB, so with S_AB = min over x in B of u_AB . (x - r) the
+// separation is (S_AB + S_BA) / |u|_p' (any common reference r). One block a
+// B: its points relative to r in registers, the directions to 32 blocks A at a
+// time in shared memory. Rounding: a sum of DP terms errs by less than 2^-16
+// of sum |u_k| ext_k, ext the block's largest |x_k - r_k|, which is taken off
+// S; |u|_p' is taken 2^-9 up. A non-finite value anywhere ends in a separation
+// of 0. FP32 issue bound: 100,000 x 32 (781 blocks, 2.5e9 multiply-adds) 0.24 ms.
+__global__ void __launch_bounds__(64) k_near_centres(const f32* __restrict__ abox, u32 ntiles, u32 dp,
+                                                     f32* __restrict__ cen) {
+    pdl_wait();
+    pdl_trigger();
+    const u32 b = blockIdx.x, k = threadIdx.x;
+    if (k >= dp) return;
+    f32 lo = INFINITY, hi = -INFINITY;
+    for (u32 t = b * kBlockTiles; t < min(ntiles, (b + 1) * kBlockTiles); ++t) {
+        lo = fminf(lo, abox[(u64(t) * 2) * dp + k]);
+        hi = fmaxf(hi, abox[(u64(t) * 2 + 1) * dp + k]);
+    }
+    cen[u64(b) * dp + k] = 0.5f * lo + 0.5f * hi;
+}
+
+template <int DP>
+__global__ void __launch_bounds__(128) k_near_sep(const f32* __restrict__ xt, const u32* __restrict__ id,
+                                                  const f32* __restrict__ cen, u32 ntiles, u32 nblk, int kind, f32 p,
+                                                  float2* __restrict__ out) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ alignas(16) f32 su[32][DP];
+    __shared__ f32 ext[DP], part[32][4];
+    const u32 B = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const u32 tile = B * kBlockTiles + w;
+    const bool live = tile < ntiles && id[tile * kTile + lane] != 0xffffffffu;
+    f32 y[DP];
+    if (tid < DP) ext[tid] = 0.0f;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < DP; ++k) {
+        y[k] = live ? __fsub_rn(xt[(u64(tile) * DP + k) * kTile + lane], cen[k]) : 0.0f;   // r: block 0's centre
+        const u32 a = __float_as_uint(fabsf(y[k]));   // (a NaN's bits are above every number's)
+        const u32 m = __reduce_max_sync(0xffffffffu, a);
+        if (lane == 0) atomicMax(reinterpret_cast<u32*>(&ext[k]), m);
+    }
+    const f32 pd = p / (p - 1.0f);   // (used for Lp only: p > 1)
+    for (u32 A0 = blockIdx.y * 32; A0 < nblk; A0 += gridDim.y * 32) {
+        __syncthreads();
+        for (u32 e = tid; e < 32 * DP; e += 128) {
+            const u32 a = e / DP, k = e % DP;
+            f32 u = 0.0f;
+            if (A0 + a < nblk) {
+                const f32 d = cen[u64(B) * DP + k] - cen[u64(A0 + a) * DP + k];
+                u = kind == M_L2 ? d
+                    : kind == M_L1 ? (d < 0.0f ? -1.0f : d > 0.0f ? 1.0f : 0.0f)
+                                   : copysignf(__powf(fabsf(d), p - 1.0f), d);
+                if (kind == M_LP && d == 0.0f) u = 0.0f;
+            }
+            su[a][k] = u;
+        }
+        __syncthreads();
+#pragma unroll 2
+        for (u32 a = 0; a < 32; ++a) {
+            f32 s[2] = {0.0f, 0.0f};
+            const float4* u4 = reinterpret_cast<const float4*>(su[a]);
+#pragma unroll
+            for (int k = 0; k < DP / 4; ++k) {
+                const float4 u = u4[k];
+                s[0] = fmaf(u.x, y[4 * k], s[0]);
+                s[1] = fmaf(u.y, y[4 * k + 1], s[1]);
+                s[0] = fmaf(u.z, y[4 * k + 2], s[0]);
+                s[1] = fmaf(u.w, y[4 * k + 3], s[1]);
+            }
+            // (a NaN projection counts as -inf: no separation)
+            const f32 v = s[0] + s[1];
+            const u32 m = __reduce_min_sync(0xffffffffu, ordered(!live ? INFINITY : v == v ? v : -INFINITY));
+            if (lane == 0) part[a][w] = from_ordered(m);
+        }
+        __syncthreads();
+        if (tid < 32 && A0 + tid < nblk) {
+            const f32 s = fminf(fminf(part[tid][0], part[tid][1]), fminf(part[tid][2], part[tid][3]));
+            f32 mag = 0.0f, nrm = 0.0f;
+            for (int k = 0; k < DP; ++k) {
+                const f32 u = fabsf(su[tid][k]);
+                mag = fmaf(u, ext[k], mag);
+                nrm += kind == M_L2 ? u * u : kind == M_L1 ? 0.0f : __powf(u, pd);
+            }
+            if (kind == M_L1) nrm = 1.0f;
+            else nrm = nrm >= 0x1p-100f ? (kind == M_L2 ? sqrtf(nrm) : __powf(nrm, 1.0f / pd)) : INFINITY;
+            out[u64(A0 + tid) * nblk + B] = make_float2(s - 0x1p-16f * mag, nrm * (1.0f + 0x1p-9f));
+        }
+    }
+}
+
+// sep[A][B] from both directions' sums.
+__global__ void __launch_bounds__(256) k_near_sep_join(const float2* __restrict__ s, u32 nblk, f32* __restrict__ sep) {
+    pdl_wait();
+    pdl_trigger();
+    const u32 B = blockIdx.x * blockDim.x + threadIdx.x, A = blockIdx.y;
+    if (B >= nblk) return;
+    const float2 ab = s[u64(A) * nblk + B], ba = s[u64(B) * nblk + A];
+    const f32 g = (ab.x + ba.x) * (1.0f - 0x1p-20f) / fmaxf(ab.y, ba.y);
+    sep[u64(A) * nblk + B] = A != B && g > 0.0f && g < INFINITY ? g : 0.0f;
+}
+
 // A block takes a super tile, a warp a tile of it.
 __global__ void __launch_bounds__(1024) k_near_components(const u32* __restrict__ id, u32 ntiles,
                                                           const u32* __restrict__ comp, u32* __restrict__ cpos,
@@ -207,6 +313,35 @@ void near_queries(tt_ctx* c, const View& v, u32 dim, const u32* cpos, const unsi
                cpos, near, kb, bd, queries_per_warp(padded_dim(dim)), qlist, nq);
     TT_LAUNCH("k_near_queries");
     ++c->launches;
+}
+
+// Slots: S_NEAR_SEP (result), S_NEAR_ST.
+void near_separations(tt_ctx* c, View& v, u32 dim, int kind, f32 p) {
+    const u32 dp = padded_dim(dim);
+    v.nblk = div_up(v.ntiles, kBlockTiles);
+    if (dp < kProjectDim || kind == M_LINF || v.n < kSepMinPoints || v.nblk > kSepMaxBlocks) return;
+    const u64 pairs = u64(v.nblk) * v.nblk;
+    f32* cen = c->arena.get<f32>(S_NEAR_ST, std::max<u64>(u64(v.nblk) * dp, 2 * kCodeDims));
+    f32* sep = c->arena.get<f32>(S_NEAR_SEP, 3 * pairs + 2);
+    float2* s = reinterpret_cast<float2*>(sep + ((pairs + 1) & ~u64(1)));
+    launch_pdl(k_near_centres, v.nblk, 64, 0, c->stream, v.abox, v.ntiles, dp, cen);
+    TT_LAUNCH("k_near_centres");
+    // enough blocks for the chip when there are few Bs
+    const dim3 grid(v.nblk, std::min<u32>(div_up(v.nblk, 32), std::max<u32>(1, 1216 / v.nblk)));
+    auto go = [&](auto d) {
+        launch_pdl(k_near_sep<decltype(d)::value>, grid, 128, 0, c->stream, v.xt, v.id, static_cast<const f32*>(cen),
+                   v.ntiles, v.nblk, kind, p, s);
+    };
+    if (dp == 16) go(std::integral_constant<int, 16>{});
+    else if (dp == 32) go(std::integral_constant<int, 32>{});
+    else if (dp == 48) go(std::integral_constant<int, 48>{});
+    else go(std::integral_constant<int, 64>{});
+    TT_LAUNCH("k_near_sep");
+    launch_pdl(k_near_sep_join, dim3(div_up(v.nblk, 256), v.nblk), 256, 0, c->stream, static_cast<const float2*>(s),
+               v.nblk, sep);
+    TT_LAUNCH("k_near_sep_join");
+    c->launches += 3;
+    v.sep = sep;
 }
 
 // Slots: S_NEAR_X, S_NEAR_ID, S_NEAR_BOX (results); S_TC_KEYS, S_TC_VALS,

@@ -53,6 +53,8 @@ struct View {
     const f32* tbox = nullptr;   // [2 * dp][tpad]
     const f32* sbox = nullptr;   // [2 * dp][spad]
     const f32* abox = nullptr;   // [ntiles][2][dp]: the tiles' corners again (dp >= kProjectDim; else null)
+    const f32* sep = nullptr;    // [nblk][nblk]: lower bounds between blocks of 4 tiles (near_separations; or null)
+    u32 nblk = 0;
     u32 n = 0, ntiles = 0, nsup = 0, tpad = 0, spad = 0;
     f32 p = 2.0f;    // Lp: the exponent
 };
@@ -67,6 +69,11 @@ inline u32 padded_dim(u32 dim) {
 constexpr u32 queries_per_warp(u32 dp) { return dp <= 4 ? 1 : dp <= 8 ? 2 : dp <= 16 ? 4 : 8; }
 
 // tt_near.cu
+constexpr u32 kBlockTiles = 4;          // tiles a separation block
+constexpr u32 kSepMaxBlocks = 4096;     // 64 MB of separations
+constexpr u32 kSepMinPoints = 2048;
+// Fills v.sep for the metric where it pays (kProjectDim, L1, L2, Lp).
+void near_separations(tt_ctx* c, View& v, u32 dim, int kind, f32 p);
 View near_order(tt_ctx* c, const f32* x, u32 n, u32 dim);
 
 // tt_near_<kind>.cu
@@ -190,6 +197,7 @@ struct WarpQ {
     alignas(16) f32 qt[DP][QW];   // the same, coordinate-major
     f32 thr[QW];   // eval values above it cannot matter (negative: no query)
     f32 bnd[QW];   // distances above it cannot matter (bound_margin)
+    u32 blk[QW];   // its separation block
     u32 own[QW];
 };
 
@@ -254,9 +262,11 @@ __device__ __forceinline__ u32 box_needs(const f32* __restrict__ box, u32 pad, u
 // to the queries' centre g; each errs by at most (DP + 2) 2^-24 of
 // sum |u_k| |x_k - g_k|, which the box corners bound (err: 2^-17 times
 // both sides' sums); |u|_p' is taken 2^-9 up.
-// (100,000 mixture points in R^32: the foreign searches of a spanning tree 45
-// ms with the boxes alone, 30 ms with the directions; L1.5 lists: 20 % of the
-// tiles pass the boxes of 8 queries, 6 % are their own cluster's.)
+// The same test between blocks of 128 points, tabulated once (tt_near.cu
+// near_separations), replaces the boxes where it is built.
+// (100,000 mixture points in R^32: the foreign searches of a spanning tree take
+// 45 ms with the boxes alone, 30 with the directions, 9.7 with the table and
+// the bounds refreshed; L1.5 lists 13.5 ms, 6.7 with the table.)
 template <int DP>
 struct Direction {
     alignas(16) f32 g[DP];     // the queries' centre
@@ -359,6 +369,7 @@ __device__ __forceinline__ u32 project(const View& v, const WarpQ<DP, QW>& W, Di
 struct SkipNone {
     __device__ __forceinline__ bool tile(u32) const { return false; }
     __device__ __forceinline__ bool super(u32) const { return false; }
+    __device__ __forceinline__ void refresh() const {}   // bounds that other warps lower
 };
 
 // Walks the tiles in reach of the warp's queries; visit(tile, coordinates,
@@ -380,14 +391,15 @@ __device__ __forceinline__ void walk(const View& v, WarpQ<DP, QW>& W, DirectionO
         }
         return m;
     };
-    auto load_visit = [&](u32 tile, u32 need) -> bool {
+    // along: worth a test along the direction to the tile
+    auto load_visit = [&](u32 tile, u32 need, bool along = true) -> bool {
         f32 c[DP];
         const f32* xt = v.xt + u64(tile) * (DP * kTile) + lane;
 #pragma unroll
         for (int k = 0; k < DP; ++k) c[k] = __ldg(xt + k * kTile);
         const u32 cid = __ldg(v.id + tile * kTile + lane);
         if constexpr (projects<KIND, DP>()) {
-            if (tile != home) {
+            if (along && tile != home) {
                 need = project<KIND, DP, QW>(v, W, D, tile, c, cid != 0xffffffffu, need);
                 if (!need) return false;
             }
@@ -416,6 +428,43 @@ __device__ __forceinline__ void walk(const View& v, WarpQ<DP, QW>& W, DirectionO
             if (load_visit(s * 32 + src, QW == 1 ? 1u : __shfl_sync(0xffffffffu, need, src))) thr = group_thr();
         }
     };
+    if constexpr (projects<KIND, DP>()) {
+        if (v.sep) {
+            // Separations between blocks of points instead of boxes: 32 blocks
+            // a test, the closest first, then the block's tiles (each tested
+            // along its own direction before its candidates are).
+            const u32 hb = home / kBlockTiles;
+            const u32 mine = lane < QW ? W.blk[lane] : W.blk[0];
+            const bool one = __all_sync(0xffffffffu, mine == hb);
+            const u32 br = (v.nblk + 31) / 32, b0 = hb / 32;
+            for (u32 r = 0; r < br; ++r) {   // the home round first
+                const u32 base = (r == 0 ? b0 : r <= b0 ? r - 1 : r) * 32;
+                const u32 t = base + lane;
+                u32 b = 0xffffffffu;
+                if (t < v.nblk) {
+                    f32 d = __ldg(v.sep + u64(hb) * v.nblk + t);
+                    if (!one)
+                        for (int q = 0; q < QW; ++q) d = fminf(d, __ldg(v.sep + u64(W.blk[q]) * v.nblk + t));
+                    b = __float_as_uint(d);
+                }
+                for (;;) {
+                    skip.refresh();
+                    f32 far = lane < QW ? W.bnd[lane] : 0.0f;   // the largest distance that still matters
+#pragma unroll
+                    for (int o = 16; o; o >>= 1) far = fmaxf(far, __shfl_xor_sync(0xffffffffu, far, o));
+                    const u32 m = __reduce_min_sync(0xffffffffu, b);
+                    if (m == 0xffffffffu || __uint_as_float(m) > far) break;
+                    const u32 src = u32(__ffs(__ballot_sync(0xffffffffu, b == m)) - 1);
+                    if (lane == src) b = 0xffffffffu;
+                    for (u32 tile = (base + src) * kBlockTiles;
+                         tile < min(v.ntiles, (base + src + 1) * kBlockTiles); ++tile)
+                        if (tile != home && !skip.tile(tile))   // (blocks that overlap: no direction helps)
+                            load_visit(tile, (1u << QW) - 1u, m != 0u);
+                }
+            }
+            return;
+        }
+    }
     if (!skip.super(s0)) descend(s0);
     const u32 rounds = (v.nsup + 31) / 32, r0 = s0 / 32;
     for (u32 r = 0; r < rounds; ++r) {   // the home round first
@@ -445,6 +494,7 @@ __device__ __forceinline__ void load_queries(const View& v, u32 p0, f32 thr0, Wa
         const u32 p = p0 + lane;
         W.thr[lane] = p < v.n ? thr0 : -1.0f;
         W.bnd[lane] = p < v.n ? INFINITY : 0.0f;
+        W.blk[lane] = p0 / (kTile * kBlockTiles);
         W.own[lane] = p < v.n ? v.id[p] : 0xffffffffu;
     }
     __syncwarp();
@@ -576,8 +626,8 @@ __global__ void __launch_bounds__(32 * kWarps)
 // coordinate differences, as rounded, are at least the gap's.
 // Survivors are queued and evaluated 32 at a time, one a lane, so that the
 // long exact path runs in full warps.
-// 100,000 x 32 mixture points, L1.5, k = 15: 13.5 ms, 2.1 instructions a cycle
-// (exhaustive scan with early exits: 390 ms). Bound by issue and the
+// 100,000 x 32 mixture points, L1.5, k = 15: 6.7 ms (exhaustive scan with early
+// exits: 390 ms). Bound by issue and the
 // special-function unit (one square root a coordinate).
 template <int KIND>
 __device__ __forceinline__ f32 lp_thr(f32 d, f32 p) {
@@ -693,10 +743,27 @@ __global__ void __launch_bounds__(32 * kWarps)
 // edge index. A query without a candidate within the bound leaves ~0.
 constexpr u32 kMixed = 0xfffffffeu, kNoComp = 0xffffffffu;
 
+template <int KIND, typename WQ>
 struct SkipComp {
     const u32* tcomp;
     const u32* scomp;
     u32 comp;   // the queries' shared component, or kNoComp
+    WQ* W;
+    const u32* cq;   // the queries' components
+    u32 queries;
+    const u32* bd;
+    // takes up the components' bounds as other warps have left them
+    __device__ __forceinline__ void refresh() const {
+        const u32 lane = threadIdx.x & 31;
+        if (lane < queries && cq[lane] != kNoComp) {
+            const u32 b = *reinterpret_cast<const volatile u32*>(bd + cq[lane]);
+            if (b != 0xffffffffu) {
+                W->thr[lane] = fminf(W->thr[lane], bound_of<KIND>(__uint_as_float(b)));
+                W->bnd[lane] = fminf(W->bnd[lane], bound_margin(__uint_as_float(b)));
+            }
+        }
+        __syncwarp();
+    }
     __device__ __forceinline__ bool tile(u32 t) const { return __ldg(tcomp + t) == comp; }
     __device__ __forceinline__ bool super(u32 s) const { return __ldg(scomp + s) == comp; }
 };
@@ -734,6 +801,7 @@ __global__ void __launch_bounds__(32 * kWarps)
     const u32 first = __ballot_sync(0xffffffffu, mypos != 0xffffffffu);   // never empty: lists start groups with a query
     const u32 p_home = __shfl_sync(0xffffffffu, mypos, __ffs(first) - 1);
     const u32 c_home = __shfl_sync(0xffffffffu, mycomp, __ffs(first) - 1);
+    if (lane < QW) W.blk[lane] = (mypos != 0xffffffffu ? mypos : p_home) / (kTile * kBlockTiles);
     const bool one = __all_sync(0xffffffffu, mypos == 0xffffffffu || mycomp == c_home);
 #pragma unroll 1
     for (u32 e = lane; e < QW * DP; e += 32) {
@@ -742,7 +810,7 @@ __global__ void __launch_bounds__(32 * kWarps)
         W.q[q][k] = W.qt[k][q] = v.xt[u64(p / kTile) * (DP * kTile) + k * kTile + p % kTile];
     }
     __syncwarp();
-    const SkipComp skip{tcomp, scomp, one ? c_home : kNoComp};
+    const SkipComp<KIND, WarpQ<DP, QW>> skip{tcomp, scomp, one ? c_home : kNoComp, &W, cq, QW, bd};
     walk<KIND, DP, CH, QW>(
         v, W, sd[projects<KIND, DP>() ? w : 0], p_home / kTile,
         [&](u32 tile, const f32(&c)[DP], u32 cid, u32 need) -> bool {
