@@ -164,9 +164,10 @@ u64 assemble2(tt_ctx* c, const Complex& cx, const u64* keys, u64 m, const u64* p
 
 // ---- tt_knn.cu
 namespace near { struct View; }
-// (order: the points' spatial order if the caller has it)
+// (order, optional: the points' spatial order, if the caller has it (order->xt);
+// else the order the lists were made in is left there, if there is one)
 void knn_exact(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, u32 k, u32* ids, f32* dists,
-               bool defer = false, const near::View* order = nullptr);
+               bool defer = false, near::View* order = nullptr);
 const u32* pivot_order(tt_ctx* c, const f32* x, u32 n, u32 dim);   // the points sorted by nearest pivot
 double tc_gram_check(tt_ctx* c, u32 products, u64 seed);   // tt_knn_tc.cu
 void selftest_wait_timeout(tt_ctx* c, u32 polls);           // tt_diag.cu

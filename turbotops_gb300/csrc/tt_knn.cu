@@ -461,7 +461,7 @@ static void near_lists(tt_ctx* c, const near::View& v, u32 dim, int kind, u32 k,
 }
 
 void knn_exact(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, u32 k, u32* ids, f32* dists, bool defer,
-               const near::View* order_known) {
+               near::View* order) {
     if (k == 0 || n < 2) return;
     // L2 in R^32: the tensor-core Gram filter (tt_knn_tc.cu) unless the
     // context asks for the exhaustive scan; both give the same lists
@@ -471,11 +471,12 @@ void knn_exact(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, u32 k, 
     }
     if (c->knn_mode == 0 && near_applicable(n, dim, kind) && k <= 32) {
         near::View v;
-        if (order_known) {
-            v = *order_known;
+        if (order && order->xt) {
+            v = *order;
         } else {
             v = near::near_order(c, x, n, dim);
             near::near_separations(c, v, dim, kind, p);
+            if (order) *order = v;
         }
         near_lists(c, v, dim, kind, k, ids, dists);
         if (!defer) TT_CUDA(cudaStreamSynchronize(c->stream));
@@ -490,9 +491,9 @@ void knn_exact(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, u32 k, 
     }
     u32* err = error_word(c);
     // (dimensions the scans refuse keep their own error: no order for them)
-    const u32* order = kind == M_LP && n >= 4096 && dim <= scan::kMaxDim ? pivot_order(c, x, n, dim) : nullptr;
-    if (k <= 16) scan_all(c, kind, x, n, dim, p, KnnOp<16>{ids, dists, k, order}, nullptr, err);
-    else if (k <= 32) scan_all(c, kind, x, n, dim, p, KnnOp<32>{ids, dists, k, order}, nullptr, err);
+    const u32* queries = kind == M_LP && n >= 4096 && dim <= scan::kMaxDim ? pivot_order(c, x, n, dim) : nullptr;
+    if (k <= 16) scan_all(c, kind, x, n, dim, p, KnnOp<16>{ids, dists, k, queries}, nullptr, err);
+    else if (k <= 32) scan_all(c, kind, x, n, dim, p, KnnOp<32>{ids, dists, k, queries}, nullptr, err);
     else invalid("gb300: exact kNN supports k <= 32");
     check_error_word(c, err);
 }

@@ -161,18 +161,20 @@ u64 mst_deaths(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, f32* de
     f32* kd = nullptr;
     near::View v;
     u32 *cpos = nullptr, *tcomp = nullptr, *scomp = nullptr;
-    if (ordered) {
-        v = near::near_order(c, x, n, dim);
-        near::near_separations(c, v, dim, kind, p);
-        cpos = c->arena.get<u32>(S_MST_C, u64(v.ntiles) * (near::kTile + 1) + v.nsup);
-        tcomp = cpos + u64(v.ntiles) * near::kTile;
-        scomp = tcomp + v.ntiles;
-    }
     if (lists) {
         kid = c->arena.get<u32>(S_KNN_I, u64(n) * K + 1);
         kd = c->arena.get<f32>(S_KNN_D, u64(n) * K + 1);
-        knn_exact(c, x, n, dim, kind, p, K, kid, kd, false, ordered ? &v : nullptr);
+        knn_exact(c, x, n, dim, kind, p, K, kid, kd, false, ordered ? &v : nullptr);   // ... and its order
         settle_finite(c);   // a pending check of the points: a NaN leaves a list short
+    }
+    if (ordered) {
+        if (!v.xt) {   // the tensor-core lists keep their own order
+            v = near::near_order(c, x, n, dim);
+            near::near_separations(c, v, dim, kind, p);
+        }
+        cpos = c->arena.get<u32>(S_MST_C, u64(v.ntiles) * (near::kTile + 1) + v.nsup);
+        tcomp = cpos + u64(v.ntiles) * near::kTile;
+        scomp = tcomp + v.ntiles;
     }
     u32* kb = lists ? c->arena.get<u32>(S_MST_KB, n + 1) : nullptr;
     u32* qlist = lists ? c->arena.get<u32>(S_MST_Q, u64(n) + 2 + near::kTile) : nullptr;

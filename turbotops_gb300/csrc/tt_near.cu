@@ -206,18 +206,18 @@ __global__ void __launch_bounds__(128) k_near_sep(const f32* __restrict__ xt, co
         __syncthreads();
 #pragma unroll 2
         for (u32 a = 0; a < 32; ++a) {
-            f32 s[2] = {0.0f, 0.0f};
+            f32 s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
             const float4* u4 = reinterpret_cast<const float4*>(su[a]);
 #pragma unroll
             for (int k = 0; k < DP / 4; ++k) {
                 const float4 u = u4[k];
                 s[0] = fmaf(u.x, y[4 * k], s[0]);
                 s[1] = fmaf(u.y, y[4 * k + 1], s[1]);
-                s[0] = fmaf(u.z, y[4 * k + 2], s[0]);
-                s[1] = fmaf(u.w, y[4 * k + 3], s[1]);
+                s[2] = fmaf(u.z, y[4 * k + 2], s[2]);
+                s[3] = fmaf(u.w, y[4 * k + 3], s[3]);
             }
             // (a NaN projection counts as -inf: no separation)
-            const f32 v = s[0] + s[1];
+            const f32 v = (s[0] + s[1]) + (s[2] + s[3]);
             const u32 m = __reduce_min_sync(0xffffffffu, ordered(!live ? INFINITY : v == v ? v : -INFINITY));
             if (lane == 0) part[a][w] = from_ordered(m);
         }
@@ -327,7 +327,7 @@ void near_separations(tt_ctx* c, View& v, u32 dim, int kind, f32 p) {
     launch_pdl(k_near_centres, v.nblk, 64, 0, c->stream, v.abox, v.ntiles, dp, cen);
     TT_LAUNCH("k_near_centres");
     // enough blocks for the chip when there are few Bs
-    const dim3 grid(v.nblk, std::min<u32>(div_up(v.nblk, 32), std::max<u32>(1, 1216 / v.nblk)));
+    const dim3 grid(v.nblk, std::min<u32>(div_up(v.nblk, 32), std::max<u32>(1, 2432 / v.nblk)));
     auto go = [&](auto d) {
         launch_pdl(k_near_sep<decltype(d)::value>, grid, 128, 0, c->stream, v.xt, v.id, static_cast<const f32*>(cen),
                    v.ntiles, v.nblk, kind, p, s);
@@ -344,9 +344,9 @@ void near_separations(tt_ctx* c, View& v, u32 dim, int kind, f32 p) {
     v.sep = sep;
 }
 
-// Slots: S_NEAR_X, S_NEAR_ID, S_NEAR_BOX (results); S_TC_KEYS, S_TC_VALS,
-// S_NEAR_ST and the radix sort's own while it runs.
-View near_order(tt_ctx* c, const f32* x, u32 n, u32 dim) {
+// The View of the points in the order perm. Slots: S_NEAR_X, S_NEAR_ID,
+// S_NEAR_BOX (results).
+View near_regroup(tt_ctx* c, const f32* x, u32 n, u32 dim, const u32* perm) {
     View v;
     const u32 dp = padded_dim(dim);
     v.n = n;
@@ -354,24 +354,6 @@ View near_order(tt_ctx* c, const f32* x, u32 n, u32 dim) {
     v.nsup = div_up(v.ntiles, 32);
     v.tpad = v.nsup * 32;
     v.spad = div_up(v.nsup, 32) * 32;
-    const u32* perm;
-    if (dim <= kCodeDims) {
-        u64* key = c->arena.get<u64>(S_TC_KEYS, n);
-        u32* val = c->arena.get<u32>(S_TC_VALS, n);
-        f32* st = c->arena.get<f32>(S_NEAR_ST, 2 * kCodeDims);
-        const u32 bits = std::max<u32>(1, (n <= 8192 ? 11 : 22) / dim);
-        launch_pdl(k_near_stats, dim, kStatThreads, 0, c->stream, x, n, dim, st);
-        TT_LAUNCH("k_near_stats");
-        launch_pdl(k_near_codes, std::min<u32>(div_up(n, 256), 8 * u32(c->sms)), 256, 0, c->stream, x, n, dim, bits, st,
-                   key, val);
-        TT_LAUNCH("k_near_codes");
-        c->launches += 2;
-        u64* kb = c->arena.get<u64>(S_SORT_A, n);
-        u32* vb = c->arena.get<u32>(S_SORT_VA, n);
-        perm = radix_sort<u32>(c, key, val, n, kb, vb, int(bits * dim)) ? vb : val;
-    } else {
-        perm = pivot_order(c, x, n, dim);
-    }
     f32* xt = c->arena.get<f32>(S_NEAR_X, u64(v.ntiles) * dp * kTile);
     u32* id = c->arena.get<u32>(S_NEAR_ID, u64(v.ntiles) * kTile);
     const bool directions = dp >= kProjectDim;
@@ -391,6 +373,25 @@ View near_order(tt_ctx* c, const f32* x, u32 n, u32 dim) {
     v.sbox = sbox;
     v.abox = abox;
     return v;
+}
+
+// Slots: near_regroup's; S_TC_KEYS, S_TC_VALS, S_NEAR_ST and the radix sort's
+// own while it runs.
+View near_order(tt_ctx* c, const f32* x, u32 n, u32 dim) {
+    if (dim > kCodeDims) return near_regroup(c, x, n, dim, pivot_order(c, x, n, dim));
+    u64* key = c->arena.get<u64>(S_TC_KEYS, n);
+    u32* val = c->arena.get<u32>(S_TC_VALS, n);
+    f32* st = c->arena.get<f32>(S_NEAR_ST, 2 * kCodeDims);
+    const u32 bits = std::max<u32>(1, (n <= 8192 ? 11 : 22) / dim);
+    launch_pdl(k_near_stats, dim, kStatThreads, 0, c->stream, x, n, dim, st);
+    TT_LAUNCH("k_near_stats");
+    launch_pdl(k_near_codes, std::min<u32>(div_up(n, 256), 8 * u32(c->sms)), 256, 0, c->stream, x, n, dim, bits, st,
+               key, val);
+    TT_LAUNCH("k_near_codes");
+    c->launches += 2;
+    u64* kb = c->arena.get<u64>(S_SORT_A, n);
+    u32* vb = c->arena.get<u32>(S_SORT_VA, n);
+    return near_regroup(c, x, n, dim, radix_sort<u32>(c, key, val, n, kb, vb, int(bits * dim)) ? vb : val);
 }
 
 }  // namespace near

@@ -75,6 +75,7 @@ constexpr u32 kSepMinPoints = 2048;
 // Fills v.sep for the metric where it pays (kProjectDim, L1, L2, Lp).
 void near_separations(tt_ctx* c, View& v, u32 dim, int kind, f32 p);
 View near_order(tt_ctx* c, const f32* x, u32 n, u32 dim);
+View near_regroup(tt_ctx* c, const f32* x, u32 n, u32 dim, const u32* perm);   // in a given order
 
 // tt_near_<kind>.cu
 template <int KIND>
@@ -370,6 +371,7 @@ struct SkipNone {
     __device__ __forceinline__ bool tile(u32) const { return false; }
     __device__ __forceinline__ bool super(u32) const { return false; }
     __device__ __forceinline__ void refresh() const {}   // bounds that other warps lower
+    static constexpr bool kAlong = false;   // the direction test pays only between blocks that are apart
 };
 
 // Walks the tiles in reach of the warp's queries; visit(tile, coordinates,
@@ -458,8 +460,7 @@ __device__ __forceinline__ void walk(const View& v, WarpQ<DP, QW>& W, DirectionO
                     if (lane == src) b = 0xffffffffu;
                     for (u32 tile = (base + src) * kBlockTiles;
                          tile < min(v.ntiles, (base + src + 1) * kBlockTiles); ++tile)
-                        if (tile != home && !skip.tile(tile))   // (blocks that overlap: no direction helps)
-                            load_visit(tile, (1u << QW) - 1u, m != 0u);
+                        if (tile != home && !skip.tile(tile)) load_visit(tile, (1u << QW) - 1u, Skip::kAlong || m != 0u);
                 }
             }
             return;
@@ -750,6 +751,7 @@ struct SkipComp {
     u32 comp;   // the queries' shared component, or kNoComp
     WQ* W;
     const u32* cq;   // the queries' components
+    static constexpr bool kAlong = true;   // a block may hold points of two clusters
     u32 queries;
     const u32* bd;
     // takes up the components' bounds as other warps have left them
