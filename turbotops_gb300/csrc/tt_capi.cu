@@ -323,19 +323,8 @@ int tt_dense_distances(tt_ctx* c, const float* x, uint32_t n, uint32_t dim, int 
     return guard(c, [&] {
         check_metric(kind, p);
         if (n && (!x || !mat)) invalid("gb300: null buffer");
-        u32* rowmax = enclosing ? c->arena.get<u32>(S_ROWMAX, u64(n) + 1) : nullptr;
-        dense_matrix(c, x, n, dim, kind, p, mat, rowmax);
-        if (enclosing) {
-            if (n == 0) {
-                *enclosing = INFINITY;
-                return;
-            }
-            min_bits(c, rowmax, n, rowmax + n);
-            u32 b = 0;
-            TT_CUDA(cudaMemcpyAsync(&b, rowmax + n, 4, cudaMemcpyDeviceToHost, c->stream));
-            TT_CUDA(cudaStreamSynchronize(c->stream));
-            *enclosing = bitsf(b);
-        }
+        if (!enclosing) dense_matrix(c, x, n, dim, kind, p, mat, nullptr);
+        else *enclosing = n ? dense_radius(c, x, n, dim, kind, p, mat) : INFINITY;
     });
 }
 
@@ -599,20 +588,9 @@ int tt_dense_front_h(tt_ctx* c, const float* x_h, uint32_t n, uint32_t dim, int 
         if (n) TT_CUDA(cudaMemcpyAsync(x, x_h, sizeof(f32) * n * dim, cudaMemcpyHostToDevice, c->stream));
         check_finite_dev(c, x, u64(n) * dim);
         f32* mat = c->arena.get<f32>(S_MAT, u64(n) * n + 1);
-        u32* rowmax = c->arena.get<u32>(S_ROWMAX, u64(n) + 1);
-        dense_matrix(c, x, n, dim, kind, p, mat, std::isinf(t) ? rowmax : nullptr);
         float thr = t;
-        if (std::isinf(t)) {
-            if (n == 0) {
-                thr = INFINITY;
-            } else {
-                min_bits(c, rowmax, n, rowmax + n);
-                u32 b = 0;
-                TT_CUDA(cudaMemcpyAsync(&b, rowmax + n, 4, cudaMemcpyDeviceToHost, c->stream));
-                TT_CUDA(cudaStreamSynchronize(c->stream));
-                thr = bitsf(b);
-            }
-        }
+        if (!std::isinf(t)) dense_matrix(c, x, n, dim, kind, p, mat, nullptr);
+        else if (n) thr = dense_radius(c, x, n, dim, kind, p, mat);
         *thr_inout = thr;
         Complex cx{mat, nullptr, nullptr, nullptr, n, thr};
         Dim0Out r;
@@ -655,16 +633,9 @@ int tt_dense_redzed_pred_h(tt_ctx* c, const float* x_h, uint32_t n, uint32_t dim
         if (n) TT_CUDA(cudaMemcpyAsync(x, x_h, sizeof(f32) * n * dim, cudaMemcpyHostToDevice, c->stream));
         check_finite_dev(c, x, u64(n) * dim);
         f32* mat = c->arena.get<f32>(S_MAT, u64(n) * n + 1);
-        u32* rowmax = c->arena.get<u32>(S_ROWMAX, u64(n) + 1);
-        dense_matrix(c, x, n, dim, kind, p, mat, std::isinf(t) ? rowmax : nullptr);
         float thr = t;
-        if (std::isinf(t) && n) {
-            min_bits(c, rowmax, n, rowmax + n);
-            u32 b = 0;
-            TT_CUDA(cudaMemcpyAsync(&b, rowmax + n, 4, cudaMemcpyDeviceToHost, c->stream));
-            TT_CUDA(cudaStreamSynchronize(c->stream));
-            thr = bitsf(b);
-        }
+        if (!std::isinf(t)) dense_matrix(c, x, n, dim, kind, p, mat, nullptr);
+        else if (n) thr = dense_radius(c, x, n, dim, kind, p, mat);
         *thr_inout = thr;
         f32* d = nullptr;
         int32_t* v = nullptr;

@@ -60,6 +60,39 @@ void launch_dense(u32 n, cudaStream_t s, const f32* x, u32 dim, f32 p, f32* mat,
     }
 }
 
+// A small cloud's matrix and enclosing radius in one block: points in shared
+// memory, a thread a pair, row maxima by shared atomics; the radius into
+// page-locked memory. (Otherwise: two memsets, two kernels and a copy.)
+constexpr u32 kOneN = 128;
+constexpr u32 kOneFloats = 12000;   // points x dim that 48 KB hold beside the maxima
+template <int KIND>
+__global__ void __launch_bounds__(1024) k_dense_one(const f32* __restrict__ x, u32 n, u32 dim, f32 p,
+                                                   f32* __restrict__ mat, f32* __restrict__ radius) {
+    extern __shared__ f32 pt[];   // n x dim
+    __shared__ u32 rmax[kOneN];
+    for (u32 e = threadIdx.x; e < n * dim; e += blockDim.x) pt[e] = x[e];
+    if (threadIdx.x < kOneN) rmax[threadIdx.x] = 0;
+    __syncthreads();
+    const u32 pairs = n * (n - 1) / 2;
+    for (u32 e = threadIdx.x; e < pairs; e += blockDim.x) {
+        u32 a, b;
+        decode_edge(e, a, b);
+        const f32 d = metric_dist(KIND, p, Row{pt + b * dim}, Row{pt + a * dim}, dim);
+        mat[a * n + b] = d;
+        mat[b * n + a] = d;
+        atomicMax(&rmax[a], __float_as_uint(d));
+        atomicMax(&rmax[b], __float_as_uint(d));
+    }
+    if (threadIdx.x < n) mat[threadIdx.x * n + threadIdx.x] = 0.0f;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        u32 m = 0xffffffffu;
+        for (u32 i = threadIdx.x; i < n; i += 32) m = min(m, rmax[i]);
+        m = __reduce_min_sync(0xffffffffu, m);
+        if (threadIdx.x == 0) *radius = __uint_as_float(m);
+    }
+}
+
 __global__ void k_min_bits(const u32* __restrict__ v, u32 n, u32* __restrict__ out) {
     u32 m = 0xffffffffu;
     for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) m = min(m, v[i]);
@@ -82,6 +115,32 @@ void dense_matrix(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, f32*
     }
     TT_LAUNCH("k_dense");
     ++c->launches;
+}
+
+// The matrix and, on the host once the stream has caught up, the enclosing
+// radius (n >= 1; slot S_ROWMAX).
+f32 dense_radius(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, f32* mat) {
+    u32* h = static_cast<u32*>(c->pinned.get(4 * sizeof(u64)));
+    if (n <= kOneN && n * dim <= kOneFloats) {
+        auto go = [&](auto kernel) {
+            kernel<<<1, 1024, sizeof(f32) * n * dim, c->stream>>>(x, n, dim, p, mat, reinterpret_cast<f32*>(h));
+        };
+        switch (kind) {
+            case M_L1: go(k_dense_one<M_L1>); break;
+            case M_L2: go(k_dense_one<M_L2>); break;
+            case M_LINF: go(k_dense_one<M_LINF>); break;
+            default: go(k_dense_one<M_LP>); break;
+        }
+        TT_LAUNCH("k_dense_one");
+        ++c->launches;
+    } else {
+        u32* rowmax = c->arena.get<u32>(S_ROWMAX, u64(n) + 1);
+        dense_matrix(c, x, n, dim, kind, p, mat, rowmax);
+        min_bits(c, rowmax, n, rowmax + n);
+        TT_CUDA(cudaMemcpyAsync(h, rowmax + n, 4, cudaMemcpyDeviceToHost, c->stream));
+    }
+    TT_CUDA(cudaStreamSynchronize(c->stream));
+    return bitsf(*h);
 }
 
 void min_bits(tt_ctx* c, const u32* v, u32 n, u32* out) {

@@ -245,20 +245,16 @@ __device__ __forceinline__ bool warp_any_above(const DenseCx& cx, u32 f0, u32 f1
 // points in R^4 under L1: 0.85 and 0.33 ms). Bound by load latency (L1 / L2).
 // Beside that order there is no dependence on the sorted keys: the results
 // are gathered by index when the columns are emitted.
-__global__ void __launch_bounds__(256)
-    k_apparent_pairs(const f32* __restrict__ mat, u32 n, f32 thr, u32* __restrict__ res) {
-    pdl_wait();
-    pdl_trigger();
+__device__ __forceinline__ void apparent_pairs(const f32* __restrict__ mat, u32 n, f32 thr, u32 a, u32 b0,
+                                               u32* __restrict__ res) {
     const DenseCx cx{mat, n};
-    const u32 lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const u32 b0 = blockIdx.x * 32, b = b0 + lane;
-    for (u32 a = blockIdx.y * 8 + wid; a < n; a += gridDim.y * 8) {
-        if (b0 >= a) continue;   // warp-uniform
+    const u32 lane = threadIdx.x & 31, b = b0 + lane;
+    {
         const f32* ra = mat + u64(a) * n;
         const u32 bl = min(b, n - 1);   // lanes past the row read in bounds
         const f32 d = b < a ? ra[b] : INFINITY;
         const bool kept = b < a && d <= thr;
-        if (!__any_sync(0xffffffffu, kept)) continue;
+        if (!__any_sync(0xffffffffu, kept)) return;
         u32 w = NOV;
         f32 da = 0.0f, db = 0.0f;   // lengths (a, w), (b, w)
         u32 hi = n;                 // candidates at and above hi are tested
@@ -359,6 +355,15 @@ __global__ void __launch_bounds__(256)
             res[u64(a) * (a - 1) / 2 + b] =
                 (w == NOV ? kAppNone : w) | (apparent ? kAppApparent : 0u) | (em ? kAppEm : 0u);
     }
+}
+
+__global__ void __launch_bounds__(256)
+    k_apparent_pairs(const f32* __restrict__ mat, u32 n, f32 thr, u32* __restrict__ res) {
+    pdl_wait();
+    pdl_trigger();
+    const u32 b0 = blockIdx.x * 32;
+    for (u32 a = blockIdx.y * 8 + (threadIdx.x >> 5); a < n; a += gridDim.y * 8)
+        if (b0 < a) apparent_pairs(mat, n, thr, a, b0, res);   // (warp-uniform)
 }
 
 // (The wide key layout, more than kPackedMaxN vertices: a warp for each sorted
@@ -799,6 +804,187 @@ __global__ void k_forest_filter(const u64* __restrict__ keys, const u64* __restr
     }
 }
 
+// --------------------------------------------------------------------------
+// The whole stage of a tiny dense complex (n <= kTinyN) in one block: the kept
+// edges' keys in shared memory, ordered by a bitonic sort (the keys are
+// distinct and their order total), the apparent scan, the spanning forest, and
+// the outputs with the counts of what is kept into page-locked memory. A cloud
+// of 64 points is then one launch and one wait (with the stages as kernels of
+// their own, about twenty launches of 2 to 4 us: 155 us a pass with its
+// matrix and the copies of its results; now 110).
+// --------------------------------------------------------------------------
+constexpr u32 kTinyN = 128;
+constexpr u32 kTinyPairs = kTinyN * (kTinyN - 1) / 2;   // 8,128
+constexpr u32 kTinyKeys = 8192;
+constexpr u32 kTinyThreads = 1024;
+struct TinySmem {
+    u64 key[kTinyKeys];
+    u32 res[kTinyPairs];
+    u8 tree[kTinyKeys];
+    u32 comp[kTinyN], parent[kTinyN], best[kTinyN];
+    u32 warp[kTinyThreads / 32];
+    u32 hooked;
+};
+
+__global__ void __launch_bounds__(kTinyThreads)
+    k_dim0_tiny(const f32* __restrict__ mat, u32 n, f32 thr, int want_cols, u64* __restrict__ keys,
+                u8* __restrict__ app, u8* __restrict__ tree, f32* __restrict__ h0, u64* __restrict__ h0_edge,
+                u64* __restrict__ cidx, f32* __restrict__ cd, u64* __restrict__ emi, u8* __restrict__ emf,
+                u64* __restrict__ status) {
+    extern __shared__ __align__(16) unsigned char tiny_raw[];
+    TinySmem& S = *reinterpret_cast<TinySmem*>(tiny_raw);
+    const u32 tid = threadIdx.x, lane = tid & 31, w = tid >> 5, lt = (1u << lane) - 1u;
+    const u32 pairs = n * (n - 1) / 2;
+    u32 P = 2;
+    while (P < pairs) P <<= 1;
+    const EdgeFmt fmt{};
+    // keys of the kept edges, the rest after every key
+    u32 m = 0;
+    for (u32 e0 = 0; e0 < P; e0 += kTinyThreads) {
+        const u32 e = e0 + tid;
+        bool keep = false;
+        if (e < P) {
+            u64 k = ~0ull;
+            if (e < pairs) {
+                u32 a, b;
+                decode_edge(e, a, b);
+                const f32 d = mat[a * n + b];
+                keep = d <= thr;
+                if (keep) k = key_rips(d, e);
+            }
+            S.key[e] = k;
+            S.tree[e] = 0;
+        }
+        m += __syncthreads_count(keep);
+    }
+    if (tid < n) {
+        S.comp[tid] = S.parent[tid] = tid;
+        S.best[tid] = NOV;
+    }
+    if (tid == 0) S.hooked = 0;
+    if (want_cols)   // (row, 32 columns) tasks, a warp each
+        for (u32 t = w, chunks = (n + 31) / 32; t < n * chunks; t += kTinyThreads / 32) {
+            const u32 a = t / chunks, b0 = t % chunks * 32;
+            if (b0 < a) apparent_pairs(mat, n, thr, a, b0, S.res);
+        }
+    __syncthreads();
+    for (u32 size = 2; size <= P; size <<= 1)
+        for (u32 stride = size >> 1; stride; stride >>= 1) {
+            for (u32 i = tid; i < P / 2; i += kTinyThreads) {
+                const u32 lo = 2 * i - (i & (stride - 1)), hi = lo + stride;
+                const u64 x = S.key[lo], y = S.key[hi];
+                if ((x > y) == ((lo & size) == 0)) {
+                    S.key[lo] = y;
+                    S.key[hi] = x;
+                }
+            }
+            __syncthreads();
+        }
+    // the spanning forest (k_forest_block's rounds)
+    for (;;) {
+        bool any = false;
+        for (u32 r = tid; r < m; r += kTinyThreads) {
+            u32 a, b;
+            decode_edge(fmt.rips(S.key[r]), a, b);
+            const u32 ca = S.comp[a], cb = S.comp[b];
+            if (ca == cb) continue;
+            any = true;
+            if (*reinterpret_cast<volatile u32*>(&S.best[ca]) > r) atomicMin(&S.best[ca], r);
+            if (*reinterpret_cast<volatile u32*>(&S.best[cb]) > r) atomicMin(&S.best[cb], r);
+        }
+        if (!__syncthreads_or(any)) break;
+        if (tid < n && S.comp[tid] == tid && S.best[tid] != NOV) {
+            const u32 r = S.best[tid];
+            u32 a, b;
+            decode_edge(fmt.rips(S.key[r]), a, b);
+            const u32 o = S.comp[a] == tid ? S.comp[b] : S.comp[a];
+            S.tree[r] = 1;
+            if (!(S.best[o] == r && tid < o)) {   // mutual: o hooks onto this one
+                S.parent[tid] = o;
+                atomicAdd(&S.hooked, 1u);
+            }
+        }
+        __syncthreads();
+        u32 root = 0;
+        if (tid < n) {
+            root = S.parent[S.comp[tid]];
+            for (u32 q = 0; S.parent[root] != root && q < n; ++q) root = S.parent[root];
+        }
+        __syncthreads();
+        if (tid < n) {
+            S.comp[tid] = S.parent[tid] = root;
+            S.best[tid] = NOV;
+        }
+        __syncthreads();
+        if (S.hooked == n - 1) break;   // (read after a barrier, next written after one)
+    }
+    __syncthreads();
+    // columns in all (they are written in descending order), then the outputs
+    u32 ncols = 0;
+    if (want_cols)
+        for (u32 e0 = 0; e0 < m; e0 += kTinyThreads) {
+            const u32 e = e0 + tid;
+            const bool col = e < m && !S.tree[e] && !(S.res[u32(fmt.rips(S.key[e]))] & kAppApparent);
+            ncols += __syncthreads_count(col);
+        }
+    u32 oh = 0, oc = 0;   // bars and columns before this chunk
+    for (u32 e0 = 0; e0 < m; e0 += kTinyThreads) {
+        const u32 e = e0 + tid;
+        const bool in = e < m;
+        const u64 key = in ? S.key[e] : 0ull;
+        const u32 idx = u32(fmt.rips(key));
+        const f32 d = fmt.d(key);
+        const bool t = in && S.tree[e];
+        const u32 r = in && want_cols ? S.res[idx] : 0u;
+        const bool ap = (r & kAppApparent) != 0;
+        const bool bar = t && d > 0.0f, col = in && want_cols && !t && !ap;
+        const u32 hb = __ballot_sync(0xffffffffu, bar), cb = __ballot_sync(0xffffffffu, col);
+        __syncthreads();   // the last chunk's counts are read
+        if (lane == 0) S.warp[w] = (u32(__popc(hb)) << 16) | __popc(cb);
+        __syncthreads();
+        u32 before = 0, all = 0;   // bars << 16 | columns (at most 1,024 each)
+#pragma unroll
+        for (u32 q = 0; q < kTinyThreads / 32; ++q) {
+            const u32 x = S.warp[q];
+            before += q < w ? x : 0u;
+            all += x;
+        }
+        if (in) {
+            keys[e] = key;
+            tree[e] = t;
+            if (want_cols) app[e] = ap;
+        }
+        if (bar) {
+            const u32 o = oh + (before >> 16) + __popc(hb & lt);
+            h0[o] = d;
+            h0_edge[o] = idx;
+        }
+        if (col) {
+            const u32 o = ncols - 1 - (oc + (before & 0xffffu) + __popc(cb & lt));
+            cidx[o] = idx;
+            cd[o] = d;
+            const u32 cw = r & kAppNone;
+            if (cw == kAppNone) {
+                emi[o] = kNone;
+                emf[o] = 0;
+            } else {
+                u32 c0, c1, c2 = cw;
+                decode_edge(idx, c0, c1);
+                sort3(c0, c1, c2);
+                emi[o] = tri_idx(c0, c1, c2);
+                emf[o] = (r & kAppEm) != 0;
+            }
+        }
+        oh += all >> 16;
+        oc += all & 0xffffu;
+    }
+    if (tid == 0) {
+        status[0] = (u64(oh) << 32) | oc;
+        status[1] = S.hooked;
+        status[2] = m;
+    }
+}
+
 inline u32 grid_for(u64 work, u32 per_block) {
     const u64 g = (work + per_block - 1) / per_block;
     return u32(std::max<u64>(1, std::min<u64>(g, 64ull * kSMs)));
@@ -924,6 +1110,23 @@ static void dim0_small(tt_ctx* c, const Complex& cx, u32 maxdim, Dim0Out& out) {
     out.emi = c->arena.get<u64>(S_OUT3, (want_cols ? cap : 0) + 1);
     out.emf = c->arena.get<u8>(S_OUT4, (want_cols ? cap : 0) + 1);
     out.h0_edge = c->arena.get<u64>(S_OUT5, n + 1);
+    u64* h = static_cast<u64*>(c->pinned.get(4 * sizeof(u64)));
+    auto finish = [&] {
+        TT_CUDA(cudaStreamSynchronize(s));
+        out.m = h[2];
+        out.nh0 = h[0] >> 32;
+        out.ncols = h[0] & 0xffffffffull;
+        out.essential = n - u32(h[1]);
+    };
+    if (n <= kTinyN) {
+        TT_CUDA(cudaFuncSetAttribute(k_dim0_tiny, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(TinySmem))));
+        k_dim0_tiny<<<1, kTinyThreads, sizeof(TinySmem), s>>>(cx.mat, n, cx.thr, want_cols, keys, app, tree, out.h0,
+                                                              out.h0_edge, out.cidx, out.cd, out.emi, out.emf, h);
+        TT_LAUNCH("k_dim0_tiny");
+        c->launches += 1;
+        finish();
+        return;
+    }
     const EdgeFmt fmt{};
     TT_CUDA(cudaMemsetAsync(tot, 0, 4 * sizeof(u64), s));
     TT_CUDA(cudaMemsetAsync(tree, 0, cap + 1, s));
@@ -968,14 +1171,9 @@ static void dim0_small(tt_ctx* c, const Complex& cx, u32 maxdim, Dim0Out& out) {
                want_cols, cnt, tot, out.h0, out.h0_edge, out.cidx, out.cd, out.emi, out.emf);
     TT_LAUNCH("k_emit_dim0");
     c->launches += 2;
-    u64* h = static_cast<u64*>(c->pinned.get(4 * sizeof(u64)));
     TT_CUDA(cudaMemcpyAsync(h, tot, 2 * sizeof(u64), cudaMemcpyDeviceToHost, s));
     TT_CUDA(cudaMemcpyAsync(h + 2, mdev, sizeof(u64), cudaMemcpyDeviceToHost, s));
-    TT_CUDA(cudaStreamSynchronize(s));
-    out.m = h[2];
-    out.nh0 = h[0] >> 32;
-    out.ncols = h[0] & 0xffffffffull;
-    out.essential = n - u32(h[1]);
+    finish();
 }
 
 void dim0(tt_ctx* c, const Complex& cx, u32 maxdim, Dim0Out& out, u64 m_known) {

@@ -87,6 +87,7 @@ struct EdgeFmt {
 // ---- tt_dense.cu
 void dense_matrix(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, f32* mat, u32* rowmax);
 void min_bits(tt_ctx* c, const u32* v, u32 n, u32* out);
+f32 dense_radius(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, f32* mat);
 
 // ---- tt_sort.cu
 template <typename T>

@@ -219,16 +219,7 @@ void persistence_points(tt_ctx* c, const f32* x_h, u32 n, u32 dim, int kind, f32
         check_dense_budget(c, n);
         out.method = "dense";
         f32* mat = c->arena.get<f32>(S_MAT, u64(n) * n + 1);
-        u32* rowmax = c->arena.get<u32>(S_ROWMAX, u64(n) + 1);
-        dense_matrix(c, x, n, dim, kind, p, mat, rowmax);
-        f32 t = INFINITY;
-        if (n) {
-            min_bits(c, rowmax, n, rowmax + n);
-            u32 b = 0;
-            TT_CUDA(cudaMemcpyAsync(&b, rowmax + n, 4, cudaMemcpyDeviceToHost, c->stream));
-            sync(c);
-            t = bitsf(b);
-        }
+        const f32 t = n ? dense_radius(c, x, n, dim, kind, p, mat) : INFINITY;
         out.threshold = t;
         if (n == 0) return;
         Complex cx{mat, nullptr, nullptr, nullptr, n, t};

@@ -203,13 +203,7 @@ extern "C" int tt_topo_forward(tt_ctx* c, const float* x, const uint32_t* sizes,
                 }
                 const u32 n = C.n;
                 f32* mat = c->arena.get<f32>(S_MAT, u64(n) * n + 1);
-                u32* rowmax = c->arena.get<u32>(S_ROWMAX, u64(n) + 1);
-                dense_matrix(c, x + C.off * dim, n, dim, kind, p, mat, rowmax);
-                min_bits(c, rowmax, n, rowmax + n);
-                u32 b = 0;
-                TT_CUDA(cudaMemcpyAsync(&b, rowmax + n, 4, cudaMemcpyDeviceToHost, c->stream));
-                TT_CUDA(cudaStreamSynchronize(c->stream));
-                C.thr = bitsf(b);
+                C.thr = dense_radius(c, x + C.off * dim, n, dim, kind, p, mat);
                 Complex cx{mat, nullptr, nullptr, nullptr, n, C.thr};
                 Dim0Out r;
                 dim0(c, cx, 1, r);
