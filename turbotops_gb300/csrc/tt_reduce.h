@@ -47,6 +47,18 @@ Bars compute_pairs(const HostComplex& cx, uint32_t dim, uint32_t maxdim, const s
                    const uint64_t* em_idx, const uint8_t* em_app, std::vector<uint64_t>& pivots,
                    ReduceStats& st, unsigned threads = 0);
 
+// The same pairs, bars and pivots as compute_pairs(hc, 1, ...) on a dense
+// complex, from its edges in filtration order: `keys` are the m kept edges as
+// dim0 sorts them (float bits of d << 33 | (2^33 - 1 - index), ascending),
+// `cols` the dimension-1 columns. Returns false, with nothing written, where
+// it does not apply (more than kCocycleMaxN points; many equal lengths) or
+// where its work would pass `budget` (64-bit words touched): the caller then
+// runs compute_pairs. st.emergent counts the pairs of length zero.
+constexpr uint32_t kCocycleMaxN = 8192;
+bool dense_pairs_dim1(const HostComplex& hc, const std::vector<Entry>& cols, const uint64_t* keys, uint64_t m,
+                      Bars& bars, std::vector<uint64_t>& pivots, ReduceStats& st,
+                      uint64_t budget = uint64_t(4) << 30);
+
 // Reducer::assemble(dim) (rips.hpp:981-1023): the dimension-(dim + 1)
 // columns — every cofacet of the dimension-dim `simplices` (any order) through
 // a vertex above the simplex's largest, so each once; neither a pivot of

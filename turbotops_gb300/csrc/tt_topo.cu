@@ -3,10 +3,11 @@
 //
 // No counterpart in the reference (its Barcode keeps values only,
 // rips.hpp:52-67). Forward: for every cloud the GPU runs the dense front end
-// (distances, enclosing radius, dim0); host threads run compute_pairs(1) for
-// the clouds whose front end is done while the GPU works on the next ones,
-// recording each bar's critical
-// simplices; each bar value is then the length of one edge:
+// (distances, enclosing radius, dim0); host threads reduce dimension 1 of the
+// clouds whose front end is done while the GPU works on the next ones (by
+// cocycles, dense_pairs_dim1; compute_pairs where that does not apply),
+// recording each bar's critical simplices; each bar value is then the length
+// of one edge:
 //   H0 death   the spanning-tree edge that merged two components
 //   H1 birth   the column's edge
 //   H1 death   the longest edge of the pivot triangle (the edge whose length
@@ -97,7 +98,7 @@ struct Cloud {
     u64 off = 0;
     f32 thr = 0;
     std::vector<f32> mat, h0d, cd;
-    std::vector<u64> h0e, ci, emi;
+    std::vector<u64> h0e, ci, emi, keys;
     std::vector<u8> emf;
     host::Bars bars;
 };
@@ -176,7 +177,8 @@ extern "C" int tt_topo_forward(tt_ctx* c, const float* x, const uint32_t* sizes,
                     host::HostComplex hc{C.mat.data(), nullptr, nullptr, nullptr, C.n, C.thr};
                     std::vector<u64> piv;
                     host::ReduceStats st;
-                    C.bars = host::compute_pairs(hc, 1, 1, cols, C.emi.data(), C.emf.data(), piv, st, per_cloud);
+                    if (!host::dense_pairs_dim1(hc, cols, C.keys.data(), C.keys.size(), C.bars, piv, st))
+                        C.bars = host::compute_pairs(hc, 1, 1, cols, C.emi.data(), C.emf.data(), piv, st, per_cloud);
                 }
             } catch (const std::exception& e) {
                 errs[t] = e.what();
@@ -214,6 +216,9 @@ extern "C" int tt_topo_forward(tt_ctx* c, const float* x, const uint32_t* sizes,
                 C.cd.resize(r.ncols);
                 C.emi.resize(r.ncols);
                 C.emf.resize(r.ncols);
+                C.keys.resize(n <= host::kCocycleMaxN ? r.m : 0);
+                if (!C.keys.empty())
+                    TT_CUDA(cudaMemcpyAsync(C.keys.data(), r.keys, 8 * r.m, cudaMemcpyDeviceToHost, c->stream));
                 TT_CUDA(cudaMemcpyAsync(C.mat.data(), mat, 4 * u64(n) * n, cudaMemcpyDeviceToHost, c->stream));
                 if (r.nh0) {
                     TT_CUDA(cudaMemcpyAsync(C.h0d.data(), r.h0, 4 * r.nh0, cudaMemcpyDeviceToHost, c->stream));
