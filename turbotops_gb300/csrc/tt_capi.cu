@@ -226,6 +226,7 @@ void tt_ctx_destroy(tt_ctx* c) {
     if (c->stream) cudaStreamSynchronize(c->stream);
     c->arena.release();
     c->pinned.release();
+    c->staging.release();
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
     if (c->aux) {
         cudaStreamSynchronize(c->aux);

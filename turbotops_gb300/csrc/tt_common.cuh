@@ -150,7 +150,8 @@ struct tt_ctx {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     tt::Arena arena;
-    tt::Pinned pinned;
+    tt::Pinned pinned;                       // a call's counts and flags
+    tt::Pinned staging;                      // tt_topo_forward: the clouds' outputs (at most 256 MB)
     std::string last_error;
     int sms = tt::kSMs;
     double last_kernel_ms = 0.0;   // device time of the last stage (CUDA events)

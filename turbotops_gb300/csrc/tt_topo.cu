@@ -93,14 +93,57 @@ void decode3(u64 idx, u32 n, u32& c0, u32& c1, u32& c2) {   // c0 > c1 > c2
     decode2(idx - u64(lo) * (lo - 1) * (lo - 2) / 6, c1, c2);
 }
 
+// A cloud's outputs on the host: in the context's page-locked staging (the
+// copies are then asynchronous and touch no fresh pages), or, past its limit,
+// in memory of their own.
+template <typename T>
+struct Out {
+    T* p = nullptr;
+    u64 count = 0;
+    std::vector<T> own;
+    T* data() { return p; }
+    const T* data() const { return p; }
+    u64 size() const { return count; }
+    const T& operator[](u64 i) const { return p[i]; }
+};
+
 struct Cloud {
     u32 n = 0;
     u64 off = 0;
     f32 thr = 0;
-    std::vector<f32> mat, h0d, cd;
-    std::vector<u64> h0e, ci, emi, keys;
-    std::vector<u8> emf;
+    Out<f32> mat, h0d, cd;
+    Out<u64> h0e, ci, emi, keys;
+    Out<u8> emf;
     host::Bars bars;
+};
+
+constexpr u64 kStagingMax = u64(256) << 20;
+
+// Takes the clouds' outputs off the device, one after the other.
+struct Staging {
+    tt_ctx* c;
+    unsigned char* base = nullptr;
+    u64 left = 0;
+    Staging(tt_ctx* ctx, const uint32_t* sizes, u32 count) : c(ctx) {
+        u64 want = 0;   // matrix and keys, H0, a few columns a point
+        for (u32 q = 0; q < count; ++q) want += 8 * u64(sizes[q]) * sizes[q] + 256 * u64(sizes[q]) + 1024;
+        left = std::min(want, kStagingMax);
+        if (left) base = static_cast<unsigned char*>(c->staging.get(left));
+    }
+    template <typename T>
+    void take(Out<T>& o, const T* dev, u64 count) {
+        o.count = count;
+        const u64 bytes = (count * sizeof(T) + 15) & ~u64(15);
+        if (bytes <= left) {
+            o.p = reinterpret_cast<T*>(base);
+            base += bytes;
+            left -= bytes;
+        } else {
+            o.own.resize(count);
+            o.p = o.own.data();
+        }
+        if (count) TT_CUDA(cudaMemcpyAsync(o.p, dev, count * sizeof(T), cudaMemcpyDeviceToHost, c->stream));
+    }
 };
 
 // Hands clouds from the thread that runs their device front end to the
@@ -193,46 +236,33 @@ extern "C" int tt_topo_forward(tt_ctx* c, const float* x, const uint32_t* sizes,
         // device front end, cloud by cloud; each cloud goes to the reducers
         // once its outputs are on the host
         auto front_end = [&] {
+            Staging st(c, sizes, count);
             u64 off = 0;
             for (u32 q = 0; q < count; ++q) {
                 Cloud& C = cl[q];
                 C.n = sizes[q];
                 C.off = off;
                 off += C.n;
-                if (C.n == 0) {
-                    queue.publish(q);
-                    continue;
-                }
+                if (C.n == 0) continue;   // (published with the next cloud)
                 const u32 n = C.n;
                 f32* mat = c->arena.get<f32>(S_MAT, u64(n) * n + 1);
                 C.thr = dense_radius(c, x + C.off * dim, n, dim, kind, p, mat);
                 Complex cx{mat, nullptr, nullptr, nullptr, n, C.thr};
+                // (the radius has just been waited for, and with it the copies of the cloud before)
+                if (q) queue.publish(q - 1);
                 Dim0Out r;
                 dim0(c, cx, 1, r);
-                C.mat.resize(u64(n) * n);
-                C.h0d.resize(r.nh0);
-                C.h0e.resize(r.nh0);
-                C.ci.resize(r.ncols);
-                C.cd.resize(r.ncols);
-                C.emi.resize(r.ncols);
-                C.emf.resize(r.ncols);
-                C.keys.resize(n <= host::kCocycleMaxN ? r.m : 0);
-                if (!C.keys.empty())
-                    TT_CUDA(cudaMemcpyAsync(C.keys.data(), r.keys, 8 * r.m, cudaMemcpyDeviceToHost, c->stream));
-                TT_CUDA(cudaMemcpyAsync(C.mat.data(), mat, 4 * u64(n) * n, cudaMemcpyDeviceToHost, c->stream));
-                if (r.nh0) {
-                    TT_CUDA(cudaMemcpyAsync(C.h0d.data(), r.h0, 4 * r.nh0, cudaMemcpyDeviceToHost, c->stream));
-                    TT_CUDA(cudaMemcpyAsync(C.h0e.data(), r.h0_edge, 8 * r.nh0, cudaMemcpyDeviceToHost, c->stream));
-                }
-                if (r.ncols) {
-                    TT_CUDA(cudaMemcpyAsync(C.ci.data(), r.cidx, 8 * r.ncols, cudaMemcpyDeviceToHost, c->stream));
-                    TT_CUDA(cudaMemcpyAsync(C.cd.data(), r.cd, 4 * r.ncols, cudaMemcpyDeviceToHost, c->stream));
-                    TT_CUDA(cudaMemcpyAsync(C.emi.data(), r.emi, 8 * r.ncols, cudaMemcpyDeviceToHost, c->stream));
-                    TT_CUDA(cudaMemcpyAsync(C.emf.data(), r.emf, r.ncols, cudaMemcpyDeviceToHost, c->stream));
-                }
-                TT_CUDA(cudaStreamSynchronize(c->stream));
-                queue.publish(q);
+                st.take(C.mat, mat, u64(n) * n);
+                st.take(C.keys, r.keys, n <= host::kCocycleMaxN ? r.m : 0);
+                st.take(C.h0d, r.h0, r.nh0);
+                st.take(C.h0e, r.h0_edge, r.nh0);
+                st.take(C.ci, r.cidx, r.ncols);
+                st.take(C.cd, r.cd, r.ncols);
+                st.take(C.emi, r.emi, r.ncols);
+                st.take(C.emf, r.emf, r.ncols);
             }
+            TT_CUDA(cudaStreamSynchronize(c->stream));
+            if (count) queue.publish(count - 1);
         };
         try {
             for (u32 t = 1; t < nt; ++t) pool.emplace_back(work, t);
