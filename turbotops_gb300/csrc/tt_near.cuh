@@ -34,6 +34,9 @@
 // there boxes and candidates are tested on a fast power sum with a margin for
 // every error (below, k_near_knn_lp), and only the survivors are evaluated.
 #pragma once
+#include <cmath>
+#include <type_traits>
+
 #include "tt_internal.cuh"
 #include "tt_metric.cuh"
 
@@ -67,6 +70,7 @@ inline u32 padded_dim(u32 dim) {
 
 // Queries a warp takes at once (tt_near.cuh's header).
 constexpr u32 queries_per_warp(u32 dp) { return dp <= 4 ? 1 : dp <= 8 ? 2 : dp <= 16 ? 4 : 8; }
+constexpr u32 kFewPoints = 10000;   // lists of fewer points: half as many queries a warp (launch_knn)
 
 // tt_near.cu
 constexpr u32 kBlockTiles = 4;          // tiles a separation block
@@ -77,7 +81,8 @@ void near_separations(tt_ctx* c, View& v, u32 dim, int kind, f32 p);
 View near_order(tt_ctx* c, const f32* x, u32 n, u32 dim);
 View near_regroup(tt_ctx* c, const f32* x, u32 n, u32 dim, const u32* perm);   // in a given order
 
-// tt_near_<kind>.cu
+// tt_near_*.cu (kernels by metric, several translation units so that they
+// compile in parallel)
 template <int KIND>
 void near_knn(tt_ctx* c, const View& v, u32 dim, u32 k, u32* ids, f32* dists);
 template <int KIND>
@@ -268,21 +273,21 @@ __device__ __forceinline__ u32 box_needs(const f32* __restrict__ box, u32 pad, u
 // (100,000 mixture points in R^32: the foreign searches of a spanning tree take
 // 45 ms with the boxes alone, 30 with the directions, 9.7 with the table and
 // the bounds refreshed; L1.5 lists 13.5 ms, 6.7 with the table.)
-template <int DP>
+template <int DP, int QW>
 struct Direction {
     alignas(16) f32 g[DP];     // the queries' centre
     alignas(16) f32 u[DP];
-    f32 qy[DP][8];             // the queries relative to it, coordinate-major
+    f32 qy[DP][QW];            // the queries relative to it, coordinate-major
     f32 ext[DP];               // their largest |q_k - g_k|
 };
 struct NoDirection {};
 template <int KIND, int DP>
 constexpr bool projects() { return DP >= int(kProjectDim) && KIND != M_LINF; }
-template <int KIND, int DP>
-using DirectionOf = typename std::conditional<projects<KIND, DP>(), Direction<DP>, NoDirection>::type;
+template <int KIND, int DP, int QW>
+using DirectionOf = typename std::conditional<projects<KIND, DP>(), Direction<DP, QW>, NoDirection>::type;
 
 template <int DP, int QW>
-__device__ __forceinline__ void init_direction(const WarpQ<DP, QW>& W, Direction<DP>& D) {
+__device__ __forceinline__ void init_direction(const WarpQ<DP, QW>& W, Direction<DP, QW>& D) {
     const u32 lane = threadIdx.x & 31;
     for (u32 k = lane; k < DP; k += 32) {
         f32 lo = W.qt[k][0], hi = lo;
@@ -311,7 +316,7 @@ __device__ __forceinline__ f32 warp_sum(f32 x) {
 // The queries of `need` that the tile (candidates c, one a lane; `live`: a
 // point) may still matter to.
 template <int KIND, int DP, int QW>
-__device__ __forceinline__ u32 project(const View& v, const WarpQ<DP, QW>& W, Direction<DP>& D, u32 tile,
+__device__ __forceinline__ u32 project(const View& v, const WarpQ<DP, QW>& W, Direction<DP, QW>& D, u32 tile,
                                        const f32 (&c)[DP], bool live, u32 need) {
     const u32 lane = threadIdx.x & 31;
     f32 nrm = 0.0f, mag = 0.0f;
@@ -348,7 +353,7 @@ __device__ __forceinline__ u32 project(const View& v, const WarpQ<DP, QW>& W, Di
     nrm *= 1.0f + 0x1p-9f;
     __syncwarp();
     f32 pc[2] = {0.0f, 0.0f}, pq[2] = {0.0f, 0.0f};
-    const u32 ql = lane & 7u;
+    const u32 ql = lane % QW;
 #pragma unroll
     for (int k = 0; k < DP; ++k) {
         const f32 u = D.u[k];
@@ -378,7 +383,7 @@ struct SkipNone {
 // candidate id, queries) tests one tile against the queries of a bit mask and
 // returns whether a bound may have dropped.
 template <int KIND, int DP, int CH, int QW, typename Visit, typename Skip = SkipNone>
-__device__ __forceinline__ void walk(const View& v, WarpQ<DP, QW>& W, DirectionOf<KIND, DP>& D, u32 home, Visit&& visit,
+__device__ __forceinline__ void walk(const View& v, WarpQ<DP, QW>& W, DirectionOf<KIND, DP, QW>& D, u32 home, Visit&& visit,
                                      Skip skip = Skip{}) {
     const u32 lane = threadIdx.x & 31;
     if constexpr (projects<KIND, DP>()) init_direction<DP, QW>(W, D);
@@ -561,7 +566,7 @@ __global__ void __launch_bounds__(32 * kWarps)
     pdl_wait();
     pdl_trigger();
     __shared__ WarpQ<DP, QW> sw[kWarps];
-    __shared__ DirectionOf<KIND, DP> sd[projects<KIND, DP>() ? kWarps : 1];
+    __shared__ DirectionOf<KIND, DP, QW> sd[projects<KIND, DP>() ? kWarps : 1];
     __shared__ u64 slist[kWarps][QW][32];
     const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const u32 p0 = (blockIdx.x * kWarps + w) * QW;
@@ -648,7 +653,7 @@ __global__ void __launch_bounds__(32 * kWarps)
     pdl_wait();
     pdl_trigger();
     __shared__ WarpQ<DP, QW> sw[kWarps];
-    __shared__ DirectionOf<KIND, DP> sd[projects<KIND, DP>() ? kWarps : 1];
+    __shared__ DirectionOf<KIND, DP, QW> sd[projects<KIND, DP>() ? kWarps : 1];
     __shared__ u64 slist[kWarps][QW][32];
     __shared__ u32 spos[kWarps][64];   // survivors: position in the order, query (a ring)
     __shared__ u8 sq[kWarps][64];
@@ -778,7 +783,7 @@ __global__ void __launch_bounds__(32 * kWarps)
     pdl_wait();
     pdl_trigger();
     __shared__ WarpQ<DP, QW> sw[kWarps];
-    __shared__ DirectionOf<KIND, DP> sd[projects<KIND, DP>() ? kWarps : 1];
+    __shared__ DirectionOf<KIND, DP, QW> sd[projects<KIND, DP>() ? kWarps : 1];
     __shared__ u64 sbest[kWarps][QW];
     __shared__ u32 scq[kWarps][QW];
     const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -863,7 +868,7 @@ __global__ void __launch_bounds__(32 * kWarps)
     pdl_wait();
     pdl_trigger();
     __shared__ WarpQ<DP, 1> sw[kWarps];
-    __shared__ DirectionOf<KIND, DP> sd[projects<KIND, DP>() ? kWarps : 1];
+    __shared__ DirectionOf<KIND, DP, 1> sd[projects<KIND, DP>() ? kWarps : 1];
     __shared__ u64 srow[FILL ? kWarps : 1][FILL ? kRadiusRow : 1];
     const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const u32 p0 = blockIdx.x * kWarps + w;
@@ -940,7 +945,15 @@ __global__ void __launch_bounds__(32 * kWarps)
 template <int KIND, int DP, int CH>
 void launch_knn(tt_ctx* c, const View& v, u32 k, u32* ids, f32* dists) {
     constexpr int QW = queries_per_warp(DP);
-    launch_pdl(k_near_knn<KIND, DP, CH, QW>, div_up(div_up(v.n, QW), kWarps), 32 * kWarps, 0, c->stream, v, k, ids, dists);
+    auto go = [&](auto qw) {
+        constexpr int Q = decltype(qw)::value;
+        launch_pdl(k_near_knn<KIND, DP, CH, Q>, div_up(div_up(v.n, Q), kWarps), 32 * kWarps, 0, c->stream, v, k, ids, dists);
+    };
+    // few points: more warps count for more than the reuse of a tile's loads
+    // (3,000 x 24 uniform points 0.35 ms with 8 queries a warp, 0.25 with 4;
+    // 16,000 x 16 mixture points 0.76 and 0.85)
+    if (DP >= 16 && v.n <= kFewPoints) go(std::integral_constant<int, QW >= 4 ? QW / 2 : QW>{});
+    else go(std::integral_constant<int, QW>{});
     TT_LAUNCH("k_near_knn");
     ++c->launches;
 }
@@ -1017,12 +1030,23 @@ void near_radius_fill(tt_ctx* c, const View& v, u32 dim, f32 tau, const u64* rp,
     radius_pass<KIND, true>(c, v, dim, tau, nullptr, nullptr, rp, ci, w);
 }
 
-#define TT_NEAR_INSTANTIATE(KIND)                                                     \
-    template void near_knn<KIND>(tt_ctx*, const View&, u32, u32, u32*, f32*);         \
-    template void near_foreign<KIND>(tt_ctx*, const View&, u32, const u32*, const u32*, const u32*, const u32*, \
-                                     const u32*, u32*, unsigned long long*);          \
-    template void near_radius_count<KIND>(tt_ctx*, const View&, u32, f32, u64*, u32*); \
-    template void near_radius_fill<KIND>(tt_ctx*, const View&, u32, f32, const u64*, u32*, f32*);
+// Lp lists of one power class (a translation unit each)
+template <int CLS>
+void knn_lp_class(tt_ctx* c, const View& v, u32 dim, u32 k, u32* ids, f32* dists) {
+    constexpr int KIND = M_LP + 16 * CLS;
+    with_dim<KIND>(dim, [&](auto dp, auto) {
+        constexpr int DP = decltype(dp)::value, QW = queries_per_warp(DP);
+        auto go = [&](auto qw) {
+            constexpr int Q = decltype(qw)::value;
+            launch_pdl(k_near_knn_lp<KIND, DP, Q>, div_up(div_up(v.n, Q), kWarps), 32 * kWarps, 0, c->stream, v, dim, k,
+                       ids, dists);
+        };
+        if (DP >= 16 && v.n <= kFewPoints) go(std::integral_constant<int, QW >= 4 ? QW / 2 : QW>{});   // (as launch_knn)
+        else go(std::integral_constant<int, QW>{});
+        TT_LAUNCH("k_near_knn_lp");
+        ++c->launches;
+    });
+}
 
 #endif  // TT_NEAR_IMPL
 

@@ -1,12 +1,9 @@
-// tt_near_l1.cu — the ordered searches (tt_near.cuh) for L1.
+// tt_near_l1.cu — the ordered kNN lists (tt_near.cuh) for L1.
 #define TT_NEAR_IMPL
-#include <cmath>
-#include <type_traits>
-
 #include "tt_near.cuh"
 
 namespace tt {
 namespace near {
-TT_NEAR_INSTANTIATE(M_L1)
+template void near_knn<M_L1>(tt_ctx*, const View&, u32, u32, u32*, f32*);
 }  // namespace near
 }  // namespace tt

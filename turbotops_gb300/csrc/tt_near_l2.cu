@@ -1,12 +1,9 @@
-// tt_near_l2.cu — the ordered searches (tt_near.cuh) for L2.
+// tt_near_l2.cu — the ordered kNN lists (tt_near.cuh) for L2.
 #define TT_NEAR_IMPL
-#include <cmath>
-#include <type_traits>
-
 #include "tt_near.cuh"
 
 namespace tt {
 namespace near {
-TT_NEAR_INSTANTIATE(M_L2)
+template void near_knn<M_L2>(tt_ctx*, const View&, u32, u32, u32*, f32*);
 }  // namespace near
 }  // namespace tt

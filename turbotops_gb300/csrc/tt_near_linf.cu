@@ -1,12 +1,9 @@
-// tt_near_linf.cu — the ordered searches (tt_near.cuh) for Linf.
+// tt_near_linf.cu — the ordered kNN lists (tt_near.cuh) for Linf.
 #define TT_NEAR_IMPL
-#include <cmath>
-#include <type_traits>
-
 #include "tt_near.cuh"
 
 namespace tt {
 namespace near {
-TT_NEAR_INSTANTIATE(M_LINF)
+template void near_knn<M_LINF>(tt_ctx*, const View&, u32, u32, u32*, f32*);
 }  // namespace near
 }  // namespace tt
