@@ -131,3 +131,34 @@ def test_mst(kind, n, dim, metric):
     finally:
         c.check(c.L.tt_ctx_set_knn_mode(c.h, 0))
     assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("order", ["random", "sorted", "striped"])
+@pytest.mark.parametrize("n,tau", [(900, 0.9), (1400, 1.1), (2600, 1.0)])   # rows to 32, 512 and 1,024 entries
+def test_radius_numbering(n, tau, order):
+    """Row ids spread evenly, in one band (slots overflow), in stripes."""
+    x = synth.gauss(n, 2, n)
+    if order == "sorted":
+        x = x[np.argsort(x[:, 0])]
+    elif order == "striped":
+        x = x[np.lexsort((x[:, 1], np.round(x[:, 0], 1)))]
+    for t in (0.05, tau / 3, tau):
+        _radius_check(np.ascontiguousarray(x), t, "l2")
+
+
+def test_radius_wide_ids():
+    """Rows whose ids spread over more than 2^22: sampled rows against all points."""
+    n, tau = 4_400_000, np.float32(0.002)
+    x = synth.uniform(n, 2, 3)
+    rp, ci, w = (host(t) for t in ops.radius_graph(ctx(), dev(x), float(tau), "l2"))
+    assert rp[0] == 0 and rp[-1] == len(ci)
+    for i in (0, 1, 31, 32, 77777, n // 2, n - 1):
+        a, b = int(rp[i]), int(rp[i + 1])
+        d = x - x[i]
+        dd = np.sqrt(d[:, 0].astype(np.float64) ** 2 + d[:, 1].astype(np.float64) ** 2)
+        dd[i] = np.inf
+        sure, maybe = np.flatnonzero(dd < tau * (1 - 1e-6)), np.flatnonzero(dd < tau * (1 + 1e-6))
+        ids = ci[a:b]
+        assert b - a > 20 and (np.diff(ids) > 0).all()
+        assert set(sure) <= set(ids.tolist()) <= set(maybe.tolist())
+        np.testing.assert_allclose(w[a:b], dd[ids], rtol=1e-6)

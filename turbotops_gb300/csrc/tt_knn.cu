@@ -629,7 +629,7 @@ u64 radius_graph(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, f32 t
     scan_exclusive<u64>(c, cnt, rp, n, tot);
     TT_CUDA(cudaMemcpyAsync(rp + n, tot, 8, cudaMemcpyDeviceToDevice, c->stream));
     u64 nnz = 0;
-    u32 status[2] = {0, 0};   // error word, longest row above the ordered fill's limit
+    u32 status[2] = {0, 0};   // error word, longest row (of an ordered count)
     TT_CUDA(cudaMemcpyAsync(&nnz, tot, 8, cudaMemcpyDeviceToHost, c->stream));
     TT_CUDA(cudaMemcpyAsync(status, err, sizeof(status), cudaMemcpyDeviceToHost, c->stream));
     TT_CUDA(cudaStreamSynchronize(c->stream));
@@ -637,11 +637,11 @@ u64 radius_graph(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, f32 t
     f32* w = c->arena.get<f32>(S_OUT2, nnz + 1);
     *ci_out = ci;
     *w_out = w;
-    if (ordered && status[1] == 0) {
+    if (ordered && status[1] <= near::kRadiusRow) {
         switch (kind) {
-            case M_L1: near::near_radius_fill<M_L1>(c, v, dim, tau, rp, ci, w); break;
-            case M_L2: near::near_radius_fill<M_L2>(c, v, dim, tau, rp, ci, w); break;
-            default: near::near_radius_fill<M_LINF>(c, v, dim, tau, rp, ci, w); break;
+            case M_L1: near::near_radius_fill<M_L1>(c, v, dim, tau, status[1], rp, ci, w); break;
+            case M_L2: near::near_radius_fill<M_L2>(c, v, dim, tau, status[1], rp, ci, w); break;
+            default: near::near_radius_fill<M_LINF>(c, v, dim, tau, status[1], rp, ci, w); break;
         }
         TT_CUDA(cudaStreamSynchronize(c->stream));
         return nnz;

@@ -85,10 +85,11 @@ View near_regroup(tt_ctx* c, const f32* x, u32 n, u32 dim, const u32* perm);   /
 // compile in parallel)
 template <int KIND>
 void near_knn(tt_ctx* c, const View& v, u32 dim, u32 k, u32* ids, f32* dists);
+// (*longest: the longest row, where one is longer than kRadiusRow / 2)
 template <int KIND>
 void near_radius_count(tt_ctx* c, const View& v, u32 dim, f32 tau, u64* cnt, u32* longest);
 template <int KIND>
-void near_radius_fill(tt_ctx* c, const View& v, u32 dim, f32 tau, const u64* rp, u32* ci, f32* w);
+void near_radius_fill(tt_ctx* c, const View& v, u32 dim, f32 tau, u32 longest, const u64* rp, u32* ci, f32* w);
 void near_knn_lp(tt_ctx* c, View v, u32 dim, f32 p, u32 k, u32* ids, f32* dists);   // p <= kLpMax
 constexpr f32 kLpMax = 64.0f;
 constexpr u32 kRadiusRow = 1024;   // longest row the fill sorts
@@ -856,12 +857,104 @@ __global__ void __launch_bounds__(32 * kWarps)
 }
 
 // ---- radius graph -----------------------------------------------------------
-// Row lengths (cnt by original id) and the longest row, then the rows: a
-// warp collects a row's entries (id << 32 | distance bits) in shared memory,
-// sorts them by id and writes the row. 50,000 uniform points in R^3, 240
-// neighbours: count 0.14 ms, fill 0.48 ms (exhaustive scans 4.2 and 4.05 ms);
-// the fill is bound by its sort in shared memory.
-template <int KIND, int DP, int CH, bool FILL>
+// Row lengths (cnt by original id) and the longest row, then the rows: a warp
+// collects a row's ids and distances in shared memory, orders them by id and
+// writes the row. The order is a bitonic sort of 32-bit keys in registers: an
+// id relative to the row's smallest, above the entry's place in shared memory,
+// 1 to 32 keys a lane by the row's length. Ids that spread over more than
+// 2^22 are sorted in shared memory.
+// 50,000 uniform points in R^3, 240 neighbours: count 0.14 ms, fill 0.48 ms
+// with 64-bit keys sorted in shared memory, now 0.20 (exhaustive scans 4.2 and
+// 4.05 ms). Two row capacities (launch by the longest row): the shared memory
+// of the larger leaves 24 warps an SM.
+constexpr u32 kRowBits = 10;   // of an entry's place
+static_assert(kRadiusRow <= 1u << kRowBits, "an entry's place fits its bits");
+
+// K keys a lane, ascending over (lane, key). Each merge of two ascending runs
+// compares mirrored keys first, so that every later step keeps the smaller key
+// in the lower place.
+template <int K>
+__device__ __forceinline__ void sort_lane_keys(u32 (&key)[K]) {
+    const u32 lane = threadIdx.x & 31;
+    auto order = [&](int i, int j) {
+        const u32 x = key[i], y = key[j];
+        key[i] = min(x, y);
+        key[j] = max(x, y);
+    };
+#pragma unroll
+    for (int size = 2; size <= K; size <<= 1) {
+#pragma unroll
+        for (int i = 0; i < K; ++i)
+            if ((i & (size >> 1)) == 0) order(i, i ^ (size - 1));
+#pragma unroll
+        for (int stride = size >> 2; stride; stride >>= 1)
+#pragma unroll
+            for (int i = 0; i < K; ++i)
+                if ((i & stride) == 0) order(i, i | stride);
+    }
+#pragma unroll 1
+    for (u32 size = 2; size <= 32; size <<= 1) {   // runs of size lanes
+        {
+            const bool low = (lane & (size >> 1)) == 0;
+#pragma unroll
+            for (int i = 0; i < (K + 1) / 2; ++i) {
+                const u32 x = __shfl_xor_sync(0xffffffffu, key[K - 1 - i], size - 1);
+                const u32 y = __shfl_xor_sync(0xffffffffu, key[i], size - 1);
+                key[i] = low ? min(key[i], x) : max(key[i], x);
+                if (K > 1) key[K - 1 - i] = low ? min(key[K - 1 - i], y) : max(key[K - 1 - i], y);
+            }
+        }
+#pragma unroll 1
+        for (u32 stride = size >> 2; stride; stride >>= 1) {
+            const bool low = (lane & stride) == 0;
+#pragma unroll
+            for (int i = 0; i < K; ++i) {
+                const u32 x = __shfl_xor_sync(0xffffffffu, key[i], stride);
+                key[i] = low ? min(key[i], x) : max(key[i], x);
+            }
+        }
+#pragma unroll
+        for (int stride = K >> 1; stride; stride >>= 1)
+#pragma unroll
+            for (int i = 0; i < K; ++i)
+                if ((i & stride) == 0) order(i, i | stride);
+    }
+}
+
+// A row's entries in shared memory; the ids' words take the sorted keys (a
+// padding word after every 32, so that a lane's K stores meet no other's bank).
+template <u32 ROW>
+struct Row {
+    u32 id[ROW + ROW / 32];
+    f32 d[ROW];
+};
+
+template <int K, u32 ROW>
+__device__ __forceinline__ void sort_row(Row<ROW>& R, u32 len, u32 least, u32* __restrict__ ci, f32* __restrict__ wt) {
+    const u32 lane = threadIdx.x & 31;
+    u32 key[K];
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+        const u32 e = i * 32 + lane;
+        key[i] = e < len ? (R.id[e] - least) << kRowBits | e : 0xffffffffu;
+    }
+    sort_lane_keys<K>(key);
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+        const u32 o = lane * K + i;
+        R.id[o + o / 32] = key[i];
+    }
+    __syncwarp();
+    for (u32 e = lane; e < len; e += 32) {
+        const u32 k = R.id[e + e / 32];
+        ci[e] = (k >> kRowBits) + least;
+        wt[e] = R.d[k & ((1u << kRowBits) - 1u)];
+    }
+}
+
+// ROW: the row capacity (0: count only).
+template <int KIND, int DP, int CH, u32 ROW>
 __global__ void __launch_bounds__(32 * kWarps)
     k_near_radius(View v, f32 tau, f32 bound, u64* __restrict__ cnt, u32* __restrict__ longest,
                   const u64* __restrict__ rp, u32* __restrict__ ci, f32* __restrict__ wt) {
@@ -869,14 +962,14 @@ __global__ void __launch_bounds__(32 * kWarps)
     pdl_trigger();
     __shared__ WarpQ<DP, 1> sw[kWarps];
     __shared__ DirectionOf<KIND, DP, 1> sd[projects<KIND, DP>() ? kWarps : 1];
-    __shared__ u64 srow[FILL ? kWarps : 1][FILL ? kRadiusRow : 1];
+    __shared__ Row<ROW ? ROW : 32> srow[ROW ? kWarps : 1];
     const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const u32 p0 = blockIdx.x * kWarps + w;
     if (p0 >= v.n) return;
     WarpQ<DP, 1>& W = sw[w];
     load_queries<DP, 1>(v, p0, bound, W);
-    u64* row = srow[FILL ? w : 0];
-    u32 len = 0;
+    auto& R = srow[ROW ? w : 0];
+    u32 len = 0, least = 0xffffffffu, most = 0;
     walk<KIND, DP, CH, 1>(v, W, sd[projects<KIND, DP>() ? w : 0], p0 / kTile, [&](u32, const f32(&c)[DP], u32 cid, u32) -> bool {
         const f32 s = eval<KIND, DP, CH>(RegDiff<DP>{W.q[0], c});
         bool pass = cid != W.own[0] && cid != 0xffffffffu && s <= bound;
@@ -884,60 +977,62 @@ __global__ void __launch_bounds__(32 * kWarps)
         const f32 d = KIND == M_L2 ? __fsqrt_rn(s) : s;
         pass = pass && d <= tau;
         const u32 m = __ballot_sync(0xffffffffu, pass);
-        if constexpr (FILL) {
+        if constexpr (ROW > 0) {
             const u32 o = len + __popc(m & ((1u << lane) - 1u));
-            if (pass && o < kRadiusRow) row[o] = (u64(cid) << 32) | __float_as_uint(d);
+            if (pass && o < ROW) {
+                R.id[o] = cid;
+                R.d[o] = d;
+                least = min(least, cid);
+                most = max(most, cid);
+            }
         }
         len += __popc(m);
         return false;
     });
     const u32 own = W.own[0];
-    if constexpr (!FILL) {
+    if constexpr (ROW == 0) {
         if (lane == 0) {
             cnt[own] = len;
-            if (len > kRadiusRow) atomicMax(longest, len);
+            if (len > kRadiusRow / 2) atomicMax(longest, len);
         }
     } else {
         const u64 b = rp[own];
-        if (len <= 32) {   // one entry a lane
-            __syncwarp();
-            u64 x = lane < len ? row[lane] : ~0ull;
-#pragma unroll
-            for (u32 size = 2; size <= 32; size <<= 1) {
-#pragma unroll
-                for (u32 stride = size >> 1; stride; stride >>= 1) {
-                    const u64 y = __shfl_xor_sync(0xffffffffu, x, stride);
-                    const bool up = ((lane & size) == 0) == ((lane & stride) == 0);
-                    x = up ? (x < y ? x : y) : (x < y ? y : x);
-                }
-            }
-            if (lane < len) {
-                ci[b + lane] = u32(x >> 32);
-                wt[b + lane] = __uint_as_float(u32(x));
-            }
+        const u32 m = min(len, ROW);
+        if (m == 0) return;
+        least = __reduce_min_sync(0xffffffffu, least);
+        most = __reduce_max_sync(0xffffffffu, most);
+        __syncwarp();
+        if (most - least < (1u << (32 - kRowBits)) - 1u) {   // (the largest key is the padding's)
+            if (m <= 32) sort_row<1, ROW>(R, m, least, ci + b, wt + b);
+            else if (m <= 128) sort_row<4, ROW>(R, m, least, ci + b, wt + b);
+            else if (m <= 256) sort_row<8, ROW>(R, m, least, ci + b, wt + b);
+            else if (ROW <= 512 || m <= 512) sort_row<16, ROW>(R, m, least, ci + b, wt + b);
+            else sort_row<ROW / 32, ROW>(R, m, least, ci + b, wt + b);
             return;
         }
-        const u32 m = min(len, kRadiusRow);
-        u32 P = 64;
+        u32 P = 32;
         while (P < m) P <<= 1;
-        for (u32 i = m + lane; i < P; i += 32) row[i] = ~0ull;
+        for (u32 i = m + lane; i < P; i += 32) R.id[i] = 0xffffffffu;
         __syncwarp();
         for (u32 size = 2; size <= P; size <<= 1) {
             for (u32 stride = size >> 1; stride; stride >>= 1) {
                 for (u32 i = lane; i < P / 2; i += 32) {
                     const u32 lo = 2 * i - (i & (stride - 1)), hi = lo + stride;
-                    const u64 x = row[lo], y = row[hi];
+                    const u32 x = R.id[lo], y = R.id[hi];
                     if ((x > y) == ((lo & size) == 0)) {
-                        row[lo] = y;
-                        row[hi] = x;
+                        const f32 t = R.d[lo];
+                        R.id[lo] = y;
+                        R.id[hi] = x;
+                        R.d[lo] = R.d[hi];
+                        R.d[hi] = t;
                     }
                 }
                 __syncwarp();
             }
         }
         for (u32 i = lane; i < m; i += 32) {
-            ci[b + i] = u32(row[i] >> 32);
-            wt[b + i] = __uint_as_float(u32(row[i]));
+            ci[b + i] = R.id[i];
+            wt[b + i] = R.d[i];
         }
     }
 }
@@ -1003,7 +1098,7 @@ void near_foreign(tt_ctx* c, const View& v, u32 dim, const u32* cpos, const u32*
     });
 }
 
-template <int KIND, bool FILL>
+template <int KIND, u32 ROW>
 void radius_pass(tt_ctx* c, const View& v, u32 dim, f32 tau, u64* cnt, u32* longest, const u64* rp, u32* ci, f32* w) {
     // the largest eval value a kept pair can have (host copy of bound_of)
     f32 bound = tau;
@@ -1013,7 +1108,7 @@ void radius_pass(tt_ctx* c, const View& v, u32 dim, f32 tau, u64* cnt, u32* long
     }
     with_dim<KIND>(dim, [&](auto dp, auto ch) {
         if constexpr (decltype(dp)::value <= 8) {
-            launch_pdl(k_near_radius<KIND, decltype(dp)::value, decltype(ch)::value, FILL>, div_up(v.n, kWarps),
+            launch_pdl(k_near_radius<KIND, decltype(dp)::value, decltype(ch)::value, ROW>, div_up(v.n, kWarps),
                        32 * kWarps, 0, c->stream, v, tau, bound, cnt, longest, rp, ci, w);
             TT_LAUNCH("k_near_radius");
             ++c->launches;
@@ -1023,11 +1118,12 @@ void radius_pass(tt_ctx* c, const View& v, u32 dim, f32 tau, u64* cnt, u32* long
 
 template <int KIND>
 void near_radius_count(tt_ctx* c, const View& v, u32 dim, f32 tau, u64* cnt, u32* longest) {
-    radius_pass<KIND, false>(c, v, dim, tau, cnt, longest, nullptr, nullptr, nullptr);
+    radius_pass<KIND, 0>(c, v, dim, tau, cnt, longest, nullptr, nullptr, nullptr);
 }
 template <int KIND>
-void near_radius_fill(tt_ctx* c, const View& v, u32 dim, f32 tau, const u64* rp, u32* ci, f32* w) {
-    radius_pass<KIND, true>(c, v, dim, tau, nullptr, nullptr, rp, ci, w);
+void near_radius_fill(tt_ctx* c, const View& v, u32 dim, f32 tau, u32 longest, const u64* rp, u32* ci, f32* w) {
+    if (longest <= kRadiusRow / 2) radius_pass<KIND, kRadiusRow / 2>(c, v, dim, tau, nullptr, nullptr, rp, ci, w);
+    else radius_pass<KIND, kRadiusRow>(c, v, dim, tau, nullptr, nullptr, rp, ci, w);
 }
 
 // Lp lists of one power class (a translation unit each)

@@ -8,6 +8,6 @@ namespace near {
 template void near_foreign<M_LINF>(tt_ctx*, const View&, u32, const u32*, const u32*, const u32*, const u32*, const u32*,
                                 u32*, unsigned long long*);
 template void near_radius_count<M_LINF>(tt_ctx*, const View&, u32, f32, u64*, u32*);
-template void near_radius_fill<M_LINF>(tt_ctx*, const View&, u32, f32, const u64*, u32*, f32*);
+template void near_radius_fill<M_LINF>(tt_ctx*, const View&, u32, f32, u32, const u64*, u32*, f32*);
 }  // namespace near
 }  // namespace tt
