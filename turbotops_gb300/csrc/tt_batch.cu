@@ -20,12 +20,12 @@
 //                   than kBinMax (ties, tight clusters), the cloud marked for
 //                   the radix sort
 //   k_batch_part    the kept edges as keys (d bits << 32 | index) into their
-//                   bins, in no particular order inside a bin
+//                   items, in no particular order inside an item
 //   k_batch_items   each item ordered in shared memory and written out as
 //                   EdgeList (diameter, vertex pair)
-// A distance is moved twice that way (into its bin, and out in order), where
+// A distance is moved twice that way (into its item, and out in order), where
 // the four 8-bit passes of a radix sort read it eight times and wrote it four
-// (512 clouds, 312 M kept edges: 13.6 ms with the edge lists, now 7.0). The bin
+// (512 clouds, 312 M kept edges: 13.6 ms with the edge lists, now 4.4). The bin
 // of a distance is floor(d * bins / radius) in floats: monotone in d, so the
 // bins partition the filtration order whatever the rounding.
 // The marked clouds go through
@@ -108,23 +108,22 @@ __global__ void k_batch_radius(const u32* __restrict__ rowmax, const u32* __rest
 // A run of a cloud's rows holding about kChunkPairs pairs.
 struct Chunk {
     u32 cloud, row0, row1;
-    u32 pad;
-    u64 rank;   // its place in `ranks`: per bin, the cloud's edges of earlier-counted chunks
 };
 constexpr u64 kChunkPairs = 64 * 1024;
 constexpr u32 kMaxBins = 8192;
-constexpr int kPartThreads = 1024;
-// One block an SM (by its shared memory): the blocks then write into the bins
-// of about ten million edges at a time, which L2 holds until their lines are
-// full. With four blocks an SM on runs twice as long, partly written sectors
-// went out to memory and came back (8.2 ms for 312 M edges; now 3.4, bound by
-// the scattered 8-byte stores).
-constexpr size_t kPartSmem = 120 * 1024;
-constexpr u32 kItemCap = 4096;                 // edges an item orders at once
-constexpr u32 kItemStep = 2560;                // an item: the bins that start in one step of this many edges ...
+// A run of kPartPairs pairs of a cloud, in index order.
+struct Part {
+    u32 cloud, first;
+};
+constexpr int kPartThreads = 512;
+constexpr u32 kPartPer = 16;   // pairs a thread
+constexpr u32 kPartPairs = kPartThreads * kPartPer;
+constexpr size_t kPartSmemMax = 8 * size_t(kPartPairs) + 10 * size_t(kMaxBins);   // keys, items' words, bins' items
+constexpr u32 kItemCap = 3840;                 // edges an item orders at once
+constexpr u32 kItemStep = 2304;                // an item: the bins that start in one step of this many edges ...
 constexpr u32 kBinMax = kItemCap - kItemStep;  // ... and no bin longer than this
-constexpr int kItemThreads = 256;
-constexpr u32 kSlots = 2048;                   // linear slots an item's keys are placed by
+constexpr int kItemThreads = 384;
+constexpr u32 kSlots = 1920;                   // linear slots an item's keys are placed by
 struct Item {
     u32 begin, end;   // edges of the cloud, relative to its first
 };
@@ -161,13 +160,11 @@ __device__ __forceinline__ void for_row(const f32* __restrict__ row, u32 i, f32 
 }
 
 // Row counts and the cloud's histogram, one block a chunk: the bins counted in
-// shared memory first (one global atomic a bin and chunk; its old value is
-// where the chunk's edges go within the bin).
+// shared memory first (one global atomic a bin and chunk).
 constexpr int kHistThreads = 512;
 __global__ void __launch_bounds__(kHistThreads)
     k_batch_hist(const f32* __restrict__ mats, CloudTable T, const Chunk* __restrict__ chunks,
-                 const u32* __restrict__ radius, u64* __restrict__ row_cnt, u32* __restrict__ hist,
-                 u32* __restrict__ ranks) {
+                 const u32* __restrict__ radius, u64* __restrict__ row_cnt, u32* __restrict__ hist) {
     __shared__ u32 h[kMaxBins];
     const Chunk ck = chunks[blockIdx.x];
     const u32 c = ck.cloud, n = T.sizes[c], b0 = T.bin_off[c], bins = T.bin_off[c + 1] - b0;
@@ -189,7 +186,8 @@ __global__ void __launch_bounds__(kHistThreads)
         if (lane == 0) row_cnt[T.pt_off[c] + i] = kept;
     }
     __syncthreads();
-    for (u32 b = threadIdx.x; b < bins; b += kHistThreads) ranks[ck.rank + b] = h[b] ? atomicAdd(&hist[b0 + b], h[b]) : 0u;
+    for (u32 b = threadIdx.x; b < bins; b += kHistThreads)
+        if (h[b]) atomicAdd(&hist[b0 + b], h[b]);
 }
 
 // Exclusive scan over the 1,024 threads of the block (u32).
@@ -215,12 +213,13 @@ __device__ __forceinline__ u32 block_scan1024(u32 v, u32* warp_tot, u32& total) 
     return pre + inc - v;
 }
 
-// One block a cloud: its bins' starts (hist becomes the cursors of the
-// partition), its items, and whether it is left to the radix sort; edge_off
-// from the scanned row counts (the last block adds the total).
+// One block a cloud: its items with the partition's cursors, the item of every
+// bin, and whether the cloud is left to the radix sort; edge_off from the
+// scanned row counts (the last block adds the total).
 __global__ void __launch_bounds__(1024) k_batch_bins(CloudTable T, u32 clouds, const u64* __restrict__ row_off,
                                                      const unsigned long long* __restrict__ total,
-                                                     u32* __restrict__ hist, Item* __restrict__ items,
+                                                     const u32* __restrict__ hist, u16* __restrict__ bin_item,
+                                                     Item* __restrict__ items, u32* __restrict__ cursor,
                                                      u32* __restrict__ radix, u64* __restrict__ edge_off) {
     __shared__ u32 wt[32];
     const u32 c = blockIdx.x, b0 = T.bin_off[c], bins = T.bin_off[c + 1] - b0;
@@ -276,11 +275,12 @@ __global__ void __launch_bounds__(1024) k_batch_bins(CloudTable T, u32 clouds, c
             const u32 st = run / kItemStep;
             if (st != p && !rad) {
                 items[s0 + slot].begin = run;
+                cursor[s0 + slot] = run;
                 if (slot) items[s0 + slot - 1].end = run;
             }
             slot += st != p;
             p = st;
-            hist[b0 + b] = run;
+            bin_item[b0 + b] = u16(slot - 1);
         }
         run += v[q];
     }
@@ -289,40 +289,13 @@ __global__ void __launch_bounds__(1024) k_batch_bins(CloudTable T, u32 clouds, c
     for (u32 q = nitems + threadIdx.x; q < cap; q += blockDim.x) items[s0 + q] = Item{0, 0};
 }
 
-// The kept edges of a chunk into their bins, one block a chunk.
-__global__ void __launch_bounds__(kPartThreads)
-    k_batch_part(const f32* __restrict__ mats, CloudTable T, const Chunk* __restrict__ chunks,
-                 const u32* __restrict__ radius, const u32* __restrict__ radix, const u64* __restrict__ edge_off,
-                 const u32* __restrict__ bin_start, const u32* __restrict__ ranks, u64* __restrict__ keys) {
-    extern __shared__ u32 h[];   // [kMaxBins] (of kPartSmem bytes): the next free place of every bin
-    const Chunk ck = chunks[blockIdx.x];
-    const u32 c = ck.cloud;
-    if (radix[c]) return;
-    const u32 n = T.sizes[c], b0 = T.bin_off[c], bins = T.bin_off[c + 1] - b0;
-    const f32 thr = __uint_as_float(radius[c]), scale = __fdiv_rn(f32(bins), thr);
-    for (u32 b = threadIdx.x; b < bins; b += kPartThreads) h[b] = bin_start[b0 + b] + ranks[ck.rank + b];
-    __syncthreads();
-    const f32* mat = mats + T.mat_off[c];
-    u64* out = keys + edge_off[c];
-    for (u32 i = ck.row0 + (threadIdx.x >> 5); i < ck.row1; i += kPartThreads / 32) {
-        const u32 rbase = u32(u64(i) * (i - 1) / 2);
-        for_row(mat + u64(i) * n, i, thr, [&](const f32(&d)[kRowLoads], u32 j) {
-            u32 pos[kRowLoads];
-#pragma unroll
-            for (int q = 0; q < kRowLoads; ++q)
-                if (j + 32 * q < i && d[q] <= thr) pos[q] = atomicAdd(&h[bin_of(d[q], scale, bins)], 1u);
-#pragma unroll
-            for (int q = 0; q < kRowLoads; ++q)
-                if (j + 32 * q < i && d[q] <= thr)
-                    out[pos[q]] = (u64(__float_as_uint(d[q])) << 32) | (rbase + j + 32 * q);
-        });
-    }
-}
-
 // decode_edge for idx < 2^31 in 32-bit arithmetic (v <= 65,536, so v (v - 1)
-// fits; the closed form in FP32 is within one of the answer).
+// fits; the closed form in FP32 is within one of the answer, whose 2^17 steps
+// are far wider than the approximate root's relative error of 2^-22).
 __device__ __forceinline__ void decode_edge31(u32 idx, u32& a, u32& b) {
-    u32 v = u32((1.0f + sqrtf(fmaf(8.0f, f32(idx), 1.0f))) * 0.5f);
+    f32 r;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(fmaf(8.0f, f32(idx), 1.0f)));
+    u32 v = u32((1.0f + r) * 0.5f);
     u32 t = v * (v - 1u) / 2u;
     if (t > idx) {
         --v;
@@ -336,17 +309,101 @@ __device__ __forceinline__ void decode_edge31(u32 idx, u32& a, u32& b) {
     b = idx - t;
 }
 
+// The kept edges of a run of pairs into their items, one block a run: counted
+// by item, placed item by item in shared memory and written from there, so
+// that the stores of a warp are runs of neighbouring words (1,100 points: 240
+// items, 25 edges a run); the places in an item come from its cursor. Written
+// directly into 8,192 bins, every edge's store was a sector of its own: 3.45 ms
+// for 312 M edges, now 1.79 (6,144 pairs a block 2.4, 12,288 2.6).
+__global__ void __launch_bounds__(kPartThreads, 2)
+    k_batch_part(const f32* __restrict__ mats, CloudTable T, const Part* __restrict__ parts,
+                 const u32* __restrict__ radius, const u32* __restrict__ radix, const u64* __restrict__ edge_off,
+                 const u16* __restrict__ bin_item, u32* __restrict__ cursor, u32 max_items, u64* __restrict__ keys) {
+    extern __shared__ u64 sk[];   // [kPartPairs]
+    u32* cnt = reinterpret_cast<u32*>(sk + kPartPairs);   // [max_items] edges, then the first place
+    u32* to = cnt + max_items;                            // [max_items] the item's place in the keys less cnt
+    u16* item_of = reinterpret_cast<u16*>(to + max_items);   // [bins]
+    __shared__ u32 wt[kPartThreads / 32];
+    const Part pt = parts[blockIdx.x];
+    const u32 c = pt.cloud;
+    if (radix[c]) return;
+    const u32 n = T.sizes[c], b0 = T.bin_off[c], bins = T.bin_off[c + 1] - b0;
+    const u32 s0 = T.item_off[c], items = min(T.item_off[c + 1] - s0, bins);
+    const u32 pairs = u32(u64(n) * (n - 1) / 2), m = min(kPartPairs, pairs - pt.first);
+    const f32 thr = __uint_as_float(radius[c]), scale = __fdiv_rn(f32(bins), thr);
+    const u32 tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const f32* mat = mats + T.mat_off[c];
+    f32 d[kPartPer];
+#pragma unroll
+    for (u32 q = 0; q < kPartPer; ++q) {
+        const u32 e = q * kPartThreads + tid;
+        u32 i, j;
+        decode_edge31(pt.first + e, i, j);
+        d[q] = e < m ? mat[u64(i) * n + j] : INFINITY;
+    }
+    for (u32 b = tid; b < items; b += kPartThreads) cnt[b] = 0;
+    for (u32 b = tid; b < bins; b += kPartThreads) item_of[b] = bin_item[b0 + b];
+    __syncthreads();
+    u32 at[kPartPer];   // item, place in it (both below 2^13)
+#pragma unroll
+    for (u32 q = 0; q < kPartPer; ++q) {
+        const u32 e = q * kPartThreads + tid;
+        at[q] = 0xffffffffu;
+        if (e < m && d[q] <= thr) {
+            const u32 it = item_of[bin_of(d[q], scale, bins)];
+            at[q] = it << 16 | atomicAdd(&cnt[it], 1u);
+        }
+    }
+    __syncthreads();
+    const u32 per = (items + kPartThreads - 1) / kPartThreads, b1 = min(items, (tid + 1) * per);
+    u32 sum = 0;
+    for (u32 b = tid * per; b < b1; ++b) sum += cnt[b];
+    u32 inc = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const u32 y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= u32(o)) inc += y;
+    }
+    if (lane == 31) wt[w] = inc;
+    __syncthreads();
+    u32 run = inc - sum, kept = 0;
+#pragma unroll
+    for (u32 q = 0; q < kPartThreads / 32; ++q) {
+        run += q < w ? wt[q] : 0u;
+        kept += wt[q];
+    }
+    for (u32 b = tid * per; b < b1; ++b) {
+        const u32 k = cnt[b];
+        cnt[b] = run;
+        to[b] = (k ? atomicAdd(&cursor[s0 + b], k) : 0u) - run;
+        run += k;
+    }
+    __syncthreads();
+#pragma unroll
+    for (u32 q = 0; q < kPartPer; ++q)
+        if (at[q] != 0xffffffffu)
+            sk[cnt[at[q] >> 16] + (at[q] & 0xffffu)] =
+                (u64(__float_as_uint(d[q])) << 32) | (pt.first + q * kPartThreads + tid);
+    __syncthreads();
+    u64* out = keys + edge_off[c];
+    for (u32 e = tid; e < kept; e += kPartThreads) {
+        const u64 key = sk[e];
+        out[to[item_of[bin_of(__uint_as_float(u32(key >> 32)), scale, bins)]] + e] = key;
+    }
+}
+
 // One item: its keys counted into kSlots linear slots of its distance range
 // (about one key a slot), placed slot by slot in shared memory, and the few
 // keys of a slot put in order by insertion. An item whose distances crowd (a
 // slot of more than kSlotMax keys: ties) is ordered by a bitonic sort instead.
-// Then written out in order. 312 M edges: 3.1 ms, 1.9 instructions a cycle,
-// bound by shared-memory latency at 23 warps an SM.
+// Then written out in order. Bound by shared-memory latency and so by the warps
+// an SM: 312 M edges 3.1 ms with 256 threads on up to 4,096 keys (23 warps an
+// SM), now 2.27 with 384 on up to 3,840 (40 registers, 48 warps).
 constexpr u32 kSlotMax = 24;
-__global__ void __launch_bounds__(kItemThreads)
+__global__ void __launch_bounds__(kItemThreads, 4)
     k_batch_items(const Item* __restrict__ items, const u32* __restrict__ item_cloud, const u64* __restrict__ edge_off,
                   const u64* __restrict__ keys, f32* __restrict__ ed, int32_t* __restrict__ ev) {
-    __shared__ u64 sk[kItemCap];
+    __shared__ u64 sk[4096];   // kItemCap, up to the bitonic sort's power of two
     __shared__ u32 cnt[kSlots];
     __shared__ u32 red[2][kItemThreads / 32];
     __shared__ u32 wt[kItemThreads / 32];
@@ -356,17 +413,18 @@ __global__ void __launch_bounds__(kItemThreads)
     const u64 base = edge_off[item_cloud[blockIdx.x]] + it.begin;
     const u32 tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     constexpr u32 kPer = kItemCap / kItemThreads;
+    static_assert(kPer * kItemThreads == kItemCap && kSlots % kItemThreads == 0 && kSlots <= kItemCap && kItemCap <= 4096);
     u64 k[kPer];
     u32 lo = 0xffffffffu, hi = 0;
 #pragma unroll
     for (u32 q = 0; q < kPer; ++q) {
         const u32 e = q * kItemThreads + tid;
+        if (e < kSlots) cnt[e] = 0;
         k[q] = e < m ? keys[base + e] : ~0ull;
         if (e < m) {
             lo = min(lo, u32(k[q] >> 32));
             hi = max(hi, u32(k[q] >> 32));
         }
-        if (e < kSlots) cnt[e] = 0;
     }
     lo = __reduce_min_sync(0xffffffffu, lo);
     hi = __reduce_max_sync(0xffffffffu, hi);
@@ -381,6 +439,7 @@ __global__ void __launch_bounds__(kItemThreads)
 #pragma unroll
     for (u32 q = 0; q < kPer; ++q) {
         const u32 e = q * kItemThreads + tid;
+        if (q * kItemThreads >= m) break;
         if (e < m) {
             const f32 d = __uint_as_float(u32(k[q] >> 32));
             const u32 s = bin_of(__fsub_rn(d, dmin), scale, kSlots);
@@ -421,6 +480,7 @@ __global__ void __launch_bounds__(kItemThreads)
 #pragma unroll
         for (u32 q = 0; q < kPer; ++q) {
             const u32 e = q * kItemThreads + tid;
+            if (q * kItemThreads >= m) break;
             if (e < m) sk[cnt[at[q] >> 16] + (at[q] & 0xffffu)] = k[q];
         }
         __syncthreads();
@@ -444,6 +504,7 @@ __global__ void __launch_bounds__(kItemThreads)
         while (P < m) P <<= 1;
 #pragma unroll
         for (u32 q = 0; q < kPer; ++q) sk[q * kItemThreads + tid] = k[q];   // (past m: ~0)
+        for (u32 e = kItemCap + tid; e < P; e += kItemThreads) sk[e] = ~0ull;
         __syncthreads();
         for (u32 size = 2; size <= P; size <<= 1)
             for (u32 stride = size >> 1; stride; stride >>= 1) {
@@ -564,7 +625,6 @@ struct Batch {
     u32* radius = nullptr;
     u64* pt_off = nullptr;
     u64* mat_off = nullptr;
-    u64* pair_off = nullptr;   // first key slot of every cloud's pairs
     u32* sizes = nullptr;
     Tile* tiles[kNumShapes] = {};
     u32 ntiles[kNumShapes] = {};
@@ -578,15 +638,20 @@ struct Batch {
     u64* row_cnt = nullptr;    // kept pairs per row, then their exclusive scan
     u64* row_off = nullptr;
     unsigned long long* count = nullptr;
-    Chunk* chunks = nullptr;        // row runs of the histogram and the partition
+    Chunk* chunks = nullptr;        // row runs of the histogram
     u32 nchunks = 0;
+    Part* parts = nullptr;          // pair runs of the partition
+    u32 nparts = 0;
+    u32 part_items = 0;             // most items of a cloud
+    size_t part_smem = 0;
     u32* bin_off = nullptr;         // first bin of every cloud
     u32 total_bins = 0;
-    u32* hist = nullptr;            // bin counts, then the bins' starts
-    u32* ranks = nullptr;           // per chunk and bin (Chunk::rank)
+    u32* hist = nullptr;            // bin counts
+    u16* bin_item = nullptr;        // the item of every bin
     u32* item_off = nullptr;        // first item slot of every cloud
     u32 total_items = 0;
     Item* items = nullptr;
+    u32* cursor = nullptr;          // the next free place of every item
     u32* item_cloud = nullptr;
     u32* radix = nullptr;           // clouds left to the radix sort
     u64* edge_off = nullptr;
@@ -703,13 +768,14 @@ struct Batch {
         k_batch_radius<<<g2, 256, 0, s>>>(rowmax, row_cloud, total_pts, radius);
         TT_LAUNCH("k_batch_radius");
         const CloudTable T{pt_off, mat_off, sizes, bin_off, item_off};
-        k_batch_hist<<<nchunks, kHistThreads, 0, s>>>(mats, T, chunks, radius, row_cnt, hist, ranks);
+        k_batch_hist<<<nchunks, kHistThreads, 0, s>>>(mats, T, chunks, radius, row_cnt, hist);
         TT_LAUNCH("k_batch_hist");
         scan_exclusive<u64>(&sctx, row_cnt, row_off, total_pts, reinterpret_cast<u64*>(count), 0);
-        k_batch_bins<<<clouds, 1024, 0, s>>>(T, clouds, row_off, count, hist, items, radix, edge_off);
+        k_batch_bins<<<clouds, 1024, 0, s>>>(T, clouds, row_off, count, hist, bin_item, items, cursor, radix, edge_off);
         TT_LAUNCH("k_batch_bins");
-        k_batch_part<<<nchunks, kPartThreads, kPartSmem, s>>>(mats, T, chunks, radius, radix, edge_off, hist,
-                                                              ranks, keys);
+        if (nparts)
+            k_batch_part<<<nparts, kPartThreads, part_smem, s>>>(mats, T, parts, radius, radix, edge_off, bin_item,
+                                                                 cursor, part_items, keys);
         TT_LAUNCH("k_batch_part");
         if (total_items)
             k_batch_items<<<total_items, kItemThreads, 0, s>>>(items, item_cloud, edge_off, keys, ed, ev);
@@ -764,13 +830,13 @@ Batch* batch_create(tt_ctx* c, const u32* sizes_h, u32 clouds, u32 dim, int kind
         b->sctx.device = c->device;
         b->sctx.sms = c->sms;
         TT_CUDA(cudaStreamCreateWithFlags(&b->sctx.stream, cudaStreamNonBlocking));
-        TT_CUDA(cudaFuncSetAttribute(k_batch_part, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPartSmem)));
-        std::vector<u64> pt_off(clouds + 1, 0), mat_off(clouds + 1, 0), pair_off(clouds + 1, 0);
+        std::vector<u64> pt_off(clouds + 1, 0), mat_off(clouds + 1, 0);
         std::vector<Tile> tiles[kNumShapes];
         std::vector<u32> row_cloud;
         u64 pairs = 0;
         std::vector<Chunk> chunks;
-        u64 nranks = 0;
+        std::vector<Part> parts;
+        u32 most_bins = 0;
         std::vector<u32> bin_off(clouds + 1, 0), item_off(clouds + 1, 0), item_cloud;
         for (u32 q = 0; q < clouds; ++q) {
             const u32 n = sizes_h[q];
@@ -779,7 +845,6 @@ Batch* batch_create(tt_ctx* c, const u32* sizes_h, u32 clouds, u32 dim, int kind
             pt_off[q + 1] = pt_off[q] + n;
             mat_off[q + 1] = mat_off[q] + u64(n) * n;
             pairs += u64(n) * (n - 1) / 2;
-            pair_off[q + 1] = pairs;
             for (int si = 0; si < kNumShapes; ++si)   // the tiles on and above the diagonal
                 for (u32 i0 = 0; i0 < n; i0 += u32(kShapes[si].r))
                     for (u32 j0 = i0; j0 < n; j0 += u32(kShapes[si].c)) tiles[si].push_back(Tile{q, i0, j0});
@@ -793,13 +858,17 @@ Batch* batch_create(tt_ctx* c, const u32* sizes_h, u32 clouds, u32 dim, int kind
             for (u32 i0 = 0; i0 < n;) {
                 u32 i1 = i0;
                 for (u64 held = 0; i1 < n && held < kChunkPairs; ++i1) held += i1;
-                chunks.push_back(Chunk{q, i0, i1, 0, nranks});
-                nranks += bins;
+                chunks.push_back(Chunk{q, i0, i1});
                 i0 = i1;
+            }
+            if (bins > 1) {
+                for (u64 i0 = 0; i0 < cp; i0 += kPartPairs) parts.push_back(Part{q, u32(i0)});
+                most_bins = std::max(most_bins, bins);
             }
             bin_off[q + 1] = bin_off[q] + bins;
             const u32 cap = bins > 1 ? u32(cp / kItemStep) + 1 : 0;
             item_off[q + 1] = item_off[q] + cap;
+            b->part_items = std::max(b->part_items, std::min(cap, bins));
             item_cloud.insert(item_cloud.end(), cap, q);
         }
         // the segmented sort's capacity: every cloud's largest key count
@@ -819,7 +888,6 @@ Batch* batch_create(tt_ctx* c, const u32* sizes_h, u32 clouds, u32 dim, int kind
         b->radius = b->alloc<u32>(clouds);
         b->pt_off = b->alloc<u64>(clouds + 1);
         b->mat_off = b->alloc<u64>(clouds + 1);
-        b->pair_off = b->alloc<u64>(clouds + 1);
         b->sizes = b->alloc<u32>(clouds);
         for (int si = 0; si < kNumShapes; ++si) {
             b->ntiles[si] = u32(tiles[si].size());
@@ -837,10 +905,15 @@ Batch* batch_create(tt_ctx* c, const u32* sizes_h, u32 clouds, u32 dim, int kind
         b->total_bins = bin_off[clouds];
         b->bin_off = b->alloc<u32>(clouds + 1);
         b->hist = b->alloc<u32>(b->total_bins);
-        b->ranks = b->alloc<u32>(nranks);
+        b->bin_item = b->alloc<u16>(b->total_bins);
+        b->nparts = u32(parts.size());
+        b->parts = b->alloc<Part>(parts.size());
+        b->part_smem = 8 * size_t(kPartPairs) + 8 * size_t(b->part_items) + 2 * size_t(most_bins);
+        TT_CUDA(cudaFuncSetAttribute(k_batch_part, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPartSmemMax)));
         b->total_items = item_off[clouds];
         b->item_off = b->alloc<u32>(clouds + 1);
         b->items = b->alloc<Item>(b->total_items);
+        b->cursor = b->alloc<u32>(b->total_items);
         b->item_cloud = b->alloc<u32>(b->total_items);
         b->radix = b->alloc<u32>(clouds);
         b->edge_off = b->alloc<u64>(clouds + 1);
@@ -853,9 +926,10 @@ Batch* batch_create(tt_ctx* c, const u32* sizes_h, u32 clouds, u32 dim, int kind
         cudaStream_t s = b->sctx.stream;
         TT_CUDA(cudaMemcpyAsync(b->pt_off, pt_off.data(), 8 * (clouds + 1), cudaMemcpyHostToDevice, s));
         TT_CUDA(cudaMemcpyAsync(b->mat_off, mat_off.data(), 8 * (clouds + 1), cudaMemcpyHostToDevice, s));
-        TT_CUDA(cudaMemcpyAsync(b->pair_off, pair_off.data(), 8 * (clouds + 1), cudaMemcpyHostToDevice, s));
         TT_CUDA(cudaMemcpyAsync(b->sizes, sizes_h, 4 * clouds, cudaMemcpyHostToDevice, s));
         TT_CUDA(cudaMemcpyAsync(b->chunks, chunks.data(), sizeof(Chunk) * chunks.size(), cudaMemcpyHostToDevice, s));
+        if (!parts.empty())
+            TT_CUDA(cudaMemcpyAsync(b->parts, parts.data(), sizeof(Part) * parts.size(), cudaMemcpyHostToDevice, s));
         TT_CUDA(cudaMemcpyAsync(b->bin_off, bin_off.data(), 4 * (clouds + 1), cudaMemcpyHostToDevice, s));
         TT_CUDA(cudaMemcpyAsync(b->item_off, item_off.data(), 4 * (clouds + 1), cudaMemcpyHostToDevice, s));
         if (!item_cloud.empty())
