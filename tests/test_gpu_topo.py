@@ -154,3 +154,16 @@ def test_adjoint_at_configuration_size():
         got = np.stack([b.h1_birth[s1:e1].cpu().numpy(), b.h1_death[s1:e1].cpu().numpy()], 1)
         key = lambda a: a[np.lexsort((a[:, 1], a[:, 0]))]  # noqa: E731
         assert np.array_equal(key(got), key(dg[1])), q
+
+
+@pytest.mark.parametrize("sizes", [[1, 2, 64, 129, 600, 0, 3], [40] * 33, [2048, 300, 300], [2049, 300, 300]])
+def test_forward_streams(sizes):
+    """Front ends on several streams (small clouds) against one after the other."""
+    x = torch.from_numpy(np.concatenate([synth.uniform(n, 3, 7 + n) if n else np.zeros((0, 3), np.float32)
+                                         for n in sizes])).cuda()
+    b = topo.diagrams(x, sizes, threads=1)
+    for _ in range(3):
+        a = topo.diagrams(x, sizes, threads=0)
+        for f in ["h0_offset", "h0_death", "h0_edge", "h1_offset", "h1_birth", "h1_death", "h1_birth_edge",
+                  "h1_death_edge"]:
+            assert torch.equal(torch.as_tensor(getattr(a, f)), torch.as_tensor(getattr(b, f))), f

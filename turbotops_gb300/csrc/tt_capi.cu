@@ -222,6 +222,7 @@ int tt_ctx_create(int device, void* stream, tt_ctx** out) {
 
 void tt_ctx_destroy(tt_ctx* c) {
     if (!c) return;
+    for (tt_ctx* l : c->lanes) tt_ctx_destroy(l);
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     c->arena.release();

@@ -170,6 +170,7 @@ struct tt_ctx {
     bool fin_pending = false;       // ... not yet read
     cudaStream_t side = nullptr;    // kernels overlapped with the main stream's (created on first use)
     cudaEvent_t side_ev[2] = {nullptr, nullptr};
+    std::vector<tt_ctx*> lanes;     // tt_topo_forward: contexts of its other streams (at most 5, owned)
 };
 
 namespace tt {

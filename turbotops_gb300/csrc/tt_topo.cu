@@ -20,9 +20,11 @@
 //   Lp   sign(diff_k) (|diff_k| / d)^(p - 1)
 // one thread per edge, float atomics into the gradient.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <condition_variable>
 #include <cstdlib>
+#include <exception>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -119,17 +121,15 @@ struct Cloud {
 
 constexpr u64 kStagingMax = u64(256) << 20;
 
-// Takes the clouds' outputs off the device, one after the other.
+// The bytes of staging a cloud's outputs may take: matrix and keys, H0, a few
+// columns a point.
+u64 staging_bytes(u64 n) { return 8 * n * n + 256 * n + 1024; }
+
+// Takes a cloud's outputs off the device, into its part of the staging.
 struct Staging {
-    tt_ctx* c;
-    unsigned char* base = nullptr;
-    u64 left = 0;
-    Staging(tt_ctx* ctx, const uint32_t* sizes, u32 count) : c(ctx) {
-        u64 want = 0;   // matrix and keys, H0, a few columns a point
-        for (u32 q = 0; q < count; ++q) want += 8 * u64(sizes[q]) * sizes[q] + 256 * u64(sizes[q]) + 1024;
-        left = std::min(want, kStagingMax);
-        if (left) base = static_cast<unsigned char*>(c->staging.get(left));
-    }
+    cudaStream_t stream;
+    unsigned char* base;
+    u64 left;
     template <typename T>
     void take(Out<T>& o, const T* dev, u64 count) {
         o.count = count;
@@ -142,33 +142,61 @@ struct Staging {
             o.own.resize(count);
             o.p = o.own.data();
         }
-        if (count) TT_CUDA(cudaMemcpyAsync(o.p, dev, count * sizeof(T), cudaMemcpyDeviceToHost, c->stream));
+        if (count) TT_CUDA(cudaMemcpyAsync(o.p, dev, count * sizeof(T), cudaMemcpyDeviceToHost, stream));
     }
 };
 
-// Hands clouds from the thread that runs their device front end to the
+// The front end of a cloud of a few hundred points is a chain of some 25 small
+// kernels and two waits, so the clouds' chains run on kLanes streams, each with
+// a context (workspaces) of its own and driven by its own thread. A gradient
+// step over 64 clouds of 100 points 18.0 ms with one lane, 6.3 with four, 5.0
+// with six, 4.4 with eight; of 512 points 20.9, 17.5, 17.1 and 17.5 (the
+// reductions then take the time, and need the threads). Clouds beyond kLaneMaxN
+// fill the chip by themselves more and more (12 of 2,048 points: 414 ms, 407 with
+// six), and their workspaces are not held several times. Two clouds gain nothing
+// (2 x 300 points 2.46 ms, two lanes 2.56; 3 x 256 points 2.37 and 2.29).
+constexpr u32 kLanes = 6;
+constexpr u32 kLaneMaxN = 2048;
+
+tt_ctx* lane_context(tt_ctx* c, u32 lane) {   // lane >= 1; kept by c
+    while (c->lanes.size() < lane) {
+        auto* l = new tt_ctx;
+        c->lanes.push_back(l);
+        l->device = c->device;
+        l->sms = c->sms;
+        l->own_stream = true;
+        TT_CUDA(cudaStreamCreateWithFlags(&l->stream, cudaStreamNonBlocking));
+    }
+    if (!c->lanes[lane - 1]->stream) TT_CUDA(cudaStreamCreateWithFlags(&c->lanes[lane - 1]->stream, cudaStreamNonBlocking));
+    return c->lanes[lane - 1];
+}
+
+// Hands clouds from the threads that run their device front ends to the
 // threads that reduce them: a cloud is published once its outputs are on the
-// host, and reducers take published clouds in order, so the reductions of the
-// first clouds overlap the front end of the later ones and a thread that
-// finishes early takes the next cloud. Each cloud's reduction is independent
-// of the others, so the bars do not depend on the schedule.
+// host, and reducers take clouds in the order they were published, so the
+// reductions of the first clouds overlap the front end of the later ones and a
+// thread that finishes early takes the next cloud. Each cloud's reduction is
+// independent of the others, so the bars do not depend on the schedule.
 struct CloudQueue {
     std::mutex m;
     std::condition_variable cv;
-    u32 count, ready = 0, next = 0;
+    std::vector<u32> ready;
+    size_t next = 0, expected;
     bool stop = false;
-    explicit CloudQueue(u32 c) : count(c) {}
-    // the next cloud to reduce; count when none is left (or after stop)
+    explicit CloudQueue(size_t e) : expected(e) {}
+    // the next cloud to reduce; NOV when none is left (or after stop)
     u32 take() {
         std::unique_lock<std::mutex> lk(m);
-        cv.wait(lk, [&] { return stop || next < ready || next >= count; });
-        if (stop || next >= count) return count;
-        return next++;
+        cv.wait(lk, [&] { return stop || next < ready.size() || next >= expected; });
+        if (stop || next >= expected) return NOV;
+        const u32 q = ready[next++];
+        if (next >= expected) cv.notify_all();   // none is left for those that wait
+        return q;
     }
     void publish(u32 q) {
         {
             std::lock_guard<std::mutex> lk(m);
-            ready = q + 1;
+            ready.push_back(q);
         }
         cv.notify_all();
     }
@@ -178,6 +206,10 @@ struct CloudQueue {
             stop = true;
         }
         cv.notify_all();
+    }
+    bool halted() {
+        std::lock_guard<std::mutex> lk(m);
+        return stop;
     }
 };
 
@@ -203,55 +235,70 @@ extern "C" int tt_topo_forward(tt_ctx* c, const float* x, const uint32_t* sizes,
         if (kind < TT_METRIC_L1 || kind > TT_METRIC_LP) invalid("metric: unknown kind");
         if (kind == TT_METRIC_LP && !(p >= 1.0f)) invalid("metric: p must be in [1, inf]");
         std::vector<Cloud> cl(count);
-        // host reducers (the calling thread joins them after the front end)
+        u64 points = 0;
+        u32 maxn = 0, clouds = 0;
+        for (u32 q = 0; q < count; ++q) {
+            cl[q].n = sizes[q];
+            cl[q].off = points;
+            points += sizes[q];
+            maxn = std::max(maxn, sizes[q]);
+            clouds += sizes[q] > 0;
+        }
+        // host reducers (the calling thread and the other front-end threads
+        // join them after the front end)
         u32 nt = threads > 0 ? u32(threads) : std::max(1u, std::thread::hardware_concurrency());
         // threads beyond one per cloud go into each cloud's own reduction
         const unsigned per_cloud = count ? std::max<u32>(1, nt / std::max<u32>(count, 1)) : 1;
         nt = std::min<u32>(nt, std::max<u32>(count, 1));
-        CloudQueue queue(count);
-        std::vector<std::string> errs(nt);
-        auto work = [&](u32 t) {
+        const u32 lanes = maxn <= kLaneMaxN && clouds > 2 ? std::min(nt, kLanes) : 1;
+        std::vector<tt_ctx*> lane(lanes, c);
+        for (u32 l = 1; l < lanes; ++l) lane[l] = lane_context(c, l);
+        // every cloud's part of the staging
+        u64 want = 0;
+        for (u32 q = 0; q < count; ++q) want += staging_bytes(cl[q].n);
+        const u64 staged = std::min(want, kStagingMax);
+        auto* staging = staged ? static_cast<unsigned char*>(c->staging.get(staged)) : nullptr;
+        std::vector<Staging> out_of(count);
+        u64 at = 0;
+        for (u32 q = 0; q < count; ++q) {
+            const u64 bytes = staging_bytes(cl[q].n) & ~u64(15);
+            const bool fits = at + bytes <= staged;
+            out_of[q] = Staging{nullptr, fits ? staging + at : nullptr, fits ? bytes : 0};
+            if (fits) at += bytes;
+        }
+        CloudQueue queue(clouds);
+        std::vector<std::exception_ptr> errs(nt);
+        auto reduce = [&](Cloud& C) {
+            std::vector<host::Entry> cols(C.ci.size());
+            for (u64 i = 0; i < cols.size(); ++i) cols[i] = host::Entry{C.ci[i], C.cd[i]};
+            host::HostComplex hc{C.mat.data(), nullptr, nullptr, nullptr, C.n, C.thr};
+            std::vector<u64> piv;
+            host::ReduceStats st;
             try {
-                for (u32 q; (q = queue.take()) < count;) {
-                    Cloud& C = cl[q];
-                    if (C.n == 0) continue;
-                    std::vector<host::Entry> cols(C.ci.size());
-                    for (u64 i = 0; i < cols.size(); ++i) cols[i] = host::Entry{C.ci[i], C.cd[i]};
-                    host::HostComplex hc{C.mat.data(), nullptr, nullptr, nullptr, C.n, C.thr};
-                    std::vector<u64> piv;
-                    host::ReduceStats st;
-                    if (!host::dense_pairs_dim1(hc, cols, C.keys.data(), C.keys.size(), C.bars, piv, st))
-                        C.bars = host::compute_pairs(hc, 1, 1, cols, C.emi.data(), C.emf.data(), piv, st, per_cloud);
-                }
+                if (!host::dense_pairs_dim1(hc, cols, C.keys.data(), C.keys.size(), C.bars, piv, st))
+                    C.bars = host::compute_pairs(hc, 1, 1, cols, C.emi.data(), C.emf.data(), piv, st, per_cloud);
             } catch (const std::exception& e) {
-                errs[t] = e.what();
-                queue.halt();
+                throw Error(TT_ERR_INTERNAL, e.what());
             }
         };
-        std::vector<std::thread> pool;
-        auto join = [&] {
-            for (auto& th : pool) th.join();
-            pool.clear();
-        };
-        // device front end, cloud by cloud; each cloud goes to the reducers
+        // device front end of a lane's clouds; each cloud goes to the reducers
         // once its outputs are on the host
-        auto front_end = [&] {
-            Staging st(c, sizes, count);
-            u64 off = 0;
-            for (u32 q = 0; q < count; ++q) {
+        std::atomic<u32> next{0};
+        auto front_end = [&](tt_ctx* lc) {
+            u32 before = NOV;
+            for (u32 q; (q = next.fetch_add(1)) < count && !queue.halted();) {
                 Cloud& C = cl[q];
-                C.n = sizes[q];
-                C.off = off;
-                off += C.n;
-                if (C.n == 0) continue;   // (published with the next cloud)
+                if (C.n == 0) continue;
                 const u32 n = C.n;
-                f32* mat = c->arena.get<f32>(S_MAT, u64(n) * n + 1);
-                C.thr = dense_radius(c, x + C.off * dim, n, dim, kind, p, mat);
+                f32* mat = lc->arena.get<f32>(S_MAT, u64(n) * n + 1);
+                C.thr = dense_radius(lc, x + C.off * dim, n, dim, kind, p, mat);
                 Complex cx{mat, nullptr, nullptr, nullptr, n, C.thr};
-                // (the radius has just been waited for, and with it the copies of the cloud before)
-                if (q) queue.publish(q - 1);
+                // (the radius has just been waited for, and with it the copies of the lane's cloud before)
+                if (before != NOV) queue.publish(before);
                 Dim0Out r;
-                dim0(c, cx, 1, r);
+                dim0(lc, cx, 1, r);
+                Staging st = out_of[q];
+                st.stream = lc->stream;
                 st.take(C.mat, mat, u64(n) * n);
                 st.take(C.keys, r.keys, n <= host::kCocycleMaxN ? r.m : 0);
                 st.take(C.h0d, r.h0, r.nh0);
@@ -260,22 +307,48 @@ extern "C" int tt_topo_forward(tt_ctx* c, const float* x, const uint32_t* sizes,
                 st.take(C.cd, r.cd, r.ncols);
                 st.take(C.emi, r.emi, r.ncols);
                 st.take(C.emf, r.emf, r.ncols);
+                before = q;
             }
-            TT_CUDA(cudaStreamSynchronize(c->stream));
-            if (count) queue.publish(count - 1);
+            TT_CUDA(cudaStreamSynchronize(lc->stream));
+            if (before != NOV) queue.publish(before);
         };
+        auto work = [&](u32 t) {   // of thread t: its lane, then the reductions
+            try {
+                if (t < lanes) {
+                    TT_CUDA(cudaSetDevice(c->device));
+                    front_end(lane[t]);
+                }
+                for (u32 q; (q = queue.take()) != NOV;) reduce(cl[q]);
+            } catch (...) {
+                errs[t] = std::current_exception();
+                queue.halt();
+                if (t < lanes) cudaStreamSynchronize(lane[t]->stream);   // no copy outlives its target
+            }
+        };
+        // the other lanes' streams follow the caller's
+        if (lanes > 1) {
+            cudaEvent_t ev;
+            TT_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+            cudaError_t e = cudaEventRecord(ev, c->stream);
+            for (u32 l = 1; l < lanes && e == cudaSuccess; ++l) e = cudaStreamWaitEvent(lane[l]->stream, ev, 0);
+            cudaEventDestroy(ev);
+            TT_CUDA(e);
+        }
+        std::vector<u64> launched(lanes);
+        for (u32 l = 0; l < lanes; ++l) launched[l] = lane[l]->launches;
+        std::vector<std::thread> pool;
         try {
             for (u32 t = 1; t < nt; ++t) pool.emplace_back(work, t);
-            front_end();
         } catch (...) {
             queue.halt();
-            join();
+            for (auto& th : pool) th.join();
             throw;
         }
         work(0);
-        join();
+        for (auto& th : pool) th.join();
+        for (u32 l = 1; l < lanes; ++l) c->launches += lane[l]->launches - launched[l];
         for (auto& e : errs)
-            if (!e.empty()) throw Error(TT_ERR_INTERNAL, e);
+            if (e) std::rethrow_exception(e);
         // pack, with global point ids
         auto* R = new TopoResult;
         R->h0_off.assign(count + 1, 0);
