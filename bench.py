@@ -569,18 +569,15 @@ def batch_block(ctx, dev, reps: int = 5) -> dict:
 
 def batch_traffic(sizes, edges: int, ms: float) -> dict:
     """Algorithmic HBM bytes of one batched run: the matrices written (4 B a
-    pair, full layout) and their lower triangles read twice (count, keys),
-    the kept keys written once and moved by the stable radix passes of every
-    cloud's keys over their 31 distance bits (read for the histogram, read
-    and written by the scatter: 24 B an edge a pass; 8-bit digits, four
-    passes), the edge list emitted (8 B key read, 12 B written)."""
+    pair, full layout) and their lower triangles read twice (histogram, keys),
+    the kept keys written into their items and read back (8 B each), the edge
+    list written (12 B)."""
     pk, src = peaks()
     mat = 4 * sum(n * n for n in sizes)
     tri = 4 * sum(n * (n - 1) // 2 for n in sizes)
-    passes = -(-31 // 8)
-    b = mat + 2 * tri + 8 * edges + passes * 24 * edges + 20 * edges
+    b = mat + 2 * tri + 28 * edges
     gbs = b / (ms * 1e-3) / 1e9
-    return {"algorithmic_bytes": b, "radix_passes": passes, "achieved_gbs": gbs, "peak_gbs": pk["hbm_gbs"],
+    return {"algorithmic_bytes": b, "achieved_gbs": gbs, "peak_gbs": pk["hbm_gbs"],
             "frac": gbs / pk["hbm_gbs"], "peak_source": src}
 
 

@@ -51,9 +51,11 @@ const char* tt_last_error(const tt_ctx* ctx);
 uint64_t tt_ctx_launches(const tt_ctx* ctx);
 int tt_ctx_synchronize(tt_ctx* ctx);
 /* Exact-kNN engine: 0 = automatic (the tcgen05 tensor-core Gram filter for
- * L2 in R^32 with k <= 16 and n >= 1024, else the exhaustive scan),
- * 1 = always the exhaustive scan, 2 = the filter wherever it applies.
- * Every engine returns the same lists. */
+ * L2 in R^32 with k <= 16 and n >= 1024; the search in spatial order for the
+ * other L1, L2, Linf and Lp (p <= 64) lists of at least 512 points in at most
+ * 64 dimensions; else the exhaustive scan), 1 = always the exhaustive scan
+ * (of radius graphs and spanning trees too), 2 = the filter wherever it
+ * applies, else the scan. Every engine returns the same lists. */
 int tt_ctx_set_knn_mode(tt_ctx* ctx, int mode);
 /* Options::memory_budget (turbotops.hpp:81, rips.hpp:383-416): the bytes a
  * dense distance matrix may take; 0 = half of the host's physical memory.

@@ -16,6 +16,10 @@
 // descending order with the edge's diameter, and whether that cofacet has a
 // zero-apparent facet. Only the pivot lookup stays on the host.
 //
+// Dense complexes whose keys pack go by vertex pairs (the apparent scan needs no
+// sorted order); up to 2,048 vertices every count stays on the device
+// (dim0_small), up to 128 the whole stage is one block (k_dim0_tiny).
+//
 // The same stage covers the sparse complex (rips.hpp SparseComplex :418-472):
 // cofacets of an edge are the common neighbours of its endpoints, walked from
 // the top of their sorted CSR rows.

@@ -1,15 +1,20 @@
-// tt_knn.cu — exact all-pairs scans over a point cloud: k nearest neighbours,
-// the symmetric kNN graph, the radius graph and the per-round nearest
-// foreign neighbour of the complete-graph Borůvka MST.
+// tt_knn.cu — exact searches over a point cloud: k nearest neighbours, the
+// symmetric kNN graph, the radius graph and the per-round nearest foreign
+// neighbour of the complete-graph Borůvka MST.
 //
 // Replaces graph.hpp knn_lists_exact (:211-225, k-d tree + heap, ties by id),
 // knn_graph (:286-304) + CsrGraph::from_rows (core.hpp:113-134),
 // radius_graph (:170-201) and the distance scans of mst::h0 (mst.hpp:25-99).
 // The reference's k-d tree is an exact accelerator (its pruning is
-// conservative, graph.hpp:114-119), so an exhaustive scan with the same
-// distance bits and the same (distance, id) order returns the same lists.
+// conservative, graph.hpp:114-119), so any search with the same distance bits
+// and the same (distance, id) order that leaves out only what cannot enter
+// returns the same lists.
 //
-// One tiled all-pairs scanner (tt_scan.cuh) serves all four.
+// Three engines: the tensor-core filter (tt_knn_tc.cu; L2 lists in R^32), the
+// search in spatial order (tt_near.cuh), and the tiled exhaustive scan
+// (tt_scan.cuh), which takes what is left: few points, more than 64
+// dimensions, Lp beyond the filter's margin and in radius graphs and
+// spanning trees, and mode 1.
 #include <algorithm>
 
 #include "tt_near.cuh"

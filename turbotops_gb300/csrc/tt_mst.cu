@@ -5,7 +5,7 @@
 // of a graph has the same multiset of weights, so any MST gives the same
 // sorted death list. Here each round proposes, for every component, its
 // minimum outgoing edge under the strict order (d, combinatorial index):
-// the all-pairs scan of tt_knn.cu finds each point's nearest point of
+// a search finds each point's nearest point of
 // another component, then two passes over the points take the component's
 // minimum distance and, among its points at that distance, the minimum
 // edge index (64-bit: any n). The proposals form a forest (only mutual

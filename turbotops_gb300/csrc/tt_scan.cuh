@@ -1,6 +1,7 @@
 // tt_scan.cuh — the tiled all-pairs scanner shared by the kNN, radius-graph
 // and Borůvka kernels (tt_knn.cu and tt_mst.cu say what each visitor
-// replaces in the reference).
+// replaces in the reference, and which calls the searches in spatial order
+// of tt_near.cuh take instead).
 //
 // A CTA owns kQ queries (one per thread, the query's coordinates in
 // registers) and streams every candidate point through shared memory in tiles
