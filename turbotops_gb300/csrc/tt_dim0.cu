@@ -24,6 +24,7 @@
 // cofacets of an edge are the common neighbours of its endpoints, walked from
 // the top of their sorted CSR rows.
 #include "tt_internal.cuh"
+#include "tt_rank_groups.h"
 
 namespace tt {
 
@@ -1251,14 +1252,12 @@ void dim0(tt_ctx* c, const Complex& cx, u32 maxdim, Dim0Out& out, u64 m_known) {
         // its edges has joined, so the forest is the same, and the shortest
         // few edges a point connect nearly everything: by the time the long
         // ones join, one pass finds them inside a component (or the forest
-        // is complete and they are never read). Groups of 8 n, then 64 n
-        // edges, then the rest; with fewer than 16 n edges (kNN graphs), or
-        // fewer than 2^17 in all, the extra trips would cost more than the
-        // passes they save, and all join at once.
-        const u64 group[3] = {m < std::max<u64>(16 * u64(n), 1 << 17) ? m : 8 * u64(n), std::min<u64>(m, 72 * u64(n)), m};
+        // is complete and they are never read).
+        const RankGroups group = rank_groups(m, n);
         u32 known = 0, joined = 0;
         for (int round = 0, trip = 0; round < kRounds; ++trip) {
-            const u32 upto = u32(trip < 3 ? group[trip] : m);
+            const u32 upto = u32(trip < 3 ? group.end[trip] : m);
+            if (upto < joined || upto > m) throw Error(TT_ERR_INTERNAL, "gb300: rank groups out of order");
             if (!known && joined == upto) break;
             const int first = round;
             for (int q = 0; q < kPerTrip && round < kRounds; ++q, ++round) {
