@@ -9,6 +9,7 @@
 //
 // Tiling: the 64 x 64 tiles on and above the diagonal (tt_dense_tile.cuh:
 // each computed once, an off-diagonal tile written twice).
+#include "tt_dense_one.h"
 #include "tt_dense_tile.cuh"
 
 namespace tt {
@@ -63,8 +64,6 @@ void launch_dense(u32 n, cudaStream_t s, const f32* x, u32 dim, f32 p, f32* mat,
 // A small cloud's matrix and enclosing radius in one block: points in shared
 // memory, a thread a pair, row maxima by shared atomics; the radius into
 // page-locked memory. (Otherwise: two memsets, two kernels and a copy.)
-constexpr u32 kOneN = 128;
-constexpr u32 kOneFloats = 12000;   // points x dim that 48 KB hold beside the maxima
 template <int KIND>
 __global__ void __launch_bounds__(1024) k_dense_one(const f32* __restrict__ x, u32 n, u32 dim, f32 p,
                                                    f32* __restrict__ mat, f32* __restrict__ radius) {
@@ -121,7 +120,7 @@ void dense_matrix(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, f32*
 // radius (n >= 1; slot S_ROWMAX).
 f32 dense_radius(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, f32* mat) {
     u32* h = static_cast<u32*>(c->pinned.get(4 * sizeof(u64)));
-    if (n <= kOneN && n * dim <= kOneFloats) {
+    if (dense_one_block(n, dim)) {
         auto go = [&](auto kernel) {
             kernel<<<1, 1024, sizeof(f32) * n * dim, c->stream>>>(x, n, dim, p, mat, reinterpret_cast<f32*>(h));
         };
