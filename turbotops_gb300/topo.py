@@ -113,7 +113,7 @@ def topo_loss(x: torch.Tensor, sizes, metric: str = "l2", top: int = 4, threads:
     b = diagrams(x, sizes, metric, threads)
     loss = (b.h0_death ** 2).sum()
     count = np.diff(b.h1_offset)
-    if not count.sum() or top < 1:
+    if not count.sum():
         return loss
     # the bars as one row a cloud (-inf past its last and for essential bars):
     # a handful of launches instead of a handful a cloud
