@@ -14,7 +14,7 @@
 // search in spatial order (tt_near.cuh), and the tiled exhaustive scan
 // (tt_scan.cuh), which takes what is left: few points, more than 64
 // dimensions, Lp beyond the filter's margin and in radius graphs and
-// spanning trees, and mode 1.
+// spanning trees, mode 1, and mode 2 where the filter does not apply.
 #include <algorithm>
 
 #include "tt_near.cuh"
@@ -617,7 +617,7 @@ u64 radius_graph(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, f32 t
     u32* err = error_word(c);
     // in spatial order while the boxes can prune (few coordinates) and the
     // rows fit the ordered fill's sort; otherwise the exhaustive scan
-    const bool ordered = near_applicable(n, dim, kind) && dim <= 8;
+    const bool ordered = c->knn_mode == 0 && near_applicable(n, dim, kind) && dim <= 8;
     near::View v;
     if (ordered) {
         u32* longest = err + 1;

@@ -154,7 +154,7 @@ u64 mst_deaths(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, f32* de
     u64* bi = c->arena.get<u64>(S_UF_WORK, n + 1);
     u32* bd = c->arena.get<u32>(S_UF_WORK2, n + 1);
     // the lists first (the kNN stage's own scratch is free again after it)
-    const bool ordered = kind != M_LP && n >= kOrderMin && dim >= 1 && dim <= near::kMaxDim && c->knn_mode != 1;
+    const bool ordered = kind != M_LP && n >= kOrderMin && dim >= 1 && dim <= near::kMaxDim && c->knn_mode == 0;
     const bool lists = ordered || n >= kKnnMin;
     const u32 K = std::min<u32>(kKnnK, n - 1);
     u32* kid = nullptr;
