@@ -17,8 +17,9 @@
 //   scan            of the row counts: per-cloud offsets, the total
 //   k_batch_bins    bin offsets per cloud; consecutive bins grouped into items
 //                   of at most kItemCap edges, or, where one bin holds more
-//                   than kBinMax (ties, tight clusters), the cloud marked for
-//                   the radix sort
+//                   than kBinMax (ties, tight clusters, and clouds of more than
+//                   some 4,000 points: 5,018 in any case), the cloud marked
+//                   for the radix sort
 //   k_batch_part    the kept edges as keys (d bits << 32 | index) into their
 //                   items, in no particular order inside an item
 //   k_batch_items   each item ordered in shared memory and written out as
@@ -40,6 +41,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "tt_dense_tile.cuh"
@@ -172,19 +174,26 @@ __global__ void __launch_bounds__(kHistThreads)
     for (u32 b = threadIdx.x; b < bins; b += kHistThreads) h[b] = 0;
     __syncthreads();
     const u32 lane = threadIdx.x & 31;
-    for (u32 i = ck.row0 + (threadIdx.x >> 5); i < ck.row1; i += kHistThreads / 32) {
-        u32 kept = 0;
-        for_row(mats + T.mat_off[c] + u64(i) * n, i, thr, [&](const f32(&d)[kRowLoads], u32 j) {
+    auto count = [&](auto binned) {
+        for (u32 i = ck.row0 + (threadIdx.x >> 5); i < ck.row1; i += kHistThreads / 32) {
+            u32 kept = 0;
+            for_row(mats + T.mat_off[c] + u64(i) * n, i, thr, [&](const f32(&d)[kRowLoads], u32 j) {
 #pragma unroll
-            for (int q = 0; q < kRowLoads; ++q) {
-                const bool keep = j + 32 * q < i && d[q] <= thr;
-                if (keep) atomicAdd(&h[bin_of(d[q], scale, bins)], 1u);
-                kept += keep;
-            }
-        });
-        kept = __reduce_add_sync(0xffffffffu, kept);
-        if (lane == 0) row_cnt[T.pt_off[c] + i] = kept;
+                for (int q = 0; q < kRowLoads; ++q) {
+                    const bool keep = j + 32 * q < i && d[q] <= thr;
+                    if (decltype(binned)::value && keep) atomicAdd(&h[bin_of(d[q], scale, bins)], 1u);
+                    kept += keep;
+                }
+            });
+            kept = __reduce_add_sync(0xffffffffu, kept);
+            if (lane == 0) row_cnt[T.pt_off[c] + i] = kept;
+        }
+    };
+    if (bins == 1) {   // (a cloud without items)
+        count(std::false_type{});
+        return;
     }
+    count(std::true_type{});
     __syncthreads();
     for (u32 b = threadIdx.x; b < bins; b += kHistThreads)
         if (h[b]) atomicAdd(&hist[b0 + b], h[b]);
@@ -566,10 +575,12 @@ __global__ void k_batch_edges(const f32* __restrict__ mats, const u64* __restric
 // The segmented sort's tiles of the marked clouds' keys: cloud c's
 // ceil(count / kSegTileKeys) tiles after the previous ones', their digit
 // counts at 256 per tile in the same order; *ntiles = the list's length. One
-// block; clouds <= 65536.
+// block; clouds <= 65536. place[c]: the cloud's first tile and the keys before
+// it; a group of threads a cloud then writes its tiles (by one thread a cloud,
+// 48,800 tiles of 20,000 points took 779 us).
 __global__ void __launch_bounds__(1024) k_batch_tiles(const u64* __restrict__ off, const u32* __restrict__ radix,
-                                                      u32 clouds, SegTile* __restrict__ tiles,
-                                                      u32* __restrict__ ntiles) {
+                                                      u32 clouds, uint2* __restrict__ place,
+                                                      SegTile* __restrict__ tiles, u32* __restrict__ ntiles) {
     __shared__ u32 wt[32];
     const u32 t = threadIdx.x, per = (clouds + blockDim.x - 1) / blockDim.x;
     auto keys_of = [&](u32 c) -> u32 { return radix[c] ? u32(off[c + 1] - off[c]) : 0u; };
@@ -580,13 +591,23 @@ __global__ void __launch_bounds__(1024) k_batch_tiles(const u64* __restrict__ of
     }
     u32 total, ktotal;
     u32 run = block_scan1024(sum, wt, total), krun = block_scan1024(ksum, wt, ktotal);
+    if (t == 0) *ntiles = total;
+    if (total == 0) return;
     for (u32 c = t * per; c < min(clouds, (t + 1) * per); ++c) {
-        const u32 tc = (keys_of(c) + kSegTileKeys - 1) / kSegTileKeys;
-        for (u32 q = 0; q < tc; ++q) tiles[run + q] = SegTile{c, q, 256u * run, tc, u32(off[c]) - krun};
-        run += tc;
+        place[c] = make_uint2(run, krun);
+        run += (keys_of(c) + kSegTileKeys - 1) / kSegTileKeys;
         krun += keys_of(c);
     }
-    if (t == 0) *ntiles = total;
+    __syncthreads();
+    u32 group = 32;   // threads a cloud
+    while (group < 1024 && u64(clouds) * group * 2 <= 1024) group *= 2;
+    for (u32 c = t / group; c < clouds; c += 1024 / group) {
+        const u32 tc = (keys_of(c) + kSegTileKeys - 1) / kSegTileKeys;
+        if (!tc) continue;
+        const uint2 at = place[c];
+        for (u32 q = t % group; q < tc; q += group)
+            tiles[at.x + q] = SegTile{c, q, 256u * at.x, tc, u32(off[c]) - at.y};
+    }
 }
 
 __global__ void k_batch_emit(const u64* __restrict__ keys, const u64* __restrict__ off,
@@ -655,9 +676,11 @@ struct Batch {
     u32* item_cloud = nullptr;
     u32* radix = nullptr;           // clouds left to the radix sort
     u64* edge_off = nullptr;
+    uint2* tile_place = nullptr;    // a marked cloud's first tile, the keys before it
     SegTile* seg_tiles = nullptr;   // the segmented sort's tiles of the kept keys (built on the device)
     u32* seg_ntiles = nullptr;      // ... their number
     u32 nseg_tiles = 0;             // capacity: every cloud's largest key count in tiles
+    u32 sure_tiles = 0;             // ... of the clouds that have no items
     u64 seg_hist = 0;               // the digit counts' capacity: 256 per tile
     f32* ed = nullptr;
     int32_t* ev = nullptr;
@@ -784,13 +807,14 @@ struct Batch {
         // the distance bits alone (stable: ties keep the index order): four
         // 8-bit passes
         const u32 g3 = u32(std::min<u64>((total_pts * 32 + 255) / 256, u64(owner->sms) * 32));
-        k_batch_tiles<<<1, 1024, 0, s>>>(edge_off, radix, clouds, seg_tiles, seg_ntiles);
+        k_batch_tiles<<<1, 1024, 0, s>>>(edge_off, radix, clouds, tile_place, seg_tiles, seg_ntiles);
         TT_LAUNCH("k_batch_tiles");
         k_batch_edges<<<g3, 256, 0, s>>>(mats, mat_off, sizes, pt_off, row_cloud, total_pts, radius, radix, ib, row_off,
                                          keys);
         TT_LAUNCH("k_batch_edges");
         const bool swapped =
-            radix_sort_segments(&sctx, keys, kbuf, edge_off, seg_tiles, seg_ntiles, nseg_tiles, seg_hist, 31, ib);
+            radix_sort_segments(&sctx, keys, kbuf, edge_off, seg_tiles, seg_ntiles, nseg_tiles, sure_tiles, seg_hist, 31,
+                                ib);
         const u32 g4 = std::min<u32>(std::max<u32>(nseg_tiles, 1), u32(owner->sms) * 8);
         k_batch_emit<<<g4, 256, 0, s>>>(swapped ? kbuf : keys, edge_off, seg_tiles, seg_ntiles, ib, ed, ev);
         TT_LAUNCH("k_batch_emit");
@@ -849,11 +873,12 @@ Batch* batch_create(tt_ctx* c, const u32* sizes_h, u32 clouds, u32 dim, int kind
                 for (u32 i0 = 0; i0 < n; i0 += u32(kShapes[si].r))
                     for (u32 j0 = i0; j0 < n; j0 += u32(kShapes[si].c)) tiles[si].push_back(Tile{q, i0, j0});
             for (u32 i = 0; i < n; ++i) row_cloud.push_back(q);
-            // chunks of rows; bins of about 256 pairs (a power of two); items
-            // (a cloud beyond 32-bit edge positions goes to the radix sort: one
-            // bin, which then overflows)
+            // chunks of rows; bins of about 256 pairs (a power of two); items.
+            // A cloud whose pairs, spread evenly, would overflow the most bins
+            // there can be (5,018 points and more) goes to the radix sort at
+            // once: one bin, no items.
             const u64 cp = u64(n) * (n - 1) / 2;
-            u32 bins = cp < (1ull << 31) ? 64 : 1;
+            u32 bins = cp <= u64(kMaxBins) * kBinMax ? 64 : 1;
             while (bins > 1 && bins < kMaxBins && u64(bins) * 256 < cp) bins *= 2;
             for (u32 i0 = 0; i0 < n;) {
                 u32 i1 = i0;
@@ -874,7 +899,12 @@ Batch* batch_create(tt_ctx* c, const u32* sizes_h, u32 clouds, u32 dim, int kind
         // the segmented sort's capacity: every cloud's largest key count
         // (every pair kept) in tiles of kSegTileKeys, 256 digit counts a tile
         u64 seg_cap = 0;
-        for (u32 q = 0; q < clouds; ++q) seg_cap += div_up(u64(sizes_h[q]) * (sizes_h[q] - 1) / 2, u64(kSegTileKeys));
+        u64 sure = 0;   // ... of the clouds without items
+        for (u32 q = 0; q < clouds; ++q) {
+            const u64 t = div_up(u64(sizes_h[q]) * (sizes_h[q] - 1) / 2, u64(kSegTileKeys));
+            seg_cap += t;
+            if (item_off[q + 1] == item_off[q]) sure += t;
+        }
         if (256 * seg_cap >= (1ull << 32)) invalid("gb300: batch too large for the segmented sort's counts");
         b->ib = std::max(1, Batch::bits_for(u64(b->maxn) * (b->maxn - 1) / 2 + 1));
         if (b->ib + 31 + Batch::bits_for(clouds) > 64)
@@ -918,6 +948,8 @@ Batch* batch_create(tt_ctx* c, const u32* sizes_h, u32 clouds, u32 dim, int kind
         b->radix = b->alloc<u32>(clouds);
         b->edge_off = b->alloc<u64>(clouds + 1);
         b->nseg_tiles = u32(seg_cap);
+        b->sure_tiles = u32(sure);
+        b->tile_place = b->alloc<uint2>(clouds);
         b->seg_hist = 256 * seg_cap;
         b->seg_tiles = b->alloc<SegTile>(seg_cap);
         b->seg_ntiles = b->alloc<u32>(1);

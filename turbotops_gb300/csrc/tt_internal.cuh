@@ -112,7 +112,8 @@ struct SegTile {
 };
 constexpr u32 kSegTileKeys = 4096;   // keys a tile of the segmented sort
 bool radix_sort_segments(tt_ctx* c, u64* keys, u64* kbuf, const u64* seg_off, const SegTile* tl,
-                         const u32* ntiles_dev, u32 max_tiles, u64 hist_entries, int bits, int lo_bit);
+                         const u32* ntiles_dev, u32 max_tiles, u32 sure_tiles, u64 hist_entries, int bits,
+                         int lo_bit);
 
 // ---- tt_dim0.cu
 struct Dim0Out {

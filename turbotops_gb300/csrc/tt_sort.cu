@@ -123,39 +123,39 @@ __global__ void k_tile_scan(const T* __restrict__ in, u64 n, const T* __restrict
 // every tile (a segment's block of counts does not depend on the pass), so
 // a pass with narrower digits writes zeros into the bins it does not use;
 // the flat layout scans only the bins of the pass.
+struct TileRef {
+    u64 lo, hi;           // the tile's keys
+    u64 hbase;            // its count of digit d at hbase + d * hstride
+    u32 hstride, shift;   // its keys' positions lie shift past the scan of the counts
+    __device__ __forceinline__ u64 hidx(u32 d) const { return hbase + u64(d) * hstride; }
+};
 struct FlatTiles {
     static constexpr bool kAllBins = false;
     static constexpr bool kLoop = false;   // one tile a block
     u64 n;
     const unsigned long long* ndev;
     u32 tiles;
-    __device__ __forceinline__ bool valid(u32) const { return true; }
-    __device__ __forceinline__ void range(u32 b, u64& lo, u64& hi) const {
-        const u64 nn = ndev ? min(n, u64(*ndev)) : n;
-        lo = u64(b) * RS_TILE;
-        hi = lo < nn ? min(lo + RS_TILE, nn) : lo;
+    __device__ __forceinline__ u32 count() const { return tiles; }
+    __device__ __forceinline__ TileRef ref(u32 b) const {
+        const u64 nn = ndev ? min(n, u64(*ndev)) : n, lo = u64(b) * RS_TILE;
+        return TileRef{lo, lo < nn ? min(lo + RS_TILE, nn) : lo, b, tiles, 0};
     }
-    __device__ __forceinline__ u64 hidx(u32 b, u32 d) const { return u64(d) * tiles + b; }
-    __device__ __forceinline__ u32 shift(u32) const { return 0; }
 };
+// A block takes every gridDim-th tile (an empty list then costs a launch of few
+// blocks) and reads where the next one lies while it works on a tile (two loads,
+// one after the other).
 struct SegTiles {
     static constexpr bool kAllBins = true;
-    static constexpr bool kLoop = true;   // a block takes every gridDim-th tile: an empty list costs a launch
+    static constexpr bool kLoop = true;
     const SegTile* tl;
     const u64* seg_off;
     const u32* ntiles;   // tiles in the list
-    __device__ __forceinline__ bool valid(u32 b) const { return b < *ntiles; }
-    __device__ __forceinline__ void range(u32 b, u64& lo, u64& hi) const {
+    __device__ __forceinline__ u32 count() const { return *ntiles; }
+    __device__ __forceinline__ TileRef ref(u32 b) const {
         const SegTile e = tl[b];
-        const u64 end = seg_off[e.seg + 1];
-        lo = seg_off[e.seg] + u64(e.t) * RS_TILE;
-        hi = lo < end ? min(lo + RS_TILE, end) : lo;
+        const u64 lo = seg_off[e.seg] + u64(e.t) * RS_TILE;
+        return TileRef{lo, min(lo + RS_TILE, seg_off[e.seg + 1]), u64(e.hbase) + e.t, e.tcount, e.shift};
     }
-    __device__ __forceinline__ u64 hidx(u32 b, u32 d) const {
-        const SegTile e = tl[b];
-        return e.hbase + u64(d) * e.tcount + e.t;
-    }
-    __device__ __forceinline__ u32 shift(u32 b) const { return tl[b].shift; }
 };
 // The lanes holding the same digit as this lane (a sentinel digit marks an
 // empty slot). A warp whose 32 digits agree, the common case once the later
@@ -168,15 +168,19 @@ __device__ __forceinline__ u32 warp_peers(u32 dg) {
 // Digits of up to RS_MAXBITS bits (a pass sorts `width` bits from `shift`).
 // ndev (optional): the key count lives on the device (a graph-captured sort of
 // a data-dependent number of keys, n the capacity); tiles past it are empty.
+// Five blocks an SM with 256 bins: at 51 registers it held four, and a pass took
+// a tenth longer (135 M keys of four clouds 451 us, 409 at 46).
 template <int BINS, typename TM>
-__global__ void __launch_bounds__(RS_THREADS)
+__global__ void __launch_bounds__(RS_THREADS, BINS <= 256 ? 5 : 3)
 k_rs_upsweep(const u64* __restrict__ keys, TM tm, int shift, u32 width, u32* __restrict__ hist) {
     pdl_wait();
     pdl_trigger();
     __shared__ u32 h[RS_WARPS][BINS];
-    for (u32 b = blockIdx.x; tm.valid(b); b += gridDim.x) {
-    u64 tlo, n;   // this tile's keys: [tlo, n)
-    tm.range(b, tlo, n);
+    const u32 ntiles = tm.count();
+    if (blockIdx.x >= ntiles) return;
+    TileRef tile = tm.ref(blockIdx.x);
+    for (u32 b = blockIdx.x;;) {
+    const u64 tlo = tile.lo, n = tile.hi;
     const u32 nd = 1u << width, mask = nd - 1u;
     for (u32 t = threadIdx.x; t < RS_WARPS * nd; t += RS_THREADS) h[t / nd][t % nd] = 0;
     __syncthreads();
@@ -212,6 +216,8 @@ k_rs_upsweep(const u64* __restrict__ keys, TM tm, int shift, u32 width, u32* __r
 #pragma unroll
         for (int i = 0; i < RS_ITEMS; ++i) kv[i] = base + i < n ? keys[base + i] : 0ull;
     }
+    TileRef next;
+    if (TM::kLoop && b + gridDim.x < ntiles) next = tm.ref(b + gridDim.x);
     const int cnt_valid = base >= n ? 0 : int(min(u64(RS_ITEMS), n - base));
     u32 cur = 0, run = 0;
 #pragma unroll
@@ -235,9 +241,12 @@ k_rs_upsweep(const u64* __restrict__ keys, TM tm, int shift, u32 width, u32* __r
 #pragma unroll
             for (int q = 0; q < RS_WARPS; ++q) s += h[q][d];
         }
-        hist[tm.hidx(b, d)] = s;
+        hist[tile.hidx(d)] = s;
     }
     if (!TM::kLoop) break;
+    b += gridDim.x;
+    if (b >= ntiles) break;
+    tile = next;
     __syncthreads();   // the counters are free again
     }
 }
@@ -327,19 +336,18 @@ k_rs_scatter_local(const u64* __restrict__ kin, u64* __restrict__ kout, const V*
     __shared__ u32 tstart[RS_LBINS];          // the digit's first position in the ordered tile
     __shared__ u32 wsum[RS_WARPS];
     __shared__ u32 mbins[RS_WARPS][RS_LBINS]; // per-warp lane masks by digit (the ranking below)
-    for (u32 b = blockIdx.x; tm.valid(b); b += gridDim.x) {
-    u64 tbase, n;   // this tile's keys: [tbase, n)
-    tm.range(b, tbase, n);
-    if (tbase >= n) {   // (block-uniform)
-        if (!TM::kLoop) break;
-        continue;
-    }
+    const u32 ntiles = tm.count();
+    if (blockIdx.x >= ntiles) return;
+    TileRef tile = tm.ref(blockIdx.x);
+    for (u32 b = blockIdx.x;;) {
+    const u64 tbase = tile.lo, n = tile.hi;
+    if (!TM::kLoop && tbase >= n) break;   // (a listed tile holds keys)
     const u32 nd = 1u << width, mask = nd - 1u;
     for (u32 t = threadIdx.x; t < RS_WARPS * RS_LBINS; t += RS_THREADS) {
         cnt[t / RS_LBINS][t % RS_LBINS] = 0;
         mbins[t / RS_LBINS][t % RS_LBINS] = 0;
     }
-    for (u32 d = threadIdx.x; d < nd; d += RS_THREADS) gbase[d] = offs[tm.hidx(b, d)] + tm.shift(b);
+    for (u32 d = threadIdx.x; d < nd; d += RS_THREADS) gbase[d] = offs[tile.hidx(d)] + tile.shift;
     __syncthreads();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const u32 lt = (1u << lane) - 1u;
@@ -356,6 +364,8 @@ k_rs_scatter_local(const u64* __restrict__ kin, u64* __restrict__ kout, const V*
         key[i] = ok ? kin[k] : ~0ull;
         if constexpr (VALS) val[i] = ok ? vin[k] : V(0);
     }
+    TileRef next;
+    if (TM::kLoop && b + gridDim.x < ntiles) next = tm.ref(b + gridDim.x);
 #pragma unroll
     for (int i = 0; i < RS_ITEMS; ++i) {
         const u64 k = base + u64(i) * 32 + lane;
@@ -435,6 +445,9 @@ k_rs_scatter_local(const u64* __restrict__ kin, u64* __restrict__ kout, const V*
         if constexpr (VALS) vout[pos] = sval[j];
     }
     if (!TM::kLoop) break;
+    b += gridDim.x;
+    if (b >= ntiles) break;
+    tile = next;
     __syncthreads();   // the shared tile is free again
     }
 }
@@ -589,11 +602,12 @@ template bool radix_sort<u64>(tt_ctx*, u64*, u64*, u64, u64*, u64*, int, int, co
 // device. The list's length is on the device (ntiles_dev); max_tiles and
 // hist_entries bound it and its counts (blocks loop over the listed tiles and
 // the scan stops after their counts, so an empty list costs the launches
-// alone). Returns whether the result is in kbuf.
+// alone; the tiles that are sure to be listed have a block each). Returns whether the result is in kbuf.
 bool radix_sort_segments(tt_ctx* c, u64* keys, u64* kbuf, const u64* seg_off, const SegTile* tl,
-                         const u32* ntiles_dev, u32 max_tiles, u64 hist_entries, int bits, int lo_bit) {
+                         const u32* ntiles_dev, u32 max_tiles, u32 sure_tiles, u64 hist_entries, int bits,
+                         int lo_bit) {
     if (max_tiles == 0 || bits <= 0) return false;
-    const u32 ntiles = std::min<u32>(max_tiles, 8 * u32(kSMs));   // blocks (they loop over the listed tiles)
+    const u32 ntiles = std::min<u32>(max_tiles, std::max(sure_tiles, 8 * u32(kSMs)));   // blocks
     u32* hist = c->arena.get<u32>(S_SORT_HIST, hist_entries + 1);
     u64 *ka = keys, *kb = kbuf;
     bool swapped = false;
