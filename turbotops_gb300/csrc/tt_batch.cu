@@ -45,6 +45,7 @@
 #include <vector>
 
 #include "tt_dense_tile.cuh"
+#include "tt_warp_sort.cuh"
 
 namespace tt {
 
@@ -403,12 +404,108 @@ __global__ void __launch_bounds__(kPartThreads, 2)
 
 // One item: its keys counted into kSlots linear slots of its distance range
 // (about one key a slot), placed slot by slot in shared memory, and the few
-// keys of a slot put in order by insertion. An item whose distances crowd (a
-// slot of more than kSlotMax keys: ties) is ordered by a bitonic sort instead.
-// Then written out in order. Bound by shared-memory latency and so by the warps
+// keys of a slot put in order by insertion (order_crowded where distances crowd:
+// a slot of more than kSlotMax keys). Then written out in order. Bound by shared-memory latency and so by the warps
 // an SM: 312 M edges 3.1 ms with 256 threads on up to 4,096 keys (23 warps an
 // SM), now 2.27 with 384 on up to 3,840 (40 registers, 48 warps).
 constexpr u32 kSlotMax = 24;
+constexpr u32 kSlotWarp = 512;
+
+// A few keys in order, by insertion of the whole key.
+__device__ __forceinline__ void order_few(u64* k, u32 len) {
+    for (u32 x = 1; x < len; ++x) {
+        const u64 key = k[x];
+        u32 y = x;
+        while (y > 0 && k[y - 1] > key) {
+            k[y] = k[y - 1];
+            --y;
+        }
+        k[y] = key;
+    }
+}
+
+template <int K>
+__device__ __forceinline__ void order_ties(u64* __restrict__ k, u32 len, u32 d) {
+    const u32 lane = threadIdx.x & 31;
+    u32 idx[K];
+#pragma unroll
+    for (u32 q = 0; q < K; ++q) idx[q] = q * 32 + lane < len ? u32(k[q * 32 + lane]) : 0xffffffffu;
+    sort_lane_keys<K>(idx);
+    __syncwarp();
+#pragma unroll
+    for (u32 q = 0; q < K; ++q)
+        if (lane * K + q < len) k[lane * K + q] = (u64(d) << 32) | idx[q];
+}
+
+// A crowded slot's keys (at most kSlotWarp) in order, by one warp: ties by
+// their indices in registers, else an odd-even transposition.
+__device__ __forceinline__ void order_crowd(u64* k, u32 len) {
+    const u32 lane = threadIdx.x & 31, d = u32(k[0] >> 32);
+    bool ties = true;
+    for (u32 e = lane; e < len; e += 32) ties = ties && u32(k[e] >> 32) == d;
+    if (__all_sync(0xffffffffu, ties)) {
+        if (len <= 64) order_ties<2>(k, len, d);
+        else if (len <= 128) order_ties<4>(k, len, d);
+        else if (len <= 256) order_ties<8>(k, len, d);
+        else order_ties<kSlotWarp / 32>(k, len, d);
+        return;
+    }
+    for (u32 p = 0; p < len; ++p) {
+        for (u32 e = (p & 1u) + 2 * lane; e + 1 < len; e += 64) {
+            const u64 x = k[e], y = k[e + 1];
+            if (x > y) {
+                k[e] = y;
+                k[e + 1] = x;
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// A placed item (first[s]: the first of slot s's keys, m in all) with crowded
+// slots: a warp orders such a slot; where one holds more than kSlotWarp keys, the
+// block the whole item by a bitonic sort. (64 clouds of 300 lattice points, slots
+// of up to 300 ties: 189 us with the bitonic sort for every such item, 49 so. A
+// function of its own: beside the common case its code cost that 1 to 3 %.)
+__device__ __noinline__ void order_crowded(u64* sk, const u32* first, u32 m) {
+    __shared__ u16 crowd[kItemCap / (kSlotMax + 1) + 1];   // the crowded slots
+    __shared__ u32 ncrowd;
+    const u32 tid = threadIdx.x;
+    auto len_of = [&](u32 s) -> u32 { return (s + 1 < kSlots ? first[s + 1] : m) - first[s]; };
+    if (tid == 0) ncrowd = 0;
+    __syncthreads();
+    u32 most = 0;
+    for (u32 s = tid; s < kSlots; s += kItemThreads) {
+        const u32 len = len_of(s);
+        if (len > kSlotMax) crowd[atomicAdd(&ncrowd, 1u)] = u16(s);
+        most = max(most, len);
+    }
+    if (!__syncthreads_or(most > kSlotWarp)) {
+        for (u32 s = tid; s < kSlots; s += kItemThreads) {
+            const u32 len = len_of(s);
+            if (len <= kSlotMax) order_few(sk + first[s], len);
+        }
+        for (u32 q = tid >> 5; q < ncrowd; q += kItemThreads / 32) order_crowd(sk + first[crowd[q]], len_of(crowd[q]));
+        return;
+    }
+    u32 P = 2;
+    while (P < m) P <<= 1;
+    for (u32 e = m + tid; e < P; e += kItemThreads) sk[e] = ~0ull;
+    __syncthreads();
+    for (u32 size = 2; size <= P; size <<= 1)
+        for (u32 stride = size >> 1; stride; stride >>= 1) {
+            for (u32 i = tid; i < P / 2; i += kItemThreads) {
+                const u32 a = 2 * i - (i & (stride - 1)), b = a + stride;
+                const u64 x = sk[a], y = sk[b];
+                if ((x > y) == ((a & size) == 0)) {
+                    sk[a] = y;
+                    sk[b] = x;
+                }
+            }
+            __syncthreads();
+        }
+}
+
 __global__ void __launch_bounds__(kItemThreads, 4)
     k_batch_items(const Item* __restrict__ items, const u32* __restrict__ item_cloud, const u64* __restrict__ edge_off,
                   const u64* __restrict__ keys, f32* __restrict__ ed, int32_t* __restrict__ ev) {
@@ -485,48 +582,22 @@ __global__ void __launch_bounds__(kItemThreads, 4)
         }
     }
     __syncthreads();
-    if (!crowded) {
 #pragma unroll
-        for (u32 q = 0; q < kPer; ++q) {
-            const u32 e = q * kItemThreads + tid;
-            if (q * kItemThreads >= m) break;
-            if (e < m) sk[cnt[at[q] >> 16] + (at[q] & 0xffffu)] = k[q];
-        }
-        __syncthreads();
+    for (u32 q = 0; q < kPer; ++q) {
+        const u32 e = q * kItemThreads + tid;
+        if (q * kItemThreads >= m) break;
+        if (e < m) sk[cnt[at[q] >> 16] + (at[q] & 0xffffu)] = k[q];
+    }
+    __syncthreads();
+    if (!crowded) {
         u32 run = pre;
 #pragma unroll
         for (u32 q = 0; q < kSlotPer; ++q) {
-            const u32 len = c[q];
-            for (u32 x = 1; x < len; ++x) {   // insertion by the whole key
-                const u64 key = sk[run + x];
-                u32 y = x;
-                while (y > 0 && sk[run + y - 1] > key) {
-                    sk[run + y] = sk[run + y - 1];
-                    --y;
-                }
-                sk[run + y] = key;
-            }
-            run += len;
+            order_few(sk + run, c[q]);
+            run += c[q];
         }
     } else {
-        u32 P = 2;
-        while (P < m) P <<= 1;
-#pragma unroll
-        for (u32 q = 0; q < kPer; ++q) sk[q * kItemThreads + tid] = k[q];   // (past m: ~0)
-        for (u32 e = kItemCap + tid; e < P; e += kItemThreads) sk[e] = ~0ull;
-        __syncthreads();
-        for (u32 size = 2; size <= P; size <<= 1)
-            for (u32 stride = size >> 1; stride; stride >>= 1) {
-                for (u32 i = tid; i < P / 2; i += kItemThreads) {
-                    const u32 a = 2 * i - (i & (stride - 1)), b = a + stride;
-                    const u64 x = sk[a], y = sk[b];
-                    if ((x > y) == ((a & size) == 0)) {
-                        sk[a] = y;
-                        sk[b] = x;
-                    }
-                }
-                __syncthreads();
-            }
+        order_crowded(sk, cnt, m);
     }
     __syncthreads();
     for (u32 e = tid; e < m; e += kItemThreads) {
