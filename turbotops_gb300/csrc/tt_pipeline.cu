@@ -96,22 +96,6 @@ std::vector<u64> reduce_dim1(tt_ctx* c, const host::HostComplex& hc, u32 maxdim,
     const bool boundary = !hc.mat && maxdim == 1;   // (gives up past 8 triangles a kept edge)
     std::vector<u8> emf;
     std::vector<u64> emi;
-    // A dense complex: by cocycles, where they apply.
-    if (hc.mat && !r.eidx && hc.n <= host::kCocycleMaxN) {
-        const auto keys = to_host(c, r.keys, r.m);
-        sync(c);
-        std::vector<host::Entry> cols(r.ncols);
-        for (u64 i = 0; i < r.ncols; ++i) cols[i] = host::Entry{ci[i], cd[i]};
-        std::vector<u64> piv;
-        host::ReduceStats st;
-        host::Bars b;
-        if (host::dense_pairs_dim1(hc, cols, keys.data(), r.m, b, piv, st)) {
-            for (u64 i = 0; i < b.birth.size(); ++i) out.add(1, b.birth[i], b.death[i]);
-            out.columns.push_back(st.columns);
-            out.emergent.push_back(st.emergent);
-            return piv;
-        }
-    }
     if (!boundary) {
         emi = to_host(c, r.emi, r.ncols);
         emf = to_host(c, r.emf, r.ncols);
@@ -131,7 +115,16 @@ std::vector<u64> reduce_dim1(tt_ctx* c, const host::HostComplex& hc, u32 maxdim,
             sync(c);
             st = host::ReduceStats{};
         }
-        b = host::compute_pairs(hc, 1, maxdim, cols, emi.data(), emf.data(), piv, st);
+        // (a long column of a dense complex asks for the edges in order)
+        std::vector<u64> keys;
+        const host::SortedEdges edges{[&]() -> const u64* {
+                                          TT_CUDA(cudaSetDevice(c->device));   // (from a reducing thread)
+                                          keys = to_host(c, r.keys, r.m);
+                                          sync(c);
+                                          return keys.data();
+                                      },
+                                      r.m};
+        b = host::compute_pairs(hc, 1, maxdim, cols, emi.data(), emf.data(), piv, st, 0, r.eidx ? nullptr : &edges);
     }
     for (u64 i = 0; i < b.birth.size(); ++i) out.add(1, b.birth[i], b.death[i]);
     out.columns.push_back(st.columns);

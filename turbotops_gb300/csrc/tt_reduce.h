@@ -3,6 +3,7 @@
 #pragma once
 #include <stdint.h>
 
+#include <functional>
 #include <vector>
 
 namespace tt {
@@ -35,6 +36,17 @@ struct ReduceStats {
     uint64_t columns = 0, emergent = 0;
 };
 
+// The m kept edges of a dense complex in filtration order, as dim0 sorts them
+// (float bits of d << 33 | (2^33 - 1 - index), ascending): keys() is called at
+// most once, when a column turns out long (from whichever thread reduces it) or
+// the complex is small.
+struct SortedEdges {
+    std::function<const uint64_t*()> keys;
+    uint64_t m = 0;
+    uint64_t patience = UINT64_MAX;   // estimated ns after which a column is swept (at most a sweep's own)
+};
+constexpr uint32_t kSweepMaxN = 8192;   // points up to which long columns are swept
+
 // compute_pairs(dim) of the cohomology reducer. `cols` are the dimension-dim
 // simplices to reduce, in descending filtration order. For dim == 1 the
 // column-local part of the emergent-pair test may be supplied precomputed
@@ -42,22 +54,24 @@ struct ReduceStats {
 // reducer evaluates it. Returns the bars; `pivots` receives the index of every
 // pivot (dimension-(dim+1) simplex) found. `threads` host threads reduce
 // batches of columns in parallel (0: every hardware thread); the results do
-// not depend on it.
+// not depend on it, nor on `edges` (dimension 1 of a dense complex of at most
+// kSweepMaxN points: long columns are finished by sweeps over these, and small
+// complexes take cocycles).
 Bars compute_pairs(const HostComplex& cx, uint32_t dim, uint32_t maxdim, const std::vector<Entry>& cols,
                    const uint64_t* em_idx, const uint8_t* em_app, std::vector<uint64_t>& pivots,
-                   ReduceStats& st, unsigned threads = 0);
+                   ReduceStats& st, unsigned threads = 0, const SortedEdges* edges = nullptr);
 
 // The same pairs, bars and pivots as compute_pairs(hc, 1, ...) on a dense
-// complex, from its edges in filtration order: `keys` are the m kept edges as
-// dim0 sorts them (float bits of d << 33 | (2^33 - 1 - index), ascending),
-// `cols` the dimension-1 columns. Returns false, with nothing written, where
-// it does not apply (more than kCocycleMaxN points; many equal lengths) or
-// where its work would pass `budget` (64-bit words touched): the caller then
-// runs compute_pairs. st.emergent counts the pairs of length zero.
-constexpr uint32_t kCocycleMaxN = 8192;
+// complex, by cocycles, from its edges in filtration order (SortedEdges' keys);
+// what compute_pairs does itself up to kCocyclePoints points. Returns false, with
+// nothing written, where it does not apply (more than kSweepMaxN points; many
+// equal lengths) or where its work would pass `budget` (64-bit words touched).
+// st.emergent counts the emergent pairs, given em_idx and em_app.
+constexpr uint32_t kCocyclePoints = 256;
 bool dense_pairs_dim1(const HostComplex& hc, const std::vector<Entry>& cols, const uint64_t* keys, uint64_t m,
                       Bars& bars, std::vector<uint64_t>& pivots, ReduceStats& st,
-                      uint64_t budget = uint64_t(4) << 30);
+                      uint64_t budget = uint64_t(4) << 30, const uint64_t* em_idx = nullptr,
+                      const uint8_t* em_app = nullptr);
 
 // Reducer::assemble(dim) (rips.hpp:981-1023): the dimension-(dim + 1)
 // columns — every cofacet of the dimension-dim `simplices` (any order) through

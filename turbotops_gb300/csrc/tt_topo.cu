@@ -5,7 +5,7 @@
 // rips.hpp:52-67). Forward: for every cloud the GPU runs the dense front end
 // (distances, enclosing radius, dim0); host threads reduce dimension 1 of the
 // clouds whose front end is done while the GPU works on the next ones (by
-// cocycles, dense_pairs_dim1; compute_pairs where that does not apply),
+// columns, long ones by sweeps over the sorted edges: compute_pairs),
 // recording each bar's critical simplices; each bar value is then the length
 // of one edge:
 //   H0 death   the spanning-tree edge that merged two components
@@ -275,8 +275,8 @@ extern "C" int tt_topo_forward(tt_ctx* c, const float* x, const uint32_t* sizes,
             std::vector<u64> piv;
             host::ReduceStats st;
             try {
-                if (!host::dense_pairs_dim1(hc, cols, C.keys.data(), C.keys.size(), C.bars, piv, st))
-                    C.bars = host::compute_pairs(hc, 1, 1, cols, C.emi.data(), C.emf.data(), piv, st, per_cloud);
+                const host::SortedEdges edges{[&] { return C.keys.data(); }, C.keys.size()};
+                C.bars = host::compute_pairs(hc, 1, 1, cols, C.emi.data(), C.emf.data(), piv, st, per_cloud, &edges);
             } catch (const std::exception& e) {
                 throw Error(TT_ERR_INTERNAL, e.what());
             }
@@ -300,7 +300,7 @@ extern "C" int tt_topo_forward(tt_ctx* c, const float* x, const uint32_t* sizes,
                 Staging st = out_of[q];
                 st.stream = lc->stream;
                 st.take(C.mat, mat, u64(n) * n);
-                st.take(C.keys, r.keys, n <= host::kCocycleMaxN ? r.m : 0);
+                st.take(C.keys, r.keys, n <= host::kSweepMaxN ? r.m : 0);
                 st.take(C.h0d, r.h0, r.nh0);
                 st.take(C.h0e, r.h0_edge, r.nh0);
                 st.take(C.ci, r.cidx, r.ncols);
