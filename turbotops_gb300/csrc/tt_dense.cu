@@ -65,18 +65,18 @@ void launch_dense(u32 n, cudaStream_t s, const f32* x, u32 dim, f32 p, f32* mat,
 // memory, a thread a pair, row maxima by shared atomics; the radius into
 // page-locked memory. (Otherwise: two memsets, two kernels and a copy.)
 template <int KIND>
-__global__ void __launch_bounds__(1024) k_dense_one(const f32* __restrict__ x, u32 n, u32 dim, f32 p,
+__global__ void __launch_bounds__(1024) k_dense_one(const f32* __restrict__ x, u32 n, u32 dim, u32 stride, f32 p,
                                                    f32* __restrict__ mat, f32* __restrict__ radius) {
-    extern __shared__ f32 pt[];   // n x dim
+    extern __shared__ f32 pt[];   // n x stride
     __shared__ u32 rmax[kOneN];
-    for (u32 e = threadIdx.x; e < n * dim; e += blockDim.x) pt[e] = x[e];
+    for (u32 e = threadIdx.x; e < n * dim; e += blockDim.x) pt[e / dim * stride + e % dim] = x[e];
     if (threadIdx.x < kOneN) rmax[threadIdx.x] = 0;
     __syncthreads();
     const u32 pairs = n * (n - 1) / 2;
     for (u32 e = threadIdx.x; e < pairs; e += blockDim.x) {
         u32 a, b;
         decode_edge(e, a, b);
-        const f32 d = metric_dist(KIND, p, Row{pt + b * dim}, Row{pt + a * dim}, dim);
+        const f32 d = metric_dist(KIND, p, Row{pt + b * stride}, Row{pt + a * stride}, dim);
         mat[a * n + b] = d;
         mat[b * n + a] = d;
         atomicMax(&rmax[a], __float_as_uint(d));
@@ -120,9 +120,10 @@ void dense_matrix(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, f32*
 // radius (n >= 1; slot S_ROWMAX).
 f32 dense_radius(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, f32* mat) {
     u32* h = static_cast<u32*>(c->pinned.get(4 * sizeof(u64)));
-    if (dense_one_block(n, dim)) {
+    if (dense_one_block(n, dim, kind == M_LP)) {
+        const u32 stride = dense_one_stride(dim);
         auto go = [&](auto kernel) {
-            kernel<<<1, 1024, sizeof(f32) * n * dim, c->stream>>>(x, n, dim, p, mat, reinterpret_cast<f32*>(h));
+            kernel<<<1, 1024, sizeof(f32) * n * stride, c->stream>>>(x, n, dim, stride, p, mat, reinterpret_cast<f32*>(h));
         };
         switch (kind) {
             case M_L1: go(k_dense_one<M_L1>); break;
