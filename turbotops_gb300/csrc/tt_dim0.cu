@@ -16,8 +16,8 @@
 // descending order with the edge's diameter, and whether that cofacet has a
 // zero-apparent facet. Only the pivot lookup stays on the host.
 //
-// Dense complexes whose keys pack go by vertex pairs (the apparent scan needs no
-// sorted order); up to 2,048 vertices every count stays on the device
+// Dense complexes whose keys pack, and that keep enough of their pairs, go by vertex
+// pairs (the apparent scan needs no sorted order); up to 2,048 vertices every count stays on the device
 // (dim0_small), up to 128 the whole stage is one block (k_dim0_tiny).
 //
 // The same stage covers the sparse complex (rips.hpp SparseComplex :418-472):
@@ -371,8 +371,8 @@ __global__ void __launch_bounds__(256)
         if (b0 < a) apparent_pairs(mat, n, thr, a, b0, res);   // (warp-uniform)
 }
 
-// (The wide key layout, more than kPackedMaxN vertices: a warp for each sorted
-// edge, results by its sorted position.)
+// (The wide key layout, more than kPackedMaxN vertices, and thresholds that keep few
+// pairs: a warp for each sorted edge, results by its sorted position.)
 __global__ void k_apparent_dense(const f32* __restrict__ mat, u32 n, const u64* __restrict__ keys, EdgeFmt fmt, u64 m,
                                  u8* __restrict__ app, u32* __restrict__ emw, u8* __restrict__ emf) {
     pdl_wait();
@@ -1181,6 +1181,14 @@ static void dim0_small(tt_ctx* c, const Complex& cx, u32 maxdim, Dim0Out& out) {
     finish();
 }
 
+// The apparent scan of a dense complex goes by vertex pairs, with a word a pair,
+// where the threshold keeps at least a kPairShare-th of them. Below, the edges are
+// few and short: nearly each needs a scan of its own, a warp has several to do
+// one after the other where the next has none, and a warp for each sorted edge is
+// faster and takes a word an edge. 12,000 Gaussian points in R^3, whole stage by
+// pairs / by edges: 1/64 kept 3.8 / 2.8 ms, 1/8 6.3 / 5.2, 1/4 7.1 / 7.4, 1/2 8.2 / 12;
+// 8,000 on a circle 1.85 / 1.24, 3.0 / 2.35, 3.25 / 3.3, 3.9 / 5.5.
+constexpr u64 kPairShare = 4;
 void dim0(tt_ctx* c, const Complex& cx, u32 maxdim, Dim0Out& out, u64 m_known) {
     out = Dim0Out{};
     if (cx.mat && cx.n >= 2 && cx.n <= kSmallN) {
@@ -1189,13 +1197,13 @@ void dim0(tt_ctx* c, const Complex& cx, u32 maxdim, Dim0Out& out, u64 m_known) {
     }
     u32* err = m_known != kUnknownM ? c->arena.get<u32>(S_DIM0_ERR, 4) : nullptr;
     if (err) TT_CUDA(cudaMemsetAsync(err, 0, sizeof(u32), c->stream));
-    // packed keys of a dense complex: the apparent scan goes by vertex pairs
-    const bool pairs = cx.mat && cx.n <= kPackedMaxN;
-    const u64 m = sorted_edge_keys(c, cx, 0, !pairs && maxdim >= 1, &out.keys, &out.eidx, m_known, err);
+    const u64 m = sorted_edge_keys(c, cx, 0, !cx.mat && maxdim >= 1, &out.keys, &out.eidx, m_known, err);
     const EdgeFmt fmt{out.eidx};
     out.m = m;
     if (m >= 0xffffffffull) invalid("gb300: more than 2^32 - 1 kept edges");
     const u32 n = cx.n;
+    // (packed keys only)
+    const bool pairs = cx.mat && n <= kPackedMaxN && m >= u64(n) * (n - (n > 0)) / 2 / kPairShare;
     // per-edge flags
     u8* app = c->arena.get<u8>(S_FLAGS, 2 * m + 16);
     u8* tree = app + m + 8;
