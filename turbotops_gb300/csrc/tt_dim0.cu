@@ -17,8 +17,9 @@
 // zero-apparent facet. Only the pivot lookup stays on the host.
 //
 // Dense complexes whose keys pack, and that keep enough of their pairs, go by vertex
-// pairs (the apparent scan needs no sorted order); up to 2,048 vertices every count stays on the device
-// (dim0_small), up to 128 the whole stage is one block (k_dim0_tiny).
+// pairs (the apparent scan needs no sorted order); up to 1,280 vertices every
+// count stays on the device (dim0_small), up to 91 the whole stage is one block
+// (k_dim0_tiny).
 //
 // The same stage covers the sparse complex (rips.hpp SparseComplex :418-472):
 // cofacets of an edge are the common neighbours of its endpoints, walked from
@@ -714,7 +715,12 @@ __global__ void k_emit_dim0(const u64* __restrict__ keys, EdgeFmt fmt, const u8*
 // finishes with those. (The rounds of separate kernels cost three launches
 // and a share of a round trip each, whatever the size.)
 // --------------------------------------------------------------------------
-constexpr u32 kSmallN = 2048;
+// (Up to 1,280: with the sort on the capacity's worth of keys instead of the kept
+// ones and one block for the forest, the stage is the slower one from there on.
+// Gaussian points in R^3, this / the separate rounds in us, 1/64 of the pairs kept
+// and up to the enclosing radius: 600 points 141 / 199 and 200 / 249, 1,200 223 / 235
+// and 416 / 361, 1,500 251 / 237 and 511 / 385, 2,048 331 / 263 and 1,105 / 471.)
+constexpr u32 kSmallN = 1280;
 constexpr u32 kForestThreads = 1024;
 
 // Edges: the ranks [0, min(*m, first)) when `first`, else list[0, *count).
@@ -818,9 +824,11 @@ __global__ void k_forest_filter(const u64* __restrict__ keys, const u64* __restr
 // their own, about twenty launches of 2 to 4 us: 155 us a pass with its
 // matrix and the copies of its results; now 110).
 // --------------------------------------------------------------------------
-constexpr u32 kTinyN = 128;
-constexpr u32 kTinyPairs = kTinyN * (kTinyN - 1) / 2;   // 8,128
-constexpr u32 kTinyKeys = 8192;
+// (Up to 91: 4,095 pairs, a bitonic sort of 4,096. 91 points 110 us, dim0_small's
+// kernels 112; 92 points, sorting 8,192, 148 and 116; 128 points 238 and 116.)
+constexpr u32 kTinyN = 91;
+constexpr u32 kTinyPairs = kTinyN * (kTinyN - 1) / 2;   // 4,095
+constexpr u32 kTinyKeys = 4096;
 constexpr u32 kTinyThreads = 1024;
 struct TinySmem {
     u64 key[kTinyKeys];
