@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "../../include/turbotops_gb300.h"
+#include "tt_grow.h"
 
 namespace tt {
 
@@ -102,22 +103,21 @@ struct Arena {
 
 // Pinned host staging, grown on demand.
 struct Pinned {
-    void* p = nullptr;
-    size_t bytes = 0;
+    Grown m;
     void* get(size_t b) {
-        if (bytes < b) {
-            if (p) cudaFreeHost(p);
-            p = nullptr;
-            b = (b + b / 8 + 4095) & ~size_t(4095);
-            TT_CUDA(cudaMallocHost(&p, b));
-            bytes = b;
-        }
-        return p;
+        if (b <= m.bytes) return m.p;
+        b = (b + b / 8 + 4095) & ~size_t(4095);
+        return m.get(b,
+                     [](size_t n) {
+                         void* p = nullptr;
+                         TT_CUDA(cudaMallocHost(&p, n));
+                         return p;
+                     },
+                     [](void* p) { cudaFreeHost(p); });
     }
     void release() {
-        if (p) cudaFreeHost(p);
-        p = nullptr;
-        bytes = 0;
+        if (m.p) cudaFreeHost(m.p);
+        m = Grown{};
     }
 };
 

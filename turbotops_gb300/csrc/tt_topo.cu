@@ -256,8 +256,14 @@ extern "C" int tt_topo_forward(tt_ctx* c, const float* x, const uint32_t* sizes,
         // every cloud's part of the staging
         u64 want = 0;
         for (u32 q = 0; q < count; ++q) want += staging_bytes(cl[q].n);
-        const u64 staged = std::min(want, kStagingMax);
-        auto* staging = staged ? static_cast<unsigned char*>(c->staging.get(staged)) : nullptr;
+        u64 staged = std::min(want, kStagingMax);
+        unsigned char* staging = nullptr;
+        if (staged) try {
+                staging = static_cast<unsigned char*>(c->staging.get(staged));
+            } catch (const Error&) {   // (no page-locked memory left: the clouds' own)
+                cudaGetLastError();
+                staged = 0;
+            }
         std::vector<Staging> out_of(count);
         u64 at = 0;
         for (u32 q = 0; q < count; ++q) {
