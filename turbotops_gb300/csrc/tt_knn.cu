@@ -636,7 +636,7 @@ u64 radius_graph(tt_ctx* c, const f32* x, u32 n, u32 dim, int kind, f32 p, f32 t
     u64 nnz = 0;
     u32 status[2] = {0, 0};   // error word, longest row (of an ordered count)
     TT_CUDA(cudaMemcpyAsync(&nnz, tot, 8, cudaMemcpyDeviceToHost, c->stream));
-    TT_CUDA(cudaMemcpyAsync(status, err, sizeof(status), cudaMemcpyDeviceToHost, c->stream));
+    if (ordered) TT_CUDA(cudaMemcpyAsync(status, err, sizeof(status), cudaMemcpyDeviceToHost, c->stream));
     TT_CUDA(cudaStreamSynchronize(c->stream));
     u32* ci = c->arena.get<u32>(S_OUT1, nnz + 1);
     f32* w = c->arena.get<f32>(S_OUT2, nnz + 1);

@@ -76,6 +76,44 @@ std::vector<T> to_host(tt_ctx* c, const T* dev, u64 count) {
 
 void sync(tt_ctx* c) { TT_CUDA(cudaStreamSynchronize(c->stream)); }
 
+// Several device arrays to the host with one wait: small ones through the
+// context's page-locked memory (a copy to pageable memory is waited for by
+// itself, 6 us each).
+struct Fetch {
+    static constexpr u64 kStaged = 256 << 10;
+    struct Part {
+        void* to;
+        const void* dev;
+        u64 bytes;
+    };
+    tt_ctx* c;
+    std::vector<Part> parts;
+    explicit Fetch(tt_ctx* ctx) : c(ctx) {}
+    template <typename T>
+    void add(std::vector<T>& v, const T* dev, u64 count) {
+        v.resize(count);
+        if (count) parts.push_back(Part{v.data(), dev, count * sizeof(T)});
+    }
+    void wait() {
+        u64 total = 0;
+        for (const Part& p : parts) total += (p.bytes + 15) & ~u64(15);
+        const bool staged = total <= kStaged;
+        auto* s = staged && total ? static_cast<unsigned char*>(c->pinned.get(total)) : nullptr;
+        u64 at = 0;
+        for (const Part& p : parts) {
+            TT_CUDA(cudaMemcpyAsync(staged ? s + at : p.to, p.dev, p.bytes, cudaMemcpyDeviceToHost, c->stream));
+            at += (p.bytes + 15) & ~u64(15);
+        }
+        sync(c);
+        at = 0;
+        for (const Part& p : parts) {
+            if (staged) std::memcpy(p.to, s + at, p.bytes);
+            at += (p.bytes + 15) & ~u64(15);
+        }
+        parts.clear();
+    }
+};
+
 // H0 from a device dim0 result: finite bars in sorted-edge order, then one
 // essential bar per component (rips.hpp:850-866).
 void h0_bars(tt_ctx* c, const Dim0Out& r, Result& out) {
@@ -87,20 +125,26 @@ void h0_bars(tt_ctx* c, const Dim0Out& r, Result& out) {
 
 // compute_pairs(1) over the device's dim-1 columns; returns the pivots.
 std::vector<u64> reduce_dim1(tt_ctx* c, const host::HostComplex& hc, u32 maxdim, const Dim0Out& r, Result& out) {
-    const auto ci = to_host(c, r.cidx, r.ncols);
-    const auto cd = to_host(c, r.cd, r.ncols);
+    std::vector<u64> ci, emi, keys;
+    std::vector<f32> cd;
+    std::vector<u8> emf;
+    Fetch get(c);
+    get.add(ci, r.cidx, r.ncols);
+    get.add(cd, r.cd, r.ncols);
     // A graph complex with at most 8 triangles a kept edge (the benchmark's
     // 32-dimensional kNN graph: 0.77) is reduced through the boundary matrix
     // of its triangles: the same pairs and bars in the same order, without
     // cancelling the whole coboundary of every essential edge.
     const bool boundary = !hc.mat && maxdim == 1;   // (gives up past 8 triangles a kept edge)
-    std::vector<u8> emf;
-    std::vector<u64> emi;
     if (!boundary) {
-        emi = to_host(c, r.emi, r.ncols);
-        emf = to_host(c, r.emf, r.ncols);
+        get.add(emi, r.emi, r.ncols);
+        get.add(emf, r.emf, r.ncols);
     }
-    sync(c);
+    // the edges in order: a small dense complex always takes them, a larger one
+    // asks for them when a column is long
+    const bool small = hc.mat && !r.eidx && hc.n <= host::kCocyclePoints;
+    if (small) get.add(keys, static_cast<const u64*>(r.keys), r.m);
+    get.wait();
     std::vector<host::Entry> cols(r.ncols);
     for (u64 i = 0; i < r.ncols; ++i) cols[i] = host::Entry{ci[i], cd[i]};
     std::vector<u64> piv;
@@ -115,9 +159,8 @@ std::vector<u64> reduce_dim1(tt_ctx* c, const host::HostComplex& hc, u32 maxdim,
             sync(c);
             st = host::ReduceStats{};
         }
-        // (a long column of a dense complex asks for the edges in order)
-        std::vector<u64> keys;
         const host::SortedEdges edges{[&]() -> const u64* {
+                                          if (small) return keys.data();
                                           TT_CUDA(cudaSetDevice(c->device));   // (from a reducing thread)
                                           keys = to_host(c, r.keys, r.m);
                                           sync(c);
