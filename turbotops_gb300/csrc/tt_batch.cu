@@ -407,7 +407,7 @@ __global__ void __launch_bounds__(kPartThreads, 2)
 // keys of a slot put in order by insertion (order_crowded where distances crowd:
 // a slot of more than kSlotMax keys). Then written out in order. Bound by shared-memory latency and so by the warps
 // an SM: 312 M edges 3.1 ms with 256 threads on up to 4,096 keys (23 warps an
-// SM), now 2.27 with 384 on up to 3,840 (40 registers, 48 warps).
+// SM), now 2.17 with 384 on up to 3,840 (40 registers, 48 warps).
 constexpr u32 kSlotMax = 24;
 constexpr u32 kSlotWarp = 512;
 

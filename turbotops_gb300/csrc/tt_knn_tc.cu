@@ -1659,9 +1659,10 @@ void knn_tc(tt_ctx* c, const f32* x, u32 n, u32 k, u32* ids, f32* dists, bool de
                                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) throw Error(TT_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string(int(r)) + ")");
-    // the tiles' separations, while their table stays small (64 MB) and from
-    // kSepTiles on: kNN stage of 16-Gaussian mixtures without / with it, 40,000
-    // points 734 / 746 us, 60,000 1,115 / 941, 100,000 1,785 / 1,333
+    // the tiles' separations, while their table stays small (64 MB, as much again for
+    // the sums it is made from) and from kSepTiles on: kNN stage of 16-Gaussian
+    // mixtures without / with it, 40,000 points 734 / 746 us, 60,000 1,115 / 941,
+    // 100,000 1,785 / 1,333
     f32* sep = nullptr;
     if (ntiles >= kSepTiles && ntiles <= 4096) {
         const u64 pairs = u64(ntiles) * ntiles;

@@ -75,7 +75,7 @@ constexpr u32 kFewPoints = 10000;   // lists of fewer points: half as many queri
 
 // tt_near.cu
 constexpr u32 kBlockTiles = 4;          // tiles a separation block
-constexpr u32 kSepMaxBlocks = 4096;     // 64 MB of separations
+constexpr u32 kSepMaxBlocks = 4096;     // 64 MB of separations, 201 with the sums they are made from
 constexpr u32 kSepMinPoints = 2048;
 // Fills v.sep for the metric where it pays (kProjectDim, L1, L2, Lp).
 void near_separations(tt_ctx* c, View& v, u32 dim, int kind, f32 p);
@@ -110,9 +110,14 @@ void near_queries(tt_ctx* c, const View& v, u32 dim, const u32* cpos, const unsi
 
 #ifdef TT_NEAR_IMPL
 
-// |d|^p, fast: exponents whose power is a product with at most one square root
-// (cls 1, 2), or exp2(p log2 |d|) on the special-function unit. 0 and
-// subnormal |d| give 0, NaN stays NaN.
+// |d|^p, fast: exp2(p log2 |d|) on the special-function unit, or, for the two
+// exponents below, the product (cls 1: 1.5; cls 2: 3). Others have a short product
+// too (2.5, 4), but every class is one more copy of the kernels for all
+// dimensions, a fifth of the library's build; these two are the ones that the
+// workloads here and the tests use, and the rest take the general form (100,000 x
+// 32 mixture points, k = 15: L1.5 7.1 ms,
+// L3 6.0, by the general form 9.2). 0 and subnormal
+// |d| give 0, NaN stays NaN.
 __device__ __forceinline__ f32 sqrt_fast(f32 x) {
     f32 r;
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));

@@ -149,12 +149,14 @@ struct Staging {
 // The front end of a cloud of a few hundred points is a chain of some 25 small
 // kernels and two waits, so the clouds' chains run on kLanes streams, each with
 // a context (workspaces) of its own and driven by its own thread. A gradient
-// step over 64 clouds of 100 points 18.0 ms with one lane, 6.3 with four, 5.0
-// with six, 4.4 with eight; of 512 points 20.9, 17.5, 17.1 and 17.5 (the
-// reductions then take the time, and need the threads). Clouds beyond kLaneMaxN
-// fill the chip by themselves more and more (12 of 2,048 points: 414 ms, 407 with
-// six), and their workspaces are not held several times. Two clouds gain nothing
-// (2 x 300 points 2.46 ms, two lanes 2.56; 3 x 256 points 2.37 and 2.29).
+// step over 64 clouds of 100 points 13.4 ms with one lane, 6.9 with four, 5.3
+// with six, 4.6 with eight; of 512 points 21.6, 17.5, 17.5 and 17.5 (the
+// reductions then take the time, and need the threads); 12 of 2,048 points 86, 79,
+// 79 and 79 ms. Larger clouds fill the chip by themselves (6 of 3,000 points 218
+// ms either way), and their workspaces are not held several times. Two clouds gain
+// nothing (2 x 300 points 2.46 ms, two lanes 2.56; 3 x 256 points 2.37 and 2.29).
+// The lanes' contexts (up to 130 MB each at 2,048 points) and the staging stay
+// with the caller's context and are given back with it.
 constexpr u32 kLanes = 6;
 constexpr u32 kLaneMaxN = 2048;
 
